@@ -610,14 +610,40 @@ __global__ void __launch_bounds__(GT_WARPS * 32, 1)
 // (the dominant HBM traffic) is read once per payload with 16-byte
 // non-allocating loads, two adjacent slots per thread.  Slots z and z+1 (z even)
 // rotate to the slot pair {s, s^1}, so each gather is one 16-byte smem load.
+//
+// Bound by the HBM stream.  A thread keeps the loads of two rotations in flight
+// while it multiplies a third, and the rotations of one (256 slots, output) task are
+// split between the CTAs of a cluster, which add their residues through
+// distributed shared memory: a task is 1023 dependent memory latencies long, so
+// without the split a small database leaves the chip idle (8 outputs are 64 tasks).
+// Whole call at 1 / 8 / 96 / 192 outputs: 71 / 161 / 1667 / 3266 us (0.10 / 0.81 / 9.7 / 19.3 GB;
+// 5.9 TB/s at 192) against 898 / 941 / 2113 / 3332 us unsplit with two rotations loaded and
+// then multiplied.  Three rotations in flight (114 registers instead of 80) measured the same.
 // ---------------------------------------------------------------------------
 constexpr int PACK_THREADS = 128;
 constexpr int PACK_ZB = 2 * PACK_THREADS;  // slots per CTA
+constexpr int PACK_CHUNK = 32;             // rotations between reductions
+constexpr int PACK_MAX_SPLITS = 8;         // CTAs of a cluster (the portable limit)
 
 __device__ __forceinline__ void ldg_nc_v2(const uint64_t* p, uint64_t& a, uint64_t& b) {
     asm volatile("ld.global.nc.L1::no_allocate.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p));
 }
 
+// the six word pairs of one rotation's precomputation
+struct PackRow {
+    uint64_t t[T_EXP][2], tb[T_EXP][2];
+};
+
+__device__ __forceinline__ void pack_load(PackRow& r, const uint64_t* __restrict__ T, const uint64_t* __restrict__ Tb,
+                                          int i) {
+#pragma unroll
+    for (int k = 0; k < T_EXP; k++) {
+        ldg_nc_v2(T + (int64_t)(i * T_EXP + k) * N, r.t[k][0], r.t[k][1]);
+        ldg_nc_v2(Tb + (int64_t)(i * T_EXP + k) * N, r.tb[k][0], r.tb[k][1]);
+    }
+}
+
+// grid (N / PACK_ZB, outputs, splits), clusters of (1, 1, splits)
 __global__ void __launch_bounds__(PACK_THREADS) k_pack(const uint64_t* __restrict__ bt,
                                                        const uint64_t* __restrict__ btb,
                                                        const uint64_t* __restrict__ bth,
@@ -625,57 +651,91 @@ __global__ void __launch_bounds__(PACK_THREADS) k_pack(const uint64_t* __restric
                                                        const uint64_t* __restrict__ z_body,
                                                        uint32_t* __restrict__ S) {
     extern __shared__ uint64_t ys[];  // [3][N] condensed
-    for (int i = threadIdx.x; i < T_EXP * N; i += blockDim.x) ys[i] = y_body[i];
-    __syncthreads();
+    __shared__ uint32_t part[4][PACK_THREADS];  // this CTA's residues: [limb * 2 + slot][thread]
+    const int splits = gridDim.z, rank = blockIdx.z;
     const int j = blockIdx.y;
     const int z = blockIdx.x * PACK_ZB + 2 * threadIdx.x;
     const uint32_t ez = exponent_of_slot(z);
     const uint64_t* T = bt + (int64_t)j * NINNER * N + z;
     const uint64_t* Tb = btb + (int64_t)j * NINNER * N + z;
+    // chunks of PACK_CHUNK rotations, shared out evenly (splits <= number of chunks)
+    constexpr int CHUNKS = (NROT + PACK_CHUNK - 1) / PACK_CHUNK;
+    const int ibeg = CHUNKS * rank / splits * PACK_CHUNK;
+    int iend_all = CHUNKS * (rank + 1) / splits * PACK_CHUNK;
+    if (iend_all > NROT) iend_all = NROT;
+    PackRow ra, rb;
+    pack_load(ra, T, Tb, ibeg);
+    pack_load(rb, T, Tb, ibeg + 1 < iend_all ? ibeg + 1 : ibeg);
+    for (int i = threadIdx.x; i < T_EXP * N; i += blockDim.x) ys[i] = y_body[i];
+    __syncthreads();
     uint64_t a00 = 0, a01 = 0, a10 = 0, a11 = 0;  // a{limb}{slot}
     uint32_t g = 1;                               // 5^i mod 2N
-    for (int i0 = 0; i0 < NROT; i0 += 32) {
-        const int iend = i0 + 32 < NROT ? i0 + 32 : NROT;
-#pragma unroll 2
-        for (int i = i0; i < iend; i++) {
-            const uint32_t s1 = slot_of_exponent((g * ez) & (2 * N - 1));
-            const uint32_t s2 = slot_of_exponent(((2 * N - g) * ez) & (2 * N - 1));
-            uint64_t tv[3][2], tbv[3][2];
+    for (int e = ibeg, b = 5; e; e >>= 1, b = (b * b) & (2 * N - 1))
+        if (e & 1) g = (g * b) & (2 * N - 1);
+    auto mac = [&](const PackRow& r) {
+        const uint32_t s1 = slot_of_exponent((g * ez) & (2 * N - 1));
+        const uint32_t s2 = slot_of_exponent(((2 * N - g) * ez) & (2 * N - 1));
 #pragma unroll
-            for (int k = 0; k < T_EXP; k++) {
-                ldg_nc_v2(T + (int64_t)(i * T_EXP + k) * N, tv[k][0], tv[k][1]);
-                ldg_nc_v2(Tb + (int64_t)(i * T_EXP + k) * N, tbv[k][0], tbv[k][1]);
-            }
-#pragma unroll
-            for (int k = 0; k < T_EXP; k++) {
-                const ulonglong2 yp = *reinterpret_cast<const ulonglong2*>(ys + k * N + (s1 & ~1u));
-                const ulonglong2 bp = *reinterpret_cast<const ulonglong2*>(ys + k * N + (s2 & ~1u));
-                const uint64_t y0 = (s1 & 1) ? yp.y : yp.x, y1 = (s1 & 1) ? yp.x : yp.y;
-                const uint64_t b0 = (s2 & 1) ? bp.y : bp.x, b1 = (s2 & 1) ? bp.x : bp.y;
-                a00 += (uint64_t)(uint32_t)y0 * (uint32_t)tv[k][0] + (uint64_t)(uint32_t)b0 * (uint32_t)tbv[k][0];
-                a01 += (uint64_t)(uint32_t)y1 * (uint32_t)tv[k][1] + (uint64_t)(uint32_t)b1 * (uint32_t)tbv[k][1];
-                a10 += (y0 >> 32) * (tv[k][0] >> 32) + (b0 >> 32) * (tbv[k][0] >> 32);
-                a11 += (y1 >> 32) * (tv[k][1] >> 32) + (b1 >> 32) * (tbv[k][1] >> 32);
-            }
-            g = (g * 5) & (2 * N - 1);
+        for (int k = 0; k < T_EXP; k++) {
+            const ulonglong2 yp = *reinterpret_cast<const ulonglong2*>(ys + k * N + (s1 & ~1u));
+            const ulonglong2 bp = *reinterpret_cast<const ulonglong2*>(ys + k * N + (s2 & ~1u));
+            const uint64_t y0 = (s1 & 1) ? yp.y : yp.x, y1 = (s1 & 1) ? yp.x : yp.y;
+            const uint64_t b0 = (s2 & 1) ? bp.y : bp.x, b1 = (s2 & 1) ? bp.x : bp.y;
+            a00 += (uint64_t)(uint32_t)y0 * (uint32_t)r.t[k][0] + (uint64_t)(uint32_t)b0 * (uint32_t)r.tb[k][0];
+            a01 += (uint64_t)(uint32_t)y1 * (uint32_t)r.t[k][1] + (uint64_t)(uint32_t)b1 * (uint32_t)r.tb[k][1];
+            a10 += (y0 >> 32) * (r.t[k][0] >> 32) + (b0 >> 32) * (r.tb[k][0] >> 32);
+            a11 += (y1 >> 32) * (r.t[k][1] >> 32) + (b1 >> 32) * (r.tb[k][1] >> 32);
         }
+        g = (g * 5) & (2 * N - 1);
+    };
+    for (int i0 = ibeg; i0 < iend_all; i0 += PACK_CHUNK) {
+        const int iend = i0 + PACK_CHUNK < iend_all ? i0 + PACK_CHUNK : iend_all;
+        int i = i0;
+#pragma unroll 1
+        for (; i + 1 < iend; i += 2) {  // ra holds row i, rb row i + 1
+            mac(ra);
+            pack_load(ra, T, Tb, i + 2 < iend_all ? i + 2 : i);
+            mac(rb);
+            pack_load(rb, T, Tb, i + 3 < iend_all ? i + 3 : i);
+        }
+        if (i < iend) mac(ra);  // only the last chunk is odd
         // <= 192 products of two 28-bit values plus a residue: no overflow
         a00 = modq(a00, 0); a01 = modq(a01, 0);
         a10 = modq(a10, 1); a11 = modq(a11, 1);
     }
-    const uint64_t* Th = bth + (int64_t)j * T_EXP * N + z;
+    if (rank == 0) {
+        const uint64_t* Th = bth + (int64_t)j * T_EXP * N + z;
 #pragma unroll
-    for (int k = 0; k < T_EXP; k++) {
-        const uint64_t t0 = Th[k * N], t1 = Th[k * N + 1];
-        const uint64_t z0 = z_body[k * N + z], z1 = z_body[k * N + z + 1];
-        a00 += (uint64_t)(uint32_t)z0 * (uint32_t)t0;
-        a01 += (uint64_t)(uint32_t)z1 * (uint32_t)t1;
-        a10 += (z0 >> 32) * (t0 >> 32);
-        a11 += (z1 >> 32) * (t1 >> 32);
+        for (int k = 0; k < T_EXP; k++) {
+            const uint64_t t0 = Th[k * N], t1 = Th[k * N + 1];
+            const uint64_t z0 = z_body[k * N + z], z1 = z_body[k * N + z + 1];
+            a00 += (uint64_t)(uint32_t)z0 * (uint32_t)t0;
+            a01 += (uint64_t)(uint32_t)z1 * (uint32_t)t1;
+            a10 += (z0 >> 32) * (t0 >> 32);
+            a11 += (z1 >> 32) * (t1 >> 32);
+        }
+        a00 = modq(a00, 0); a01 = modq(a01, 0);
+        a10 = modq(a10, 1); a11 = modq(a11, 1);
     }
     uint32_t* Sj = S + (int64_t)j * 2 * N;
-    *reinterpret_cast<uint2*>(Sj + z) = make_uint2(modq(a00, 0), modq(a01, 0));
-    *reinterpret_cast<uint2*>(Sj + N + z) = make_uint2(modq(a10, 1), modq(a11, 1));
+    part[0][threadIdx.x] = (uint32_t)a00;
+    part[1][threadIdx.x] = (uint32_t)a01;
+    part[2][threadIdx.x] = (uint32_t)a10;
+    part[3][threadIdx.x] = (uint32_t)a11;
+    umma::cluster_sync();
+    for (int v = rank; v < 4; v += splits) {  // CTA `rank` adds up residue kinds rank, rank + splits, ...
+        uint64_t sum = 0;
+        for (int r = 0; r < splits; r++) {
+            uint32_t x;
+            asm volatile("ld.shared::cluster.u32 %0, [%1];"
+                         : "=r"(x)
+                         : "r"(umma::map_to_rank(&part[v][threadIdx.x], (uint32_t)r))
+                         : "memory");
+            sum += x;
+        }
+        Sj[(v >> 1) * N + z + (v & 1)] = modq(sum, v >> 1);
+    }
+    umma::cluster_sync();  // no CTA leaves while its residues are being read
 }
 
 // ---------------------------------------------------------------------------
@@ -1078,12 +1138,34 @@ cudaError_t launch_gemv(const uint16_t* db, int db_rows, int64_t db_cols, int nq
     return cudaGetLastError();
 }
 
+// CTAs per (256 slots, output) task: doubled until the grid is about 6 CTAs per SM (4 fit),
+// where the stream is bandwidth-bound and the last wave short.  Measured packing times with
+// 1 / 2 / 4 / 8 CTAs per task: 8 outputs 485 / 261 / 169 / 161 us, 32 outputs 631 / 608 / 608 /
+// 592 us, 64 outputs 1194 / 1091 / 1137 / 1150 us, 96 outputs 1788 / 1667 / 1678 / 1697 us,
+// 192 outputs 3300 / 3266 / 3322 / 3354 us.
+int pack_splits(int num_outputs, int sm_count) {
+    const int tasks = N / PACK_ZB * num_outputs;
+    int s = 2;
+    while (s < PACK_MAX_SPLITS && tasks * s < 6 * sm_count) s *= 2;
+    return s;
+}
+
 cudaError_t launch_pack(const uint64_t* bt, const uint64_t* btb, const uint64_t* bth, const uint64_t* y,
-                        const uint64_t* z, uint32_t* S, int num_outputs, cudaStream_t st) {
-    const int smem = T_EXP * N * 8;
-    dim3 grid(N / PACK_ZB, num_outputs);
-    k_pack<<<grid, PACK_THREADS, smem, st>>>(bt, btb, bth, y, z, S);
-    return cudaGetLastError();
+                        const uint64_t* z, uint32_t* S, int num_outputs, int sm_count, cudaStream_t st) {
+    const int splits = pack_splits(num_outputs, sm_count);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(N / PACK_ZB, num_outputs, splits);
+    cfg.blockDim = dim3(PACK_THREADS);
+    cfg.dynamicSmemBytes = T_EXP * N * 8;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = splits;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_pack, bt, btb, bth, y, z, S);
 }
 
 cudaError_t launch_intt_crt(const uint32_t* S, const uint32_t* iw, const uint32_t* iwp, uint64_t* R,

@@ -27,7 +27,7 @@ cudaError_t launch_gemv(const uint16_t* db, int db_rows, int64_t db_cols, int nq
 cudaError_t make_u16_col_map(CUtensorMap* map, const uint16_t* db, int db_rows, int64_t db_cols, uint32_t box_rows,
                              uint32_t box_cols);
 cudaError_t launch_pack(const uint64_t* bt, const uint64_t* btb, const uint64_t* bth, const uint64_t* y,
-                        const uint64_t* z, uint32_t* S, int num_outputs, cudaStream_t st);
+                        const uint64_t* z, uint32_t* S, int num_outputs, int sm_count, cudaStream_t st);
 // R = from_ntt(S) per (client, output) polynomial pair; with z_bodies non-null the
 // z_body x That term of client f / instances is added to S first
 cudaError_t launch_intt_crt(const uint32_t* S, const uint32_t* iw, const uint32_t* iwp, uint64_t* R,

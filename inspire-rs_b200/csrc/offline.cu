@@ -513,6 +513,7 @@ extern "C" int ipr_offline_precompute(int device, const uint16_t* d_db, uint64_t
 struct ipr_inspiring {
     int device = 0;
     int max_sets = 0;
+    int sm_count = 148;
     std::vector<void*> allocs;
     uint32_t *fw = nullptr, *fwp = nullptr, *iw = nullptr, *iwp = nullptr, *wm = nullptr, *vm = nullptr;
     uint32_t *act = nullptr, *E = nullptr, *r0 = nullptr, *S = nullptr;
@@ -546,6 +547,7 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
     auto* c = new ipr_inspiring();
     c->device = device;
     c->max_sets = max_sets;
+    cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     ipr::HostParams hp;
     ipr::host_params_init(hp);
     std::vector<uint32_t> query, wmask, vmask;
@@ -598,7 +600,7 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     k_off_finish<<<(unsigned)sets, 512, coll_smem, st>>>(c->r0, c->xb, 0, c->vm, c->fw, c->fwp, c->iw, c->iwp, c->bth,
                                                          c->a_hat);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "offline kernels");
-    if ((e = launch_pack(c->bt, c->btb, c->bth, d_y_body, d_z_body, c->S, sets, st)) != cudaSuccess ||
+    if ((e = launch_pack(c->bt, c->btb, c->bth, d_y_body, d_z_body, c->S, sets, c->sm_count, st)) != cudaSuccess ||
         (e = launch_intt_crt(c->S, c->iw, c->iwp, c->R, sets, st)) != cudaSuccess)
         return cuda_fail(e, "online kernels");
     k_inspiring_out<<<148, 256, 0, st>>>(c->a_hat, c->R, d_lwe, sets, d_out);

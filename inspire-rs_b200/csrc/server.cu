@@ -169,7 +169,8 @@ int enqueue(ipr_server* s, unsigned nq, const uint8_t* d_query, uint8_t* d_resp,
             }
         }
         rec(2);
-        CU(ipr::launch_pack(s->d_bt, s->d_btb, s->d_bth, s->d_y, s->d_z, s->d_S, (int)p.instances, st));
+        CU(ipr::launch_pack(s->d_bt, s->d_btb, s->d_bth, s->d_y, s->d_z, s->d_S, (int)p.instances, s->sm_count,
+                            st));
         rec(3);
         if (s->fold_mode >= 2) {
             const bool chain = s->fold_mode >= 3;
