@@ -1,0 +1,248 @@
+// ntt_lazy.cuh — the lazily reduced register NTTs of the dependent chains (the RGSW fold and
+// the offline collapse): forward transforms of gadget digits (< 2^19) and inverse transforms
+// of canonical values without the factor N^-1, on the register layouts of ntt_regs.cuh.
+//
+// The inverse transforms are Gentleman-Sande butterflies with the plain inverse twiddles;
+// N^-1 is folded into their callers' operands.  Every reduction is a few conditional
+// subtractions with the stated bounds, all below 16 q < 2^32.
+#pragma once
+#include <cstdint>
+
+#include "ipr_device.cuh"
+#include "ntt_regs.cuh"
+
+namespace ipr {
+namespace nttl {
+
+constexpr int EPT = nttr::EPT;
+using nttr::csub;
+using nttr::eA;
+using nttr::eB;
+
+// x < 16q (< 2^32) to [0, 2q) by three conditional subtractions on the ALU pipe: the fold is
+// bound by its integer multiplies, so these cost less than a Barrett reduction's two
+__device__ __forceinline__ uint32_t red16(uint32_t x, uint32_t q) {
+    return csub(csub(csub(x, 8 * q), 4 * q), 2 * q);
+}
+
+// forward butterfly by stage: MODE 0 leaves x unreduced (the bound grows by 2q), MODE 1
+// first brings x (< 16q) to [0, 2q).  Outputs: x + w*y, x - w*y + 2q, w*y in [0, 2q).
+template <int MODE>
+__device__ __forceinline__ void fwd_b(uint32_t& x, uint32_t& y, uint32_t w, uint32_t wp, uint32_t q) {
+    const uint32_t xx = MODE == 1 ? red16(x, q) : x;
+    const uint32_t qn = shoup_lazy(y, w, wp, q);
+    x = xx + qn;
+    y = xx + 2 * q - qn;
+}
+
+// twiddle tables interleaved with their Shoup companions ([limb][N] of (w, wp)): one 8-byte
+// load per twiddle, half the L1 requests of two separate tables.  The twiddle of element k of
+// a thread is (1 << mm) + (e >> (11 - mm)) with e = hi + k * RS + lo in every layout: hi, the
+// thread's part, is a multiple of 2^(11 - mm) at the stages run in that layout, and lo (the
+// thread bits below the register stride RS) never carries into the shifted value.  So the
+// index is the thread's base plus a compile-time constant, and the elements of one stage that
+// share a twiddle share its load.  Layout A: hi = 0, RS = 256; B: hi = 256 w, RS = 32;
+// C: hi = 256 w + 32 (l / 4), RS = 4; D: hi = 256 w + 8 l, RS = 1 (w = t / 32, l = t % 32).
+template <int RS>
+__device__ __forceinline__ int tw_idx(int mm, int hi, int k) {
+    return (1 << mm) + (hi >> (11 - mm)) + ((k * RS) >> (11 - mm));
+}
+
+template <int P, int MODE, int RS>
+__device__ __forceinline__ void fstage(uint32_t (&v)[P][EPT], int mm, int dd, int hi, const uint2* __restrict__ tw,
+                                       uint32_t q) {
+#pragma unroll
+    for (int k = 0; k < EPT; k++) {
+        if (k & dd) continue;
+        const uint2 w = __ldg(tw + tw_idx<RS>(mm, hi, k));
+#pragma unroll
+        for (int p = 0; p < P; p++) fwd_b<MODE>(v[p][k], v[p][k + dd], w.x, w.y, q);
+    }
+}
+
+// Team exchanges through xbuf.  The intra-warp transposes (B <-> C <-> D) use only the warp's
+// own 256-word region of each polynomial and synchronise only the warp, so the cross-warp
+// exchanges are fenced by where they write: A -> B stores into every warp's region, so a
+// team barrier first lets every warp finish with its region; its loads read the warp's own
+// region, which nothing else writes before the next such barrier.  B -> A stores into the
+// warp's own region (no other warp reads it until the barrier) and loads from all regions,
+// which nothing writes before the next A -> B barrier.
+template <int P>
+__device__ __forceinline__ void xchg_a2b(uint32_t (&v)[P][EPT], int t, uint32_t* xbuf, int bar) {
+    nttr::group_bar(bar);
+#pragma unroll
+    for (int p = 0; p < P; p++)
+#pragma unroll
+        for (int m = 0; m < EPT; m++) xbuf[p * N + eA(t, m)] = v[p][m];
+    nttr::group_bar(bar);
+#pragma unroll
+    for (int p = 0; p < P; p++)
+#pragma unroll
+        for (int m = 0; m < EPT; m++) v[p][m] = xbuf[p * N + eB(t, m)];
+}
+
+// XB < P: the buffer holds XB polynomials, moved XB at a time; a later chunk's stores wait at
+// a team barrier for every warp to finish loading the previous chunk from this warp's region
+template <int P, int XB = P>
+__device__ __forceinline__ void xchg_b2a(uint32_t (&v)[P][EPT], int t, uint32_t* xbuf, int bar) {
+#pragma unroll
+    for (int c0 = 0; c0 < P; c0 += XB) {
+        if (c0) nttr::group_bar(bar);
+#pragma unroll
+        for (int p = c0; p < c0 + XB && p < P; p++)
+#pragma unroll
+            for (int m = 0; m < EPT; m++) xbuf[(p - c0) * N + eB(t, m)] = v[p][m];
+        nttr::group_bar(bar);
+#pragma unroll
+        for (int p = c0; p < c0 + XB && p < P; p++)
+#pragma unroll
+            for (int m = 0; m < EPT; m++) v[p][m] = xbuf[(p - c0) * N + eA(t, m)];
+    }
+}
+
+// forward NTT of P gadget-digit polynomials (< 2^19) of one limb: layout A in, layout D out
+// in [0, 2q); xbuf holds XP >= P polynomials of this team.  Bounds: after stage s <= 6 every
+// value is below 2^19 + 2q (s + 1) <= 2^19 + 14q; stage 7 reduces x first (outputs < 4q);
+// stages 8..10 add 2q each (< 10q < 2^32); one reduction at the end.
+template <int P>
+__device__ __forceinline__ void forward_digits(uint32_t (&v)[P][EPT], int t, uint32_t* xbuf, int bar,
+                                               const uint2* __restrict__ tw, uint32_t q) {
+    const int l = t & 31, w = t >> 5;
+    uint32_t* wb = xbuf + w * 256;
+    const int hb = 256 * w, hc = 256 * w + 32 * (l >> 2), hd = 256 * w + 8 * l;
+    fstage<P, 0, 256>(v, 0, 4, 0, tw, q);
+    fstage<P, 0, 256>(v, 1, 2, 0, tw, q);
+    fstage<P, 0, 256>(v, 2, 1, 0, tw, q);
+    xchg_a2b<P>(v, t, xbuf, bar);
+    fstage<P, 0, 32>(v, 3, 4, hb, tw, q);
+    fstage<P, 0, 32>(v, 4, 2, hb, tw, q);
+    fstage<P, 0, 32>(v, 5, 1, hb, tw, q);
+    nttr::b_to_c<P>(v, l, wb);
+    fstage<P, 0, 4>(v, 6, 4, hc, tw, q);
+    fstage<P, 1, 4>(v, 7, 2, hc, tw, q);
+    fstage<P, 0, 4>(v, 8, 1, hc, tw, q);
+    nttr::c_to_d<P>(v, l, wb);
+    fstage<P, 0, 1>(v, 9, 2, hd, tw, q);
+    fstage<P, 0, 1>(v, 10, 1, hd, tw, q);
+#pragma unroll
+    for (int p = 0; p < P; p++)
+#pragma unroll
+        for (int k = 0; k < EPT; k++) v[p][k] = red16(v[p][k], q);
+}
+
+// Gentleman-Sande butterfly with a plain inverse twiddle: x + y, (x - y) * w.  Inputs below
+// OFF * q; the difference is taken as x + OFF q - y (< 2 OFF q <= 16q < 2^32); the product
+// lands in [0, 2q); the sum (< 2 OFF q <= 16q) is reduced to [0, 2q) when RED.
+template <int OFF, bool RED>
+__device__ __forceinline__ void inv_b(uint32_t& x, uint32_t& y, uint32_t w, uint32_t wp, uint32_t q) {
+    const uint32_t s = x + y;
+    const uint32_t d = x + OFF * q - y;
+    x = RED ? red16(s, q) : s;
+    y = shoup_lazy(d, w, wp, q);
+}
+
+// one inverse stage over 2 * PL polynomials: [0, PL) of limb 0, [PL, 2 PL) of limb 1
+template <int PL, int OFF, bool RED, int RS>
+__device__ __forceinline__ void istage(uint32_t (&v)[2 * PL][EPT], int mm, int dd, int hi, const uint2* __restrict__ iw) {
+#pragma unroll
+    for (int k = 0; k < EPT; k++) {
+        if (k & dd) continue;
+        const int idx = tw_idx<RS>(mm, hi, k);
+        const uint2 w0 = __ldg(iw + idx), w1 = __ldg(iw + N + idx);
+#pragma unroll
+        for (int p = 0; p < PL; p++) inv_b<OFF, RED>(v[p][k], v[p][k + dd], w0.x, w0.y, Q0);
+#pragma unroll
+        for (int p = PL; p < 2 * PL; p++) inv_b<OFF, RED>(v[p][k], v[p][k + dd], w1.x, w1.y, Q1);
+    }
+}
+
+// N * INTT of 2 * PL canonical polynomials (PL per limb): layout D in, layout A canonical out;
+// xbuf holds XB polynomials.  Value bounds entering each stage: q, 2q, 4q, 8q (then the sums
+// are reduced), 2q, 4q, 8q (reduced), 2q, 4q, 8q (reduced), 2q; below 4q at the end.
+template <int PL, int XB = 2 * PL>
+__device__ __forceinline__ void inverse_limbs(uint32_t (&v)[2 * PL][EPT], int t, uint32_t* xbuf, int bar,
+                                              const uint2* __restrict__ iw) {
+    const int l = t & 31, w = t >> 5;
+    uint32_t* wb = xbuf + w * 256;
+    const int hb = 256 * w, hc = 256 * w + 32 * (l >> 2), hd = 256 * w + 8 * l;
+    istage<PL, 1, false, 1>(v, 10, 1, hd, iw);
+    istage<PL, 2, false, 1>(v, 9, 2, hd, iw);
+    nttr::d_to_c<2 * PL, XB>(v, l, wb);
+    istage<PL, 4, false, 4>(v, 8, 1, hc, iw);
+    istage<PL, 8, true, 4>(v, 7, 2, hc, iw);
+    istage<PL, 2, false, 4>(v, 6, 4, hc, iw);
+    nttr::c_to_b<2 * PL, XB>(v, l, wb);
+    istage<PL, 4, false, 32>(v, 5, 1, hb, iw);
+    istage<PL, 8, true, 32>(v, 4, 2, hb, iw);
+    istage<PL, 2, false, 32>(v, 3, 4, hb, iw);
+    xchg_b2a<2 * PL, XB>(v, t, xbuf, bar);
+    istage<PL, 4, false, 256>(v, 2, 1, 0, iw);
+    istage<PL, 8, true, 256>(v, 1, 2, 0, iw);
+    istage<PL, 2, false, 256>(v, 0, 4, 0, iw);
+#pragma unroll
+    for (int p = 0; p < 2 * PL; p++)
+#pragma unroll
+        for (int k = 0; k < EPT; k++) {
+            const uint32_t q = p < PL ? Q0 : Q1;
+            v[p][k] = csub(csub(v[p][k], 2 * q), q);
+        }
+}
+
+// one inverse stage of a single polynomial
+template <int OFF, bool RED, int RS>
+__device__ __forceinline__ void istage_one(uint32_t (&v)[EPT], int mm, int dd, int hi, const uint2* __restrict__ iw,
+                                           uint32_t q) {
+#pragma unroll
+    for (int k = 0; k < EPT; k++) {
+        if (k & dd) continue;
+        const uint2 w = __ldg(iw + tw_idx<RS>(mm, hi, k));
+        inv_b<OFF, RED>(v[k], v[k + dd], w.x, w.y, q);
+    }
+}
+
+// N * INTT of one canonical polynomial of one limb (iw: that limb's table): layout D in, layout
+// A canonical out; the bounds of inverse_limbs
+__device__ __forceinline__ void inverse_one(uint32_t (&v)[EPT], int t, uint32_t* xbuf, int bar,
+                                            const uint2* __restrict__ iw, uint32_t q) {
+    const int l = t & 31, w = t >> 5;
+    uint32_t* wb = xbuf + w * 256;
+    const int hb = 256 * w, hc = 256 * w + 32 * (l >> 2), hd = 256 * w + 8 * l;
+    uint32_t (&p)[1][EPT] = reinterpret_cast<uint32_t (&)[1][EPT]>(v);
+    istage_one<1, false, 1>(v, 10, 1, hd, iw, q);
+    istage_one<2, false, 1>(v, 9, 2, hd, iw, q);
+    nttr::d_to_c<1>(p, l, wb);
+    istage_one<4, false, 4>(v, 8, 1, hc, iw, q);
+    istage_one<8, true, 4>(v, 7, 2, hc, iw, q);
+    istage_one<2, false, 4>(v, 6, 4, hc, iw, q);
+    nttr::c_to_b<1>(p, l, wb);
+    istage_one<4, false, 32>(v, 5, 1, hb, iw, q);
+    istage_one<8, true, 32>(v, 4, 2, hb, iw, q);
+    istage_one<2, false, 32>(v, 3, 4, hb, iw, q);
+    xchg_b2a<1>(p, t, xbuf, bar);
+    istage_one<4, false, 256>(v, 2, 1, 0, iw, q);
+    istage_one<8, true, 256>(v, 1, 2, 0, iw, q);
+    istage_one<2, false, 256>(v, 0, 4, 0, iw, q);
+#pragma unroll
+    for (int k = 0; k < EPT; k++) v[k] = csub(csub(v[k], 2 * q), q);
+}
+
+// the 8 consecutive words of layout D held by thread t (two 16-byte loads)
+__device__ __forceinline__ void load_d8(uint32_t (&r)[EPT], const uint32_t* __restrict__ p) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+    r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
+    r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+}
+
+__device__ __forceinline__ uint32_t mul_canon(uint32_t x, uint32_t w, uint32_t wp, uint32_t q) {
+    return csub(shoup_lazy(x, w, wp, q), q);
+}
+
+// 32-bit store into the shared memory of CTA `rank` of the cluster, at this CTA's address p
+__device__ __forceinline__ void st_peer(const void* p, uint32_t rank, uint32_t v) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+}  // namespace nttl
+}  // namespace ipr

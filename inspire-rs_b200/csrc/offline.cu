@@ -21,7 +21,7 @@
 //   k_off_hint     column NTTs of the DB, * query, tau_{-1}          -> act[l][I][j][s]
 //   k_off_jntt     NTT over j of 8 slots per CTA, * N^-1             -> E[l][I][s][z]
 //   k_off_gather   per 8-column tile of E, the two slot gathers        -> F[I][chain][i][l][z]
-//   k_off_collapse one CTA per (instance, chain): 1023 sequential steps of register NTTs
+//   k_off_collapse one CTA pair per (instance, chain): 1023 sequential steps of register NTTs
 //   k_off_finish   bold_t_hat and a_hat per instance
 // All values leave canonical, so the outputs equal the reference's bit for bit.
 #include <cuda_runtime.h>
@@ -35,7 +35,9 @@
 #include "ipr_b200.h"
 #include "ipr_device.cuh"
 #include "kernels.cuh"
+#include "ntt_lazy.cuh"
 #include "ntt_regs.cuh"
+#include "umma.cuh"
 
 namespace ipr {
 void set_last_error(const char* msg);
@@ -168,10 +170,10 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// smem of the collapse / finish kernels
+// smem of the finish kernel
 struct CollapseSmem {
     uint64_t x[N];               // raw value of the chain (canonical mod q)
-    uint32_t wm[3][2][N];        // W mask (collapse) or V mask (finish), NTT domain
+    uint32_t wm[3][2][N];        // V mask, NTT domain
     uint32_t xb[2][3][N];        // per limb group: NTT exchange buffers / limb staging
 };
 
@@ -200,77 +202,170 @@ __device__ __forceinline__ void to_raw(CollapseSmem& sm, uint32_t (&y)[1][EPT], 
     __syncthreads();
 }
 
-// one CTA per (instance, chain); chain 0 folds r_all with W rotated by 5^i into bold_t,
-// chain 1 folds r_bar_all with W rotated by -5^i into bold_t_bar.  Leaves the final
-// NTT-domain r_all[0] (chain 0) or raw(r_bar_all[0]) (chain 1) for k_off_finish.
-// With wrows non-null the W row of step i is read from wrows[chain][i][k][l][z] instead of
-// being rotated out of the mask (the reference's collapse takes w_all / w_bar_all as arrays).
-__global__ void __launch_bounds__(512, 1)
+// N^-1 mod q_l and N^-1 R mod q_l (R = 2^32), each with its Shoup companion
+struct CollapseScale {
+    uint32_t ninv[4], ninvr[4];  // {w0, wp0, w1, wp1}
+};
+
+struct ChainSmem {
+    uint32_t xb[3][N];            // exchange buffer of the transforms
+    uint32_t wm[3][N];            // this limb's W mask times N^-1 R
+    uint32_t pr[2][EPT][256];     // the other limb's residues of x, double buffered by step
+    uint32_t pv[2][3 * 4][256];   // the other limb's transformed digits, half of the slots
+};
+
+constexpr uint32_t INV5 = 3277;  // 5^-1 mod 2N
+
+// 32-byte store of eight words (one L2 sector)
+__device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+
+// One cluster of two CTAs (one per limb) of 256 threads per (instance, chain); chain 0 folds
+// r_all with W rotated by 5^i into bold_t, chain 1 folds r_bar_all with W rotated by -5^i
+// into bold_t_bar.  Leaves the final NTT-domain r_all[0] (chain 0) or raw(r_bar_all[0])
+// (chain 1) for k_off_finish.  With WROWS the W row of step i is read from
+// wrows[chain][i][k][l][z] instead of being rotated out of the mask (the reference's collapse
+// takes w_all / w_bar_all as arrays).
+//
+// Bound by the latency of a step where chains are few and by instruction issue where they
+// fill the chip: 1023 dependent steps of three forward transforms, a product and one inverse
+// transform per limb.  A limb needs the other only for the CRT, so each has an SM's
+// schedulers to itself, and one exchange through distributed shared memory per step carries
+// the residues (both CTAs then compose x, which thread t keeps as its 8 coefficients of layout
+// A).  The same exchange carries half of the transformed digits, so that each CTA stores
+// whole 32-byte sectors of the interleaved bold_t rows.  The transforms are the fold's lazily
+// reduced ones; their N^-1 sits in the W mask (with the Montgomery R) and in F.
+// 1 / 148 chain pairs of two at a time per SM: 5.0 / 8.0 us a step (37% and about 50% of the
+// issue slots; the rest is dependent latency, the exchange about a tenth of a step), against
+// 14 us a step for one 512-thread CTA per chain, which also stored bold_t in 4-byte pieces.
+// One instance (2 chains) 14.4 -> 5.2 ms, 74 instances 21 -> 8.2 ms.  More registers (one CTA
+// per SM, 138 instead of 128) measured the same.
+template <bool WROWS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
     k_off_collapse(const uint32_t* __restrict__ F, int64_t inst0, const uint32_t* __restrict__ wmask,
-                   const uint32_t* __restrict__ fw, const uint32_t* __restrict__ fwp, const uint32_t* __restrict__ iw,
-                   const uint32_t* __restrict__ iwp, uint64_t* __restrict__ bt, uint64_t* __restrict__ btb,
-                   uint32_t* __restrict__ r0, uint64_t* __restrict__ xbar0, const uint32_t* __restrict__ wrows) {
+                   const uint2* __restrict__ fwi, const uint2* __restrict__ iwi, CollapseScale sc,
+                   uint64_t* __restrict__ bt, uint64_t* __restrict__ btb, uint32_t* __restrict__ r0,
+                   uint64_t* __restrict__ xbar0, const uint32_t* __restrict__ wrows) {
     extern __shared__ __align__(16) uint8_t csm_raw[];
-    CollapseSmem& sm = *reinterpret_cast<CollapseSmem*>(csm_raw);
-    const int g = threadIdx.x >> 8, t = threadIdx.x & 255;
-    const int64_t I = blockIdx.x;
+    ChainSmem& sm = *reinterpret_cast<ChainSmem*>(csm_raw);
+    const int t = threadIdx.x;
+    const int g = (int)umma::cluster_rank(), peer = g ^ 1;
+    const int64_t I = blockIdx.x >> 1;
     const int chain = blockIdx.y;
     const uint32_t q = limb_q(g);
-    const uint64_t br = limb_br(g);
-    const uint32_t* Fc = F + (I * 2 + chain) * (int64_t)HALF * 2 * N;  // [i][l][z]
+    const uint32_t* Fc = F + (I * 2 + chain) * (int64_t)HALF * 2 * N + g * N;  // [i][l][z], this limb
     uint32_t* out = reinterpret_cast<uint32_t*>((chain ? btb : bt) + (inst0 + I) * (int64_t)NINNER * N);
-    if (!wrows)
-        for (int e = threadIdx.x; e < 3 * 2 * N; e += 512) (&sm.wm[0][0][0])[e] = __ldg(wmask + e);
-    const uint32_t* wr = wrows ? wrows + (int64_t)chain * NROT * 3 * 2 * N : nullptr;
-    // x = raw(r_all[1023]): r_all[1023] is never updated (packing.rs:2691)
-    uint32_t y[1][EPT];
-    {
-        const uint4* p = reinterpret_cast<const uint4*>(Fc + ((int64_t)(HALF - 1) * 2 + g) * N + eD(t, 0));
-        const uint4 a = __ldg(p), b = __ldg(p + 1);
-        y[0][0] = a.x; y[0][1] = a.y; y[0][2] = a.z; y[0][3] = a.w;
-        y[0][4] = b.x; y[0][5] = b.y; y[0][6] = b.z; y[0][7] = b.w;
-    }
-    to_raw(sm, y, g, t, iw, iwp);
-    for (int i = HALF - 2; i >= 0; i--) {
-        uint32_t f[EPT];
-        {
-            const uint4* p = reinterpret_cast<const uint4*>(Fc + ((int64_t)i * 2 + g) * N + eD(t, 0));
-            const uint4 a = __ldg(p), b = __ldg(p + 1);
-            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
-            f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-        }
-        uint32_t v[3][EPT];
-        digits(sm.x, t, v);
-        nttr::forward<3, 3>(v, t, &sm.xb[g][0][0], 1 + g, fw + g * N, fwp + g * N, q);  // layout D, canonical
-        // bold_t[i][k] condensed: limb 0 in the low word, limb 1 in the high word (condense_matrix)
+    const uint2 *fw = fwi + g * N, *iw = iwi + g * N;
+    const uint32_t nv = sc.ninv[2 * g], nvp = sc.ninv[2 * g + 1];
+    if (!WROWS)
+        for (int e = t; e < 3 * N; e += 256)
+            sm.wm[e / N][e % N] = nttl::mul_canon(__ldg(wmask + (e / N * 2 + g) * N + e % N), sc.ninvr[2 * g],
+                                                  sc.ninvr[2 * g + 1], q);
+    const uint32_t* wr = WROWS ? wrows + (int64_t)chain * NROT * 3 * 2 * N + g * N : nullptr;
+    const int z8 = 8 * t;  // layout D: this thread's slots z8 .. z8 + 7
+    const uint32_t ez = exponent_of_slot((uint32_t)z8);
+    uint64_t x[EPT];
+    uint32_t y[EPT];
+    // y (N^-1 times the limb's values, layout D) -> x: inverse transform, exchange, CRT
+    auto to_raw2 = [&](int par) {
+        nttl::inverse_one(y, t, &sm.xb[0][0], 1, iw, q);
 #pragma unroll
-        for (int k = 0; k < 3; k++)
-#pragma unroll
-            for (int m = 0; m < EPT; m++) out[(((int64_t)i * 3 + k) * N + eD(t, m)) * 2 + g] = v[k][m];
-        const uint32_t gi = gen_pow((uint32_t)i), ti = chain ? 2 * N - gi : gi;
+        for (int m = 0; m < EPT; m++) nttl::st_peer(&sm.pr[par][m][t], peer, y[m]);
+        umma::cluster_sync();
 #pragma unroll
         for (int m = 0; m < EPT; m++) {
-            const uint32_t z = (uint32_t)eD(t, m);
-            const uint32_t src = auto_src(ti, z);  // W rotated by t_i (apply_automorph_ntt)
-            uint64_t acc = (uint64_t)f[m];
+            const uint32_t o = sm.pr[par][m][t];
+            x[m] = g ? crt2m(o, y[m]) : crt2m(y[m], o);
+        }
+    };
+    // x = raw(r_all[1023]): r_all[1023] is never updated (packing.rs:2691)
+    nttl::load_d8(y, Fc + (int64_t)(HALF - 1) * 2 * N + z8);
+#pragma unroll
+    for (int m = 0; m < EPT; m++) y[m] = nttl::mul_canon(y[m], nv, nvp, q);
+    umma::cluster_sync();  // both CTAs run (their shared memory is addressable) and wm is loaded
+    to_raw2(1);
+    uint32_t gi = gen_pow(HALF - 2);
+    for (int i = HALF - 2; i >= 0; i--) {
+        const int par = i & 1;
+        uint32_t f[EPT];
+        nttl::load_d8(f, Fc + (int64_t)i * 2 * N + z8);
+        uint32_t v[3][EPT];
+#pragma unroll
+        for (int m = 0; m < EPT; m++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) v[k][m] = (uint32_t)((x[m] >> (GADGET_BITS * k)) & MASK19);
+        nttl::forward_digits<3>(v, t, &sm.xb[0][0], 1, fw, q);
+        uint32_t own[3][4];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+#pragma unroll
+            for (int m = 0; m < EPT; m++) v[k][m] = nttr::csub(v[k][m], q);
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                own[k][m] = g ? v[k][4 + m] : v[k][m];
+                nttl::st_peer(&sm.pv[par][k * 4 + m][t], peer, g ? v[k][m] : v[k][4 + m]);
+            }
+        }
+        const uint32_t ti = chain ? 2 * N - gi : gi;
+        if (WROWS) {
+            uint64_t acc[EPT];
+#pragma unroll
+            for (int m = 0; m < EPT; m++) acc[m] = f[m];
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                const uint32_t w = wr ? __ldg(wr + (((int64_t)i * 3 + k) * 2 + g) * N + z) : sm.wm[k][g][src];
-                acc += (uint64_t)w * v[k][m];  // < 2^31 + 3 q^2
+                uint32_t w[EPT];
+                nttl::load_d8(w, wr + ((int64_t)i * 3 + k) * 2 * N + z8);
+#pragma unroll
+                for (int m = 0; m < EPT; m++) acc[m] += (uint64_t)w[m] * v[k][m];  // < 2^31 + 3 q^2
             }
-            y[0][m] = mod64(acc, q, br);
+#pragma unroll
+            for (int m = 0; m < EPT; m++) y[m] = nttl::mul_canon(mod64(acc[m], q, limb_br(g)), nv, nvp, q);
+        } else {
+#pragma unroll
+            for (int m = 0; m < EPT; m++) {
+                // exponent of slot z8 + m: the three low bits of a slot are the high bits of its exponent
+                const uint32_t em = ez + (uint32_t)((((m & 1) << 2) | (m & 2) | (m >> 2)) << 9);
+                const uint32_t src = slot_of_exponent((ti * em) & (2 * N - 1));  // W rotated by t_i (apply_automorph_ntt)
+                uint64_t acc = 0;
+#pragma unroll
+                for (int k = 0; k < 3; k++) acc += (uint64_t)sm.wm[k][src] * v[k][m];  // < 3 q^2 < q R
+                const uint32_t s = redc(acc, q) + shoup_lazy(f[m], nv, nvp, q);        // < 4 q
+                y[m] = nttr::csub(nttr::csub(s, 2 * q), q);
+            }
         }
-        if (i == 0 && chain == 0) {  // r_all[0] stays in the NTT domain for k_off_finish
-            uint4* d = reinterpret_cast<uint4*>(r0 + (I * 2 + g) * N + eD(t, 0));
-            d[0] = make_uint4(y[0][0], y[0][1], y[0][2], y[0][3]);
-            d[1] = make_uint4(y[0][4], y[0][5], y[0][6], y[0][7]);
-            break;
+        gi = (gi * INV5) & (2 * N - 1);
+        const bool last = i == 0 && chain == 0;
+        if (last) {  // r_all[0] stays in the NTT domain for k_off_finish, without the N^-1
+            uint4* d = reinterpret_cast<uint4*>(r0 + (I * 2 + g) * N + z8);
+            uint32_t o[EPT];
+#pragma unroll
+            for (int m = 0; m < EPT; m++) o[m] = mod64((uint64_t)y[m] * N, q, limb_br(g));
+            d[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            d[1] = make_uint4(o[4], o[5], o[6], o[7]);
+            umma::cluster_sync();
+        } else {
+            to_raw2(par);
         }
-        __syncthreads();  // every thread has read sm.x for its digits
-        to_raw(sm, y, g, t, iw, iwp);
+        // bold_t[i][k] condensed: limb 0 in the low word, limb 1 in the high word
+        // (condense_matrix); this CTA stores slots z8 + 4 g .. + 4
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            uint32_t w[8];
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                const uint32_t o = sm.pv[par][k * 4 + m][t];
+                w[2 * m] = g ? o : own[k][m];
+                w[2 * m + 1] = g ? own[k][m] : o;
+            }
+            st_sector(out + (((int64_t)i * 3 + k) * N + z8 + 4 * g) * 2, w);
+        }
     }
-    if (chain == 1)
-        for (int e = threadIdx.x; e < N; e += 512) xbar0[I * N + e] = sm.x[e];
+    if (chain == 1 && g == 0)
+#pragma unroll
+        for (int m = 0; m < EPT; m++) xbar0[I * N + eA(t, m)] = x[m];
 }
 
 // per instance: bold_t_hat = NTT(digits(raw(r_bar_all[0]))), a_hat = raw(r_all[0] + V * bold_t_hat)
@@ -372,6 +467,47 @@ __global__ void k_narrow(const uint64_t* __restrict__ in, int64_t n, uint32_t* _
         out[e] = (uint32_t)in[e];
 }
 
+// [limb][N] twiddles and companions -> interleaved pairs; the pre-halved inverse twiddles doubled
+__global__ void k_interleave(const uint32_t* __restrict__ fw, const uint32_t* __restrict__ fwp,
+                             const uint32_t* __restrict__ iw, uint2* __restrict__ fwi, uint2* __restrict__ iwi) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 2 * N) return;
+    const uint32_t q = limb_q(e / N);
+    fwi[e] = make_uint2(fw[e], fwp[e]);
+    const uint32_t w = nttr::csub(2 * iw[e], q);
+    iwi[e] = make_uint2(w, (uint32_t)(((uint64_t)w << 32) / q));
+}
+
+constexpr uint64_t pow_mod(uint64_t b, uint64_t e, uint64_t q) {
+    uint64_t r = 1;
+    for (; e; e >>= 1, b = b * b % q)
+        if (e & 1) r = r * b % q;
+    return r;
+}
+
+CollapseScale collapse_scale() {
+    CollapseScale sc;
+    for (int l = 0; l < 2; l++) {
+        const uint64_t q = l ? Q1 : Q0, n = pow_mod(N, q - 2, q), nr = n * ((1ull << 32) % q) % q;
+        sc.ninv[2 * l] = (uint32_t)n;
+        sc.ninv[2 * l + 1] = (uint32_t)((n << 32) / q);
+        sc.ninvr[2 * l] = (uint32_t)nr;
+        sc.ninvr[2 * l + 1] = (uint32_t)((nr << 32) / q);
+    }
+    return sc;
+}
+
+// shared-memory sizes of the collapse kernels, on the current device
+cudaError_t collapse_attributes() {
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(k_off_collapse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(ChainSmem))) ||
+        (e = cudaFuncSetAttribute(k_off_collapse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(ChainSmem))))
+        return e;
+    return cudaFuncSetAttribute(k_off_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CollapseSmem));
+}
+
 int cuda_fail(cudaError_t e, const char* what) {
     static thread_local char buf[256];
     snprintf(buf, sizeof(buf), "offline precomputation: %s: %s", what, cudaGetErrorString(e));
@@ -384,20 +520,21 @@ int cuda_fail(cudaError_t e, const char* what) {
 // The collapse of `cols` columns from the reference's r_all / r_bar_all arrays with explicit W
 // rows (wrows = [2][1023][3][2][N] u32: w_all then w_bar_all) and the V mask ([3][2][N] u32):
 // bold_t / bold_t_bar [cols][3069][N], bold_t_hat [cols][3][N] condensed, a_hat [cols][N].
-// Scratch: F (cols * 32 MB), r0 (cols * 16 KB), xb (cols * 16 KB).
+// Scratch: F (cols * 32 MB), r0 (cols * 16 KB), xb (cols * 16 KB), itab (8 N words: the given
+// tables with their companions interleaved, the inverse twiddles without the halving).
 cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar_all, int64_t cols,
                                     const uint32_t* wrows, const uint32_t* vmask, const uint32_t* tab /*fw fwp iw iwp*/,
-                                    uint32_t* F, uint32_t* r0, uint64_t* xb, uint64_t* bt, uint64_t* btb, uint64_t* bth,
-                                    uint64_t* a_hat, cudaStream_t st) {
+                                    uint32_t* F, uint32_t* r0, uint64_t* xb, uint32_t* itab, uint64_t* bt, uint64_t* btb,
+                                    uint64_t* bth, uint64_t* a_hat, cudaStream_t st) {
     const int coll_smem = (int)sizeof(CollapseSmem);
-    cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_off_collapse, cudaFuncAttributeMaxDynamicSharedMemorySize, coll_smem)) ||
-        (e = cudaFuncSetAttribute(k_off_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, coll_smem)))
-        return e;
+    cudaError_t e = collapse_attributes();
+    if (e) return e;
     const uint32_t *fw = tab, *fwp = tab + 2 * N, *iw = tab + 4 * N, *iwp = tab + 6 * N;
     k_off_to_f<<<148 * 8, 256, 0, st>>>(r_all, r_bar_all, cols, F);
-    k_off_collapse<<<dim3((unsigned)cols, 2), 512, coll_smem, st>>>(F, 0, nullptr, fw, fwp, iw, iwp, bt, btb, r0, xb,
-                                                                   wrows);
+    uint2* it = reinterpret_cast<uint2*>(itab);
+    k_interleave<<<2 * N / 256, 256, 0, st>>>(fw, fwp, iw, it, it + 2 * N);
+    k_off_collapse<true><<<dim3((unsigned)(2 * cols), 2), 256, (int)sizeof(ChainSmem), st>>>(
+        F, 0, nullptr, it, it + 2 * N, collapse_scale(), bt, btb, r0, xb, wrows);
     k_off_finish<<<(unsigned)cols, 512, coll_smem, st>>>(r0, xb, 0, vmask, fw, fwp, iw, iwp, bth, a_hat);
     return cudaGetLastError();
 }
@@ -440,7 +577,7 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
     };
     cudaError_t e;
     const size_t tb = 2 * N * sizeof(uint32_t);
-    if ((e = cudaMalloc(&d_tab, 4 * tb)) != cudaSuccess || (e = cudaMalloc(&d_query, query.size() * 4)) != cudaSuccess ||
+    if ((e = cudaMalloc(&d_tab, 8 * tb)) != cudaSuccess || (e = cudaMalloc(&d_query, query.size() * 4)) != cudaSuccess ||
         (e = cudaMalloc(&d_wv, 2 * wmask.size() * 4)) != cudaSuccess ||
         (e = cudaMalloc(&d_act, chunk * 2ull * N * N * 4)) != cudaSuccess ||
         (e = cudaMalloc(&d_E, chunk * 2ull * N * N * 4)) != cudaSuccess ||
@@ -450,6 +587,7 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
         return cuda_fail(e, "scratch allocation");
     }
     uint32_t *d_fw = d_tab, *d_fwp = d_tab + 2 * N, *d_iw = d_tab + 4 * N, *d_iwp = d_tab + 6 * N;
+    uint32_t *d_fwi = d_tab + 8 * N, *d_iwi = d_tab + 12 * N;  // interleaved with their companions
     uint32_t *d_wm = d_wv, *d_vm = d_wv + wmask.size();
     int status = IPR_OK;
     do {
@@ -457,6 +595,8 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
             (e = cudaMemcpyAsync(d_fwp, hp.fwp.data(), tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_iw, hp.iw.data(), tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_iwp, hp.iwp.data(), tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(d_fwi, hp.fwi.data(), 2 * tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(d_iwi, hp.iwi.data(), 2 * tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_query, query.data(), query.size() * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_wm, wmask.data(), wmask.size() * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_vm, vmask.data(), vmask.size() * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) {
@@ -466,8 +606,7 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
         const int hint_smem = 2 * HCOLS * N * 4, gather_smem = N * GZ * 4, coll_smem = (int)sizeof(CollapseSmem);
         if ((e = cudaFuncSetAttribute(k_off_hint, cudaFuncAttributeMaxDynamicSharedMemorySize, hint_smem)) ||
             (e = cudaFuncSetAttribute(k_off_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, gather_smem)) ||
-            (e = cudaFuncSetAttribute(k_off_collapse, cudaFuncAttributeMaxDynamicSharedMemorySize, coll_smem)) ||
-            (e = cudaFuncSetAttribute(k_off_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, coll_smem))) {
+            (e = collapse_attributes())) {
             status = cuda_fail(e, "kernel attributes");
             break;
         }
@@ -478,8 +617,9 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
                 d_db, (int64_t)db_rows, (int64_t)i0 * N, ncols, d_query, d_fw, d_fwp, d_act);
             k_off_jntt<<<dim3(N / JS, (unsigned)c, 2), 256, 0, st>>>(d_act, c, d_fw, d_fwp, d_E);
             k_off_gather<<<dim3(N / GZ, (unsigned)c, 2), 256, gather_smem, st>>>(d_E, c, d_act);  // F reuses act
-            k_off_collapse<<<dim3((unsigned)c, 2), 512, coll_smem, st>>>(d_act, (int64_t)i0, d_wm, d_fw, d_fwp, d_iw,
-                                                                       d_iwp, d_bt, d_btb, d_r0, d_xb, nullptr);
+            k_off_collapse<false><<<dim3((unsigned)(2 * c), 2), 256, (int)sizeof(ChainSmem), st>>>(
+                d_act, (int64_t)i0, d_wm, reinterpret_cast<uint2*>(d_fwi), reinterpret_cast<uint2*>(d_iwi),
+                collapse_scale(), d_bt, d_btb, d_r0, d_xb, nullptr);
             k_off_finish<<<(unsigned)c, 512, coll_smem, st>>>(d_r0, d_xb, (int64_t)i0, d_vm, d_fw, d_fwp, d_iw, d_iwp,
                                                               d_bth, d_a_hat);
             if ((e = cudaGetLastError()) != cudaSuccess) status = cuda_fail(e, "launch");
@@ -516,6 +656,7 @@ struct ipr_inspiring {
     int sm_count = 148;
     std::vector<void*> allocs;
     uint32_t *fw = nullptr, *fwp = nullptr, *iw = nullptr, *iwp = nullptr, *wm = nullptr, *vm = nullptr;
+    uint32_t *fwi = nullptr, *iwi = nullptr;  // the twiddles interleaved with their companions
     uint32_t *act = nullptr, *E = nullptr, *r0 = nullptr, *S = nullptr;
     uint64_t *xb = nullptr, *a_hat = nullptr, *bt = nullptr, *btb = nullptr, *bth = nullptr, *R = nullptr;
     template <typename T>
@@ -554,7 +695,7 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
     ipr::offline_host_inputs(hp, 1, query, wmask, vmask);
     const size_t tb = 2 * ipr::N * 4, ms = (size_t)max_sets, NN = (size_t)ipr::N * ipr::N;
     if ((e = c->alloc(&c->fw, tb)) || (e = c->alloc(&c->fwp, tb)) || (e = c->alloc(&c->iw, tb)) ||
-        (e = c->alloc(&c->iwp, tb)) || (e = c->alloc(&c->wm, wmask.size() * 4)) ||
+        (e = c->alloc(&c->iwp, tb)) || (e = c->alloc(&c->fwi, 2 * tb)) || (e = c->alloc(&c->iwi, 2 * tb)) || (e = c->alloc(&c->wm, wmask.size() * 4)) ||
         (e = c->alloc(&c->vm, vmask.size() * 4)) || (e = c->alloc(&c->act, ms * 2 * NN * 4)) ||
         (e = c->alloc(&c->E, ms * 2 * NN * 4)) || (e = c->alloc(&c->r0, ms * 2 * ipr::N * 4)) ||
         (e = c->alloc(&c->xb, ms * ipr::N * 8)) || (e = c->alloc(&c->a_hat, ms * ipr::N * 8)) ||
@@ -565,15 +706,14 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
         (e = cudaMemcpy(c->fwp, hp.fwp.data(), tb, cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(c->iw, hp.iw.data(), tb, cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(c->iwp, hp.iwp.data(), tb, cudaMemcpyHostToDevice)) ||
+        (e = cudaMemcpy(c->fwi, hp.fwi.data(), 2 * tb, cudaMemcpyHostToDevice)) ||
+        (e = cudaMemcpy(c->iwi, hp.iwi.data(), 2 * tb, cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(c->wm, wmask.data(), wmask.size() * 4, cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(c->vm, vmask.data(), vmask.size() * 4, cudaMemcpyHostToDevice)) ||
         (e = ipr::init_device_kernels()) || (e = ipr::set_constants(hp.barrett, hp.q0_inv_mod_q1)) ||
         (e = cudaFuncSetAttribute(ipr::k_lwe_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * ipr::HCOLS * ipr::N * 4)) ||
         (e = cudaFuncSetAttribute(ipr::k_off_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, ipr::N * ipr::GZ * 4)) ||
-        (e = cudaFuncSetAttribute(ipr::k_off_collapse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(ipr::CollapseSmem))) ||
-        (e = cudaFuncSetAttribute(ipr::k_off_finish, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(ipr::CollapseSmem)))) {
+        (e = ipr::collapse_attributes())) {
         ipr_inspiring_destroy(c);
         return ipr::cuda_fail(e, "ipr_inspiring_create");
     }
@@ -595,8 +735,9 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     k_lwe_prep<<<dim3(N / HCOLS, (unsigned)sets), 512, 2 * HCOLS * N * 4, st>>>(d_lwe, sets, c->fw, c->fwp, c->act);
     k_off_jntt<<<dim3(N / JS, (unsigned)sets, 2), 256, 0, st>>>(c->act, sets, c->fw, c->fwp, c->E);
     k_off_gather<<<dim3(N / GZ, (unsigned)sets, 2), 256, N * GZ * 4, st>>>(c->E, sets, c->act);
-    k_off_collapse<<<dim3((unsigned)sets, 2), 512, coll_smem, st>>>(c->act, 0, c->wm, c->fw, c->fwp, c->iw, c->iwp,
-                                                                   c->bt, c->btb, c->r0, c->xb, nullptr);
+    k_off_collapse<false><<<dim3((unsigned)(2 * sets), 2), 256, (int)sizeof(ChainSmem), st>>>(
+        c->act, 0, c->wm, reinterpret_cast<uint2*>(c->fwi), reinterpret_cast<uint2*>(c->iwi), collapse_scale(), c->bt,
+        c->btb, c->r0, c->xb, nullptr);
     k_off_finish<<<(unsigned)sets, 512, coll_smem, st>>>(c->r0, c->xb, 0, c->vm, c->fw, c->fwp, c->iw, c->iwp, c->bth,
                                                          c->a_hat);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "offline kernels");
