@@ -486,6 +486,162 @@ __global__ void __launch_bounds__(F4_THREADS, STAGE ? 2 : 3)
     if (in_bounds(o + RESULT_BYTES <= ext.resp_bytes, kSiteFoldResp)) switch_keep(S_AT, t, resp + o);
 }
 
+// One chain per cluster of four CTAs of 256 threads: CTA (l, r) transforms the three digits of
+// row r of s in limb l, multiplies them with the matching bodies and forms output row r of limb
+// l.  Two exchanges through distributed shared memory per step: the half of each product that
+// belongs to the other row (CTA (l, 0) sends its row-1 sum, CTA (l, 1) its row-0 digit sum),
+// then the residues of row r between the two limbs, which both compose s (thread t keeps the
+// 8 coefficients of layout A).  A step is a chain of dependent transforms, so with few chains
+// the time is its latency: here it holds one forward batch and one single inverse transform
+// where k_fold4 runs four and four, and each CTA has an SM's schedulers for itself.
+// 31 steps of up to 32 chains: 174 us (5.6 us a step), against 482 us for k_fold4; from about
+// 0.4 chains per SM on it is bound by issue like k_fold4, at a fifth more work per chain (both
+// limbs' CTAs compose s), so the server picks the form by the number of chains.
+// Shared memory: exchange buffer 24 KB, bodies and row 0 / S staged by cp.async 32 KB, the two
+// exchange slots 16 KB.
+constexpr int FC_SMEM = (3 + 4 + 2) * N * 4;
+
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
+    k_fold_cluster(const uint32_t* __restrict__ row0s, const uint32_t* __restrict__ gsw,
+                   const uint64_t* __restrict__ a_hat, const uint32_t* __restrict__ S, int64_t s_payload_stride,
+                   const uint64_t* __restrict__ cvec, const uint2* __restrict__ fwi, const uint2* __restrict__ iwi,
+                   int interp, int64_t db_cols, int qpp, uint8_t* __restrict__ resp, int64_t resp_payload_stride,
+                   int64_t resp_query_stride, FoldExtents ext) {
+    extern __shared__ uint4 fc_smem[];
+    uint32_t* xbuf = reinterpret_cast<uint32_t*>(fc_smem);  // [3][N]
+    uint32_t* stg = xbuf + 3 * N;                           // [4][N]: bodies of digits 0..2, row 0 or S
+    uint32_t* ex1 = stg + 4 * N;                            // [8][256] from CTA (l, 1 - r)
+    uint32_t* ex2 = ex1 + N;                                // [8][256] from CTA (1 - l, r)
+    const int t = threadIdx.x;
+    const int rank = (int)umma::cluster_rank(), l = rank & 1, r = rank >> 1;
+    const int wp = blockIdx.x >> 2, qg = blockIdx.y;
+    const uint32_t q = l ? Q1 : Q0;
+    const uint2 *fw = fwi + l * N, *iw = iwi + l * N;
+    const int payload = qg / qpp, qin = qg % qpp;
+    const uint32_t* Sq = S + (int64_t)payload * s_payload_stride;
+    const uint64_t* pk_src = r ? cvec + (int64_t)qg * db_cols : a_hat;  // row r of the packed ciphertexts
+    const uint32_t* gq = gsw + (int64_t)qg * 12 * N;
+    const int z8 = 8 * t;
+    const uint64_t mask = (1ull << GADGET_BITS) - 1;
+    const int64_t s_off = (int64_t)payload * s_payload_stride;
+    auto s_ok = [&](int64_t row) { return in_bounds(s_off + (row + 1) * N <= ext.s_words, kSiteFoldS); };
+    auto pk_ok = [&](int j) {
+        return r ? in_bounds((int64_t)qg * db_cols + ((int64_t)j + 1) * N <= ext.c_words, kSiteFoldC)
+                 : in_bounds(((int64_t)j + 1) * N <= ext.ahat_words, kSiteFoldAhat);
+    };
+    uint64_t x[EPT];   // s, row r: coefficients t + 256 m
+    uint32_t pr[EPT];  // N^-1 times output row r of limb l
+    uint64_t pk[EPT];
+    auto load_pk = [&](int j) {
+        const bool ok = pk_ok(j);
+#pragma unroll
+        for (int m = 0; m < EPT; m++) pk[m] = ok ? __ldg(pk_src + (int64_t)j * N + eA(t, m)) : 0;
+    };
+    // pr -> x: inverse transform, residues of the other limb, CRT, + packed row
+    auto to_s = [&]() {
+        inverse_one(pr, t, xbuf, 1, iw, q);
+#pragma unroll
+        for (int m = 0; m < EPT; m++) st_peer(ex2 + m * 256 + t, rank ^ 1, pr[m]);
+        umma::cluster_sync();
+#pragma unroll
+        for (int m = 0; m < EPT; m++) {
+            const uint32_t o = ex2[m * 256 + t];
+            x[m] = add_q(l ? crt2m(o, pr[m]) : crt2m(pr[m], o), pk[m]);
+        }
+    };
+    umma::cluster_sync();  // every CTA of the cluster runs: its shared memory may be written
+    {  // first step: G^-1(0) = 0, so s = (a_hat[j], INTT(S[j]) + c[j]) mod q
+        const int j = wp * interp + interp - 1;
+        load_pk(j);
+#pragma unroll
+        for (int m = 0; m < EPT; m++) pr[m] = 0;
+        if (r && s_ok((int64_t)j * 2 + l)) load_d8(pr, Sq + ((int64_t)j * 2 + l) * N + z8);
+        to_s();
+    }
+    for (int step = interp - 2; step >= 0; step--) {
+        const int j = wp * interp + step;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const int64_t row = (int64_t)qg * 12 + (r + 2 * k) * 2 + l;
+            if (!in_bounds((row + 1) * N <= ext.gsw_words, kSiteFoldGsw)) continue;
+            const uint32_t* src = gq + (int64_t)((r + 2 * k) * 2 + l) * N + z8;
+            cp16(stg + k * N + z8, src);
+            cp16(stg + k * N + z8 + 4, src + 4);
+        }
+        if (!r || s_ok((int64_t)j * 2 + l)) {
+            const uint32_t* src = r ? Sq + ((int64_t)j * 2 + l) * N + z8 : row0s + l * N + z8;
+            cp16(stg + 3 * N + z8, src);
+            cp16(stg + 3 * N + z8 + 4, src + 4);
+        }
+        cp_commit();
+        uint32_t v[3][EPT];
+#pragma unroll
+        for (int m = 0; m < EPT; m++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) v[k][m] = (uint32_t)((x[m] >> (k * GADGET_BITS)) & mask);
+        forward_digits<3>(v, t, xbuf, 1, fw, q);
+        load_pk(j);
+        cp_wait<0>();
+        uint32_t acc0[EPT], acc1[EPT];  // digit sum (< 6q), Montgomery-reduced product (< 2q)
+        {
+            uint64_t part[EPT];
+#pragma unroll
+            for (int m = 0; m < EPT; m++) {
+                acc0[m] = 0;
+                part[m] = 0;
+            }
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const uint4 b0 = *reinterpret_cast<const uint4*>(stg + k * N + z8);
+                const uint4 b1 = *reinterpret_cast<const uint4*>(stg + k * N + z8 + 4);
+                const uint32_t bv[EPT] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+                for (int m = 0; m < EPT; m++) {
+                    acc0[m] += v[k][m];
+                    part[m] += (uint64_t)bv[m] * v[k][m];  // 3 terms < 6 q^2 < q 2^32
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < EPT; m++) acc1[m] = redc(part[m], q);
+        }
+#pragma unroll
+        for (int m = 0; m < EPT; m++) st_peer(ex1 + m * 256 + t, rank ^ 2, r ? acc0[m] : acc1[m]);
+        umma::cluster_sync();
+        const uint4 e0 = *reinterpret_cast<const uint4*>(stg + 3 * N + z8);
+        const uint4 e1 = *reinterpret_cast<const uint4*>(stg + 3 * N + z8 + 4);
+        const uint32_t ev[EPT] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+#pragma unroll
+        for (int m = 0; m < EPT; m++) {
+            const uint32_t o = ex1[m * 256 + t];
+            if (r) pr[m] = csub(csub(csub(acc1[m] + o + ev[m], 4 * q), 2 * q), q);  // < 5q
+            else pr[m] = csub(redc((uint64_t)ev[m] * (acc0[m] + o), q), q);         // < 12 q^2 < q 2^32
+        }
+        to_s();
+    }
+    // switch_and_keep of row r, as switch_keep; the two limbs' CTAs take half of the fields each
+    const int64_t ro = (int64_t)payload * resp_payload_stride + 8 + (int64_t)qin * resp_query_stride +
+                       (int64_t)wp * RESULT_BYTES;
+    if (!in_bounds(ro + RESULT_BYTES <= ext.resp_bytes, kSiteFoldResp)) return;
+    uint8_t* out = resp + ro;
+#pragma unroll
+    for (int mm = 0; mm < EPT / 2; mm++) {
+        const int m = l * (EPT / 2) + mm;
+        const uint64_t a = rescale_q(l ? x[EPT / 2 + mm] : x[mm], r ? QP1 : QP2);
+        const uint64_t an = __shfl_down_sync(0xffffffffu, a, 1);
+        if (t & 1) continue;
+        const int tt = eA(t, m) >> 1;
+        if (r) {
+            const uint64_t w = a | (an << 20);
+#pragma unroll
+            for (int b = 0; b < 5; b++) out[7 * N / 2 + 5 * tt + b] = (uint8_t)(w >> (8 * b));
+        } else {
+            const uint64_t w = a | (an << 28);
+#pragma unroll
+            for (int b = 0; b < 7; b++) out[7 * tt + b] = (uint8_t)(w >> (8 * b));
+        }
+    }
+}
+
 // RGSW bodies 96 KB + two team exchange buffers of 4 polynomials (2 x 32 KB) + the two
 // teams' s (2 x 32 KB) = 224 KB
 constexpr int FOLD3_SMEM = (12 + 2 * XP) * N * 4 + 2 * 2 * N * 8;
@@ -494,6 +650,8 @@ cudaError_t init_fold3_kernel() {
     cudaError_t e = cudaFuncSetAttribute(k_fold3, cudaFuncAttributeMaxDynamicSharedMemorySize, FOLD3_SMEM);
     if (e != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_fold4<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, F4_SMEM)) != cudaSuccess)
+        return e;
+    if ((e = cudaFuncSetAttribute(k_fold_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, FC_SMEM)) != cudaSuccess)
         return e;
     return cudaFuncSetAttribute(k_fold4<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, F4_SMEM_UNSTAGED);
 }
@@ -540,7 +698,7 @@ cudaError_t launch_fold4(const uint32_t* row0s, const uint32_t* gsw_scaled, cons
                          int64_t s_payload_stride, const uint64_t* cvec, const uint32_t* fwi, const uint32_t* iwi,
                          int interp, int c_groups, int num_queries, int64_t db_cols, int qpp, uint8_t* resp,
                          int64_t resp_payload_stride, int64_t resp_query_stride, const FoldExtents& ext,
-                         cudaStream_t st, bool staged) {
+                         cudaStream_t st, FoldForm form) {
     if (interp < 1 || c_groups < 1 || num_queries < 1 || num_queries > 65535 || qpp < 1) return cudaErrorInvalidValue;
     cudaError_t e;
     if ((e = check_extent(row0s, 2ull * N * 4, "fold: row 0")) != cudaSuccess ||
@@ -552,17 +710,20 @@ cudaError_t launch_fold4(const uint32_t* row0s, const uint32_t* gsw_scaled, cons
         (e = check_extent(iwi, 2ull * N * 8, "fold: inverse twiddles")) != cudaSuccess ||
         (e = check_extent(resp, (uint64_t)ext.resp_bytes, "fold: responses")) != cudaSuccess)
         return e;
-    dim3 grid(c_groups, num_queries);
-    if (staged)
-        k_fold4<true><<<grid, F4_THREADS, F4_SMEM, st>>>(
-            row0s, gsw_scaled, a_hat, S, s_payload_stride, cvec, reinterpret_cast<const uint2*>(fwi),
-            reinterpret_cast<const uint2*>(iwi), interp, c_groups, db_cols, qpp, resp, resp_payload_stride,
-            resp_query_stride, ext);
+    const uint2 *fw = reinterpret_cast<const uint2*>(fwi), *iw = reinterpret_cast<const uint2*>(iwi);
+    const dim3 grid(c_groups, num_queries);
+    if (form == FoldForm::kCluster)
+        k_fold_cluster<<<dim3(4 * c_groups, num_queries), 256, FC_SMEM, st>>>(
+            row0s, gsw_scaled, a_hat, S, s_payload_stride, cvec, fw, iw, interp, db_cols, qpp, resp,
+            resp_payload_stride, resp_query_stride, ext);
+    else if (form == FoldForm::kStaged)
+        k_fold4<true><<<grid, F4_THREADS, F4_SMEM, st>>>(row0s, gsw_scaled, a_hat, S, s_payload_stride, cvec, fw, iw,
+                                                         interp, c_groups, db_cols, qpp, resp, resp_payload_stride,
+                                                         resp_query_stride, ext);
     else
         k_fold4<false><<<grid, F4_THREADS, F4_SMEM_UNSTAGED, st>>>(
-            row0s, gsw_scaled, a_hat, S, s_payload_stride, cvec, reinterpret_cast<const uint2*>(fwi),
-            reinterpret_cast<const uint2*>(iwi), interp, c_groups, db_cols, qpp, resp, resp_payload_stride,
-            resp_query_stride, ext);
+            row0s, gsw_scaled, a_hat, S, s_payload_stride, cvec, fw, iw, interp, c_groups, db_cols, qpp, resp,
+            resp_payload_stride, resp_query_stride, ext);
     return cudaGetLastError();
 }
 

@@ -124,18 +124,25 @@ int ensure_scratch(ipr_server* s, unsigned nq) {
     return IPR_OK;
 }
 
-// The one-chain fold's occupancy for `chains` chains: two CTAs per SM staging the RGSW bodies
-// in shared memory, or three per SM reading them from L2 (more warps to hide latency, 80
-// registers).  Chains run in rounds of (CTAs per SM x SMs); a round of three per SM takes
-// about 1.22x as long as one of two per SM (measured at the 1M shape), so the three-per-SM
-// form wins where it needs fewer rounds in proportion, e.g. 1,408 chains (64 payloads) on
-// 148 SMs: 4 rounds x 1.22 against 5 rounds.  Forms 4 / 5 force one occupancy.
-bool fold_staged(const ipr_server* s, int chains) {
-    if (s->fold_mode == 4) return false;
-    if (s->fold_mode == 5) return true;
-    const int sm = s->sm_count > 0 ? s->sm_count : 1;
-    const int64_t r2 = (chains + 2 * sm - 1) / (2 * sm), r3 = (chains + 3 * sm - 1) / (3 * sm);
-    return r3 * 122 >= r2 * 100;
+// The one-chain fold's form for `chains` chains, by predicted time.  Chains run in rounds of
+// (chains per SM x SMs).  In hundredths of a round of two chains per SM staging the RGSW bodies
+// in shared memory (820 us for 31 steps):
+//   two per SM, staged       100 a round, 60 for a last round of at most one chain per SM (482 us)
+//   three per SM, bodies from L2 (more warps to hide latency, 80 registers)  122 a round
+//   four CTAs per chain      21 (174 us) while the chip is not full, then 76 per chain and SM
+// Measured at 148 SMs (us, staged form / four CTAs per chain): 32 chains 482 / 175, 64 482 / 285,
+// 96 482 / 411, 120 492 / 520, 162 808 / 671, 240 819 / 955, 384 1313 / 1586; 1,408 chains (64 payloads at
+// 1M) take 4 rounds of three per SM against 5 of two.  Forms 4 / 5 force one occupancy.
+ipr::FoldForm fold_form(const ipr_server* s, int chains) {
+    if (s->fold_mode == 4) return ipr::FoldForm::kThreePerSm;
+    if (s->fold_mode == 5) return ipr::FoldForm::kStaged;
+    const int64_t sm = s->sm_count > 0 ? s->sm_count : 1;
+    const int64_t rest = chains % (2 * sm);
+    const int64_t staged = chains / (2 * sm) * 100 + (rest == 0 ? 0 : (rest <= sm ? 60 : 100));
+    const int64_t three = (chains + 3 * sm - 1) / (3 * sm) * 122;
+    const int64_t cluster = chains * 76 / sm > 21 ? chains * 76 / sm : 21;
+    if (cluster < staged && cluster < three) return ipr::FoldForm::kCluster;
+    return three >= staged ? ipr::FoldForm::kStaged : ipr::FoldForm::kThreePerSm;
 }
 
 // enqueue the device pipeline for one payload; `prof` = event slot base or -1
@@ -185,7 +192,7 @@ int enqueue(ipr_server* s, unsigned nq, const uint8_t* d_query, uint8_t* d_resp,
                 CU(ipr::launch_fold4(s->d_row0m, s->d_gsw, s->d_ahat, s->d_S, 0, s->d_c, s->d_fwi, s->d_iwi,
                                      (int)p.interp, (int)p.c, (int)nq, (int64_t)p.db_cols, (int)nq, d_resp, 0,
                                      (int64_t)(4 + s->per_query_bytes()), ext, st,
-                                     fold_staged(s, (int)(nq * p.c))));
+                                     fold_form(s, (int)(nq * p.c))));
             }
             else
                 CU(ipr::launch_fold3(s->d_row0s, s->d_gsw, s->d_ahat, s->d_S, 0, s->d_c, s->d_fwi, s->d_iwi,
@@ -343,7 +350,7 @@ int enqueue_batch(ipr_server* s, int B, const uint8_t* d_queries, uint8_t* d_res
             if (ipr::kBoundsChecked) ext.s_words -= ipr::g_fold_extent_cut.load();
             CU(ipr::launch_fold4(s->d_row0m, s->d_gsw, s->d_ahat, s->d_bS, (int64_t)(p.instances * 2 * kN), s->d_c,
                                  s->d_fwi, s->d_iwi, (int)p.interp, (int)p.c, nqt, (int64_t)p.db_cols, 2, d_resps, rb,
-                                 (int64_t)(4 + s->per_query_bytes()), ext, st, fold_staged(s, (int)(nqt * p.c))));
+                                 (int64_t)(4 + s->per_query_bytes()), ext, st, fold_form(s, (int)(nqt * p.c))));
         }
         else
             CU(ipr::launch_fold3(s->d_row0s, s->d_gsw, s->d_ahat, s->d_bS, (int64_t)(p.instances * 2 * kN), s->d_c,

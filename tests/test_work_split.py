@@ -58,3 +58,54 @@ def test_raw_db_forms(pkg, orc, rows, per, entry, shift):
     got = d_raw.cpu().numpy().view(np.uint16)
     assert np.array_equal(got[shift // 2:shift // 2 + want.size], want)
     assert (np.delete(got, np.s_[shift // 2:shift // 2 + want.size]) == 7).all()
+
+
+@pytest.mark.parametrize("groups,queries", [(1, 1), (28, 4), (30, 4), (25, 6), (25, 8)])
+def test_fold_form_by_chains(pkg, orc, groups, queries):
+    """1 and 112 chains on clusters, 120 on two chains per SM, 150 on clusters, 200 on two per SM"""
+    plan = _plan(pkg, 2 * groups, interp=2)
+    with pkg.KeywordServer.synthetic(plan, seed=500 + groups) as srv:
+        q = orc.synth_query(29 + queries, plan.db_rows, queries)
+        got = srv.respond_to_serialized_query(q)
+        for g in {0, groups - 1}:
+            want = orc.respond(orc.SynthDB.shard_of(plan.db_rows, 2 * g, 2, 2, 1, seed=500 + groups), q)
+            for query in range(queries):
+                assert _group(got, plan.c, query, g) == _group(want, 1, query, 0)
+
+
+def test_collapse_with_given_rows_matches_oracle(pkg, orc):
+    """the collapse fed with W rows as arrays (the FFI's form) gives the oracle's precomputation"""
+    import numpy as np
+    from test_compat_offline import CC, HALF, _bind, _d2h, _dev, _free, _packing_tables
+    lib, P = _bind(pkg.lib), orc.params()
+    db = np.random.default_rng(6).integers(0, 65535, N * N, dtype=np.uint16)
+    a_hat, bt, btb, bth = orc.offline_precompute(db, N, 1)
+    tables = np.ctypeslib.as_array(P.ntt).reshape(-1).astype(np.uint64).copy()
+    mono, idx, idxb, mod_inv = _packing_tables(orc)
+    a_ct = np.ascontiguousarray(orc.prep_pack(db, N, 0, orc.hint_query(1)).reshape(N, CC))
+    _, vm, wa, wb = orc.offline_keys()
+    wa, wb, vm = (np.ascontiguousarray(x, dtype=np.uint64).reshape(-1) for x in (wa, wb, vm))
+    auto = np.stack([orc.automorph_table(2 * t + 1) for t in range(N)]).astype(np.uint32)
+    gen = np.array([orc.gen_pow(i) for i in range(HALF)], dtype=np.uint32)
+    ptrs = d_auto, d_gen, d_act = _dev(auto), _dev(gen), _dev(a_ct)
+    try:
+        lib.gpu_packing_setup(mono.ctypes.data, idx.ctypes.data, idxb.ctypes.data, mod_inv.ctypes.data, HALF, N, N, 2,
+                              P.q[0], P.q[1], P.barrett_cr1[0], P.barrett_cr1[1])
+        lib.gpu_collapse_alloc_r(1, HALF, CC)
+        lib.gpu_packing_precomp_fast_device_no_d2h(d_act)
+        lib.gpu_collapse_automorph_column(lib.gpu_packing_get_s_r_out(), lib.gpu_packing_get_s_r_bar_out(), 0, HALF, CC,
+                                          N, 2, d_auto, d_gen, N)
+        lib.gpu_collapse_setup(wa.ctypes.data, wb.ctypes.data, vm.ctypes.data, tables.ctypes.data, 1, HALF, 3, CC)
+        lib.gpu_collapse_run(1, HALF, 3, 19, P.q[0], P.q[1], P.barrett_cr1[0], P.barrett_cr1[1], P.mod0_inv_mod1,
+                             P.mod1_inv_mod0, P.modulus, P.cr0_mod, P.cr1_mod)
+        got_a = np.zeros(N, dtype=np.uint64)
+        lib.gpu_collapse_download_a_hat(got_a.ctypes.data, 1)
+        got = (got_a, _d2h(lib.gpu_collapse_get_bold_t(), 3069 * N), _d2h(lib.gpu_collapse_get_bold_t_bar(), 3069 * N),
+               _d2h(lib.gpu_collapse_get_bold_t_hat(), 3 * N))
+        lib.gpu_collapse_free_all()
+        lib.gpu_packing_teardown()
+    finally:
+        for p in ptrs:
+            _free(p)
+    for name, w, g in zip(("a_hat", "bold_t", "bold_t_bar", "bold_t_hat"), (a_hat, bt, btb, bth), got):
+        assert np.array_equal(np.asarray(w).reshape(-1), g), name
