@@ -871,7 +871,7 @@ def main():
     pack_ms = stage_ms["pack"] / max(calls, 1)
     if B > 1:  # the packing GEMM streams the slot-indexed precomputation once per batch
         pack_bytes = N * 2 * ((local.instances + 31) // 32) * 128 * 3 * N  # [slot][limb][tile][128 rows][6144]
-        kname = "k_pack_mma_pair" if min(B, PASS) >= 48 else "k_pack_mma"  # the server's default choice of form
+        kname = "k_pack_mma"
     else:
         pack_bytes = local.instances * (2 * 3069 + 3) * N * 8  # bold_t + bold_t_bar + bold_t_hat per launch
         kname = "k_pack"

@@ -200,10 +200,10 @@ int ipr_server_set_profiling(ipr_server *srv, int on);
  * 0 = shared-memory NTTs after that pass (single-payload calls only; batches then
  * use form 1).  Identical results. */
 #define IPR_OPT_FOLD_REGISTER_NTT 2
-/* IPR_OPT_PACK_CTA_PAIR: 1 = the batch path's packing GEMM runs on CTA pairs
- * (tcgen05 cta_group::2, M = 256 across two SMs); 0 = one CTA per unit;
- * 2 (default) = pairs from 48 payloads per batch up, where they are faster.
- * Identical results. */
+/* IPR_OPT_PACK_CTA_PAIR: 0, 1 or 2 (default).  Accepted for callers that set it; the batch
+ * path's packing GEMM runs on one CTA per unit under every value.  (A form on CTA pairs,
+ * tcgen05 cta_group::2, was taken out: with batches of several databases overlapping on the
+ * device it did not finish.) */
 #define IPR_OPT_PACK_CTA_PAIR 3
 /* IPR_OPT_GEMV_TILE: cap on the first-dimension GEMM's query-byte tile height
  * (16, 32, 64, 128 or 256; 0 = 256, the default).  A query takes 7 byte rows (the bytes
@@ -236,7 +236,7 @@ int ipr_server_set_option(ipr_server *srv, int option, int64_t value);
 #define IPR_AUTOTUNE_MAX 8
 typedef struct {
     int candidates;                    /* how many were timed */
-    int pack_cta_pair[IPR_AUTOTUNE_MAX];
+    int pack_cta_pair[IPR_AUTOTUNE_MAX]; /* the option's value; no effect on the work */
     int gemv_tile[IPR_AUTOTUNE_MAX];
     double ms[IPR_AUTOTUNE_MAX];       /* mean device time per batch of `payloads` */
     int chosen;                        /* index of the candidate now in force */

@@ -326,17 +326,11 @@ int enqueue_batch(ipr_server* s, int B, const uint8_t* d_queries, uint8_t* d_res
     rec(2);
     {
         const int nt = ipr::pack_mma_nt(B);
-        const bool pair = s->pack_pair == 1 || (s->pack_pair == 2 && B >= 48);
         const CUtensorMap* ty;
-        int e = y8_map(s, pair ? nt / 2 : nt, &ty);  // the pair form loads half the client rows per CTA
+        int e = y8_map(s, nt, &ty);
         if (e) return e;
         CU(ipr::launch_build_y8(s->d_ybs, s->d_y8, B, s->y8_np, st));
-        if (pair)
-            CU(ipr::launch_pack_mma_pair(&s->tm_tpp, ty, (int)p.instances, B, s->y8_np, s->d_bS, s->d_err, s->sm_count,
-                                         st));
-        else
-            CU(ipr::launch_pack_mma(&s->tm_tpp, ty, (int)p.instances, B, s->y8_np, s->d_bS, s->d_err, s->sm_count,
-                                    st));
+        CU(ipr::launch_pack_mma(&s->tm_tpp, ty, (int)p.instances, B, s->y8_np, s->d_bS, s->d_err, s->sm_count, st));
     }
     rec(3);
     if (s->fold_mode >= 2) {
@@ -434,7 +428,6 @@ int init_common(ipr_server* s, int device, const ipr_plan* plan) {
     CU(ipr::init_fold2_kernel());
     CU(ipr::init_fold3_kernel());
     CU(ipr::init_pack_mma_kernel());
-    CU(ipr::init_pack_pair_kernel());
     ipr::host_params_init(s->hp);
     CU(ipr::set_constants(s->hp.barrett, s->hp.q0_inv_mod_q1));
     int st;
@@ -1007,9 +1000,9 @@ int ipr_server_autotune(ipr_server* s, int payloads, int reps, ipr_autotune_resu
     }
     CU(cudaMemcpyAsync(s->d_bq, s->h_bq, (size_t)payloads * qb, cudaMemcpyHostToDevice, s->stream));
     const int old_pair = s->pack_pair, old_tile = s->g1_tile;
-    // CTA pairs pay off only for large batches, so the automatic threshold (2) competes with
-    // pairs never (0) and always (1), and every candidate is timed at the requested batch
-    // size and at a quarter of it: the score is the device time per payload summed over both
+    // every value of the packing option is listed although all run the same kernel; every candidate
+    // is timed at the requested batch size and at a quarter of it: the score is the device time
+    // per payload summed over both
     static const int pairs[] = {2, 0, 1}, tiles[] = {0, 128};
     *out = ipr_autotune_result{};
     for (int pr : pairs)

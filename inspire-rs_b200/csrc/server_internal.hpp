@@ -47,7 +47,7 @@ struct ipr_server {
                                // CTAs per SM by chain count (4: three, 5: two), 2 fused fold
                                // on two chains per CTA (k_fold_prep + k_fold3), 1 k_intt_crt + k_fold2,
                                // 0 smem fold
-    int pack_pair = 2;         // batch packing GEMM on CTA pairs: 0 never, 1 always, 2 from 48 payloads up
+    int pack_pair = 2;         // IPR_OPT_PACK_CTA_PAIR as set (no effect)
     int g1_tile = 0;           // first-dimension GEMM query-byte tile height cap (0 = 256)
     int gemv_form = 6;         // form of the CUDA-core GEMV (IPR_OPT_GEMV_FORM)
     std::map<int, CUtensorMap> tm_qb;  // per query-byte tile height

@@ -109,7 +109,7 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {  //
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  // one full warp
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
 }
-// ---- CTA pairs (cta_group::2): one MMA spans the tensor cores of two SMs ----------------
+// ---- clusters ------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -124,44 +124,6 @@ __device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
     return r;
 }
-// arrive on a barrier of either CTA of the pair (default release semantics: no cluster-wide
-// fence, which per k-step or per unit would stall the issuing warp)
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// M = 256 across the pair: A rows 0..127 and B rows 0..N/2-1 from this CTA's shared memory,
-// the rest from the peer's at the same offsets; D rows 128 r .. 128 r + 127 in CTA r's TMEM
-__device__ __forceinline__ void mma_u8_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
-}
-// arrive on the mbarrier at `cluster_addr` (this CTA's or the peer's) once the pair's MMAs
-// issued so far complete; one commit per barrier to be signalled
-__device__ __forceinline__ void commit_pair(uint32_t cluster_addr) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr)
-                 : "memory");
-}
-// tile load into this CTA's shared memory whose completion is counted on an mbarrier of the
-// pair (`mbar_cluster_addr`, e.g. the leader's)
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y,
-                                                 uint32_t mbar_cluster_addr) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
-        "%3}], [%4];" ::"r"(smem_addr(dst)),
-        "l"(map), "r"(x), "r"(y), "r"(mbar_cluster_addr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {  // warp w of both CTAs
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)), "r"(ncols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
-}
-
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 

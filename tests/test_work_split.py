@@ -34,6 +34,20 @@ def test_single_payload_packing_split(pkg, orc, instances):
                 assert _group(got, plan.c, query, g) == _group(want, 1, query, 0)
 
 
+@pytest.mark.parametrize("instances", [1, 3])
+@pytest.mark.parametrize("payloads", [2, 4, 5, 20, 33, 64])
+def test_batch_packing_tiles(pkg, orc, instances, payloads):
+    """one to sixteen column groups of four clients, fewer units than SMs and more"""
+    plan = _plan(pkg, instances)
+    seed = 700 + instances
+    with pkg.KeywordServer.synthetic(plan, seed=seed) as srv:
+        qs = [orc.synth_query(900 + i, plan.db_rows, 2) for i in range(payloads)]
+        got = srv.respond_batch(qs)
+        sdb = orc.SynthDB(plan.db_rows, instances, 1, instances, seed=seed)
+        for i in {0, payloads // 2, payloads - 1}:
+            assert got[i] == orc.respond(sdb, qs[i])
+
+
 @pytest.mark.parametrize("rows,per,entry,shift", [
     (2048, 2, 1216, 0),   # whole 64-row tiles, a last chunk of 192 bytes
     (64, 3, 256, 0), (72, 2, 272, 0), (8, 5, 16, 0),    # one chunk, chunk + 16 bytes, ragged row tile, smallest
