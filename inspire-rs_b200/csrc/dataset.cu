@@ -14,8 +14,11 @@
 // is derived on the host.  Keccak-f[1600] round constants and rotation offsets come from
 // FIPS 202's definitions (the rc(t) LFSR, the (t+1)(t+2)/2 rho offsets).
 //
-// One thread per record: a record is ~45 Keccak-f permutations, six or eight 256-point
-// NTTs mod 3329 and k^2 base-case products, small enough for local memory.
+// Two kernels.  k_dataset_keys gives each SHAKE stream of a record (k^2 matrix entries, 2k noise
+// polynomials) a thread of its own with the Keccak state in registers, collects the sampled
+// polynomials of a few records in shared memory, and transforms and multiplies them there a
+// warp per polynomial; k_dataset_ids hashes one record per thread.  Both are bound by Keccak
+// instruction issue.  DATASET_FIGURES
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -28,11 +31,53 @@ namespace ipr {
 
 namespace {
 
-__constant__ uint64_t c_keccak_rc[24];
-__constant__ int16_t c_zeta[128];   // 17^BitRev7(i) mod 3329
-__constant__ int16_t c_gamma[128];  // 17^(2 BitRev7(i) + 1) mod 3329
-
 constexpr int MQ = 3329;
+
+// FIPS 202 Algorithm 5, bit i of r holds R[i]
+constexpr int rc_bit(int t) {
+    if (t % 255 == 0) return 1;
+    unsigned r = 1;
+    for (int i = 1; i <= t % 255; i++) {
+        r <<= 1;
+        r ^= ((r >> 8) & 1) * 0x71u;
+        r &= 0xFF;
+    }
+    return r & 1;
+}
+constexpr int brv7(int x) {
+    int r = 0;
+    for (int i = 0; i < 7; i++) r |= ((x >> i) & 1) << (6 - i);
+    return r;
+}
+constexpr int pow17(int e) {
+    int r = 1, b = 17;
+    for (; e; e >>= 1, b = b * b % MQ)
+        if (e & 1) r = r * b % MQ;
+    return r;
+}
+struct KeccakTable {
+    uint64_t rc[24];
+};
+constexpr KeccakTable keccak_table() {
+    KeccakTable t{};
+    for (int ir = 0; ir < 24; ir++)
+        for (int j = 0; j <= 6; j++)
+            if (rc_bit(j + 7 * ir)) t.rc[ir] |= 1ull << ((1 << j) - 1);
+    return t;
+}
+struct MlkemTable {
+    uint16_t zeta[128], gamma[128];  // 17^BitRev7(i), 17^(2 BitRev7(i) + 1) mod 3329
+};
+constexpr MlkemTable mlkem_table() {
+    MlkemTable t{};
+    for (int i = 0; i < 128; i++) {
+        t.zeta[i] = (uint16_t)pow17(brv7(i));
+        t.gamma[i] = (uint16_t)pow17(2 * brv7(i) + 1);
+    }
+    return t;
+}
+__constant__ KeccakTable c_keccak = keccak_table();
+__device__ const MlkemTable d_mlkem = mlkem_table();
 
 __host__ __device__ constexpr int rho_offset(int x, int y) {  // FIPS 202 Algorithm 2
     if (x == 0 && y == 0) return 0;
@@ -48,7 +93,7 @@ __host__ __device__ constexpr int rho_offset(int x, int y) {  // FIPS 202 Algori
 
 __device__ __forceinline__ uint64_t rotl64(uint64_t v, int n) { return n ? (v << n) | (v >> (64 - n)) : v; }
 
-__device__ void keccakf(uint64_t (&a)[25]) {
+__device__ __forceinline__ void keccakf(uint64_t (&a)[25]) {
 #pragma unroll 1
     for (int ir = 0; ir < 24; ir++) {
         uint64_t c[5], d[5], b[25];
@@ -67,47 +112,13 @@ __device__ void keccakf(uint64_t (&a)[25]) {
 #pragma unroll
             for (int y = 0; y < 5; y++)
                 a[x + 5 * y] = b[x + 5 * y] ^ (~b[(x + 1) % 5 + 5 * y] & b[(x + 2) % 5 + 5 * y]);
-        a[0] ^= c_keccak_rc[ir];
+        a[0] ^= c_keccak.rc[ir];
     }
 }
 
-// a Keccak sponge over one thread's state; rate in bytes
-struct Sponge {
-    uint64_t s[25];
-    int rate, pos;
-    __device__ void init(int r) {
-#pragma unroll
-        for (int i = 0; i < 25; i++) s[i] = 0;
-        rate = r;
-        pos = 0;
-    }
-    __device__ void absorb_byte(uint8_t v) {
-        s[pos >> 3] ^= (uint64_t)v << (8 * (pos & 7));
-        if (++pos == rate) {
-            keccakf(s);
-            pos = 0;
-        }
-    }
-    __device__ void finish(uint8_t ds) {  // pad10*1 with the domain bits
-        s[pos >> 3] ^= (uint64_t)ds << (8 * (pos & 7));
-        s[(rate - 1) >> 3] ^= 0x80ull << (8 * ((rate - 1) & 7));
-        keccakf(s);
-        pos = 0;
-    }
-    __device__ uint8_t squeeze_byte() {
-        if (pos == rate) {
-            keccakf(s);
-            pos = 0;
-        }
-        const uint8_t v = (uint8_t)(s[pos >> 3] >> (8 * (pos & 7)));
-        pos++;
-        return v;
-    }
-};
-
 __device__ __forceinline__ uint32_t rotl32(uint32_t v, int n) { return (v << n) | (v >> (32 - n)); }
 
-__device__ void chacha20_block(const uint32_t key[8], uint64_t counter, uint8_t out[64]) {
+__device__ __forceinline__ void chacha20_block(const uint32_t key[8], uint64_t counter, uint32_t (&out)[16]) {
     uint32_t s[16], x[16];
     s[0] = 0x61707865u;
     s[1] = 0x3320646eu;
@@ -133,188 +144,306 @@ __device__ void chacha20_block(const uint32_t key[8], uint64_t counter, uint8_t 
         qr(0, 5, 10, 15); qr(1, 6, 11, 12); qr(2, 7, 8, 13); qr(3, 4, 9, 14);
     }
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-        const uint32_t v = x[i] + s[i];
+    for (int i = 0; i < 16; i++) out[i] = x[i] + s[i];
+}
+
+// x mod 3329 for x < 2^32: quotient by the high half of a product with floor(2^32 / 3329),
+// which is at most one too small, and one correction
+__device__ __forceinline__ uint32_t modq12(uint32_t x) {
+    constexpr uint32_t INV = (uint32_t)((1ull << 32) / MQ);
+    const uint32_t r = x - __umulhi(x, INV) * MQ;
+    return min(r, r - MQ);
+}
+
+// One CTA: R records.  Its first MW warps run the K*K matrix streams of all records, the next NW
+// warps the 2K noise streams, so that a warp's lanes take the same branch and the same number of
+// permutations (3 or 4 against 1, or 2 for eta 3).
+template <int K>
+struct Keys {
+    static constexpr int R = K == 2 ? 16 : (K == 3 ? 7 : 4);  // the matrix streams fill two warps
+    static constexpr int MW = (R * K * K + 31) / 32, NW = (R * 2 * K + 31) / 32;
+    static constexpr int THREADS = 32 * (MW + NW);
+    static constexpr int STREAMS = K * K + 2 * K;
+    static constexpr int ETA1 = K == 2 ? 3 : 2;
+    static constexpr int LD = 258;              // halfwords per polynomial: an odd word count, no bank conflicts
+    static constexpr int PK = 384 * K + 32, REC = 32 + PK;
+    uint16_t poly[R][STREAMS][LD];              // A[i][j] (i * K + j), then s[0..K), e[0..K)
+    uint64_t seed[R][8];                        // rho (4 words), sigma (4 words)
+};
+
+// eight coefficients of a polynomial in registers: layout B e = lane + 32 m, layout C
+// e = 32 (lane / 4) + 4 m + lane % 4, layout D e = 8 lane + m, so that every butterfly of FIPS 203
+// Algorithm 9 (NTT) pairs two registers
+__device__ __forceinline__ void mlkem_ntt_warp(uint16_t* f, int lane) {
+    uint32_t v[8];
+    auto layer = [&](int dd, int shift, int base, auto e) {  // zeta index base + (e >> shift)
 #pragma unroll
-        for (int b = 0; b < 4; b++) out[4 * i + b] = (uint8_t)(v >> (8 * b));
-    }
-}
-
-__device__ __forceinline__ int16_t red(int v) { return (int16_t)(v % MQ); }  // v >= 0
-
-// FIPS 203 Algorithm 9 (NTT), coefficients in [0, q)
-__device__ void mlkem_ntt(int16_t* f) {
-    int i = 1;
-#pragma unroll 1
-    for (int len = 128; len >= 2; len >>= 1)
-#pragma unroll 1
-        for (int start = 0; start < 256; start += 2 * len) {
-            const int zeta = c_zeta[i++];
-#pragma unroll 4
-            for (int j = start; j < start + len; j++) {
-                const int t = zeta * f[j + len] % MQ;
-                f[j + len] = red(f[j] - t + MQ);
-                f[j] = red(f[j] + t);
-            }
+        for (int m = 0; m < 8; m++) {
+            if (m & dd) continue;
+            const uint32_t z = d_mlkem.zeta[base + (e(m) >> shift)];
+            const uint32_t t = modq12(z * v[m + dd]);
+            const uint32_t a = v[m], lo = a + t, hi = a + MQ - t;
+            v[m] = min(lo, lo - MQ);
+            v[m + dd] = min(hi, hi - MQ);
         }
-}
-
-// FIPS 203 Algorithm 8 with PRF_eta(sigma, n) = SHAKE256(sigma || n) (64 eta bytes)
-__device__ void sample_cbd(const uint8_t sigma[32], int n, int eta, int16_t* f) {
-    Sponge sp;
-    sp.init(136);
-    for (int i = 0; i < 32; i++) sp.absorb_byte(sigma[i]);
-    sp.absorb_byte((uint8_t)n);
-    sp.finish(0x1F);
-    // eta = 2: one byte gives two coefficients; eta = 3: three bytes give four
-    if (eta == 2) {
-        for (int i = 0; i < 128; i++) {
-            const uint32_t b = sp.squeeze_byte();
-            const int x0 = (b & 1) + ((b >> 1) & 1), y0 = ((b >> 2) & 1) + ((b >> 3) & 1);
-            const int x1 = ((b >> 4) & 1) + ((b >> 5) & 1), y1 = ((b >> 6) & 1) + ((b >> 7) & 1);
-            f[2 * i] = red(x0 - y0 + MQ);
-            f[2 * i + 1] = red(x1 - y1 + MQ);
-        }
-    } else {
-        for (int i = 0; i < 64; i++) {
-            const uint32_t b = sp.squeeze_byte() | ((uint32_t)sp.squeeze_byte() << 8) |
-                               ((uint32_t)sp.squeeze_byte() << 16);
+    };
+    auto eb = [&](int m) { return lane + 32 * m; };
+    auto ec = [&](int m) { return 32 * (lane >> 2) + 4 * m + (lane & 3); };
+    auto ed = [&](int m) { return 8 * lane + m; };
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const uint32_t w = b >> (6 * c);
-                const int x = (w & 1) + ((w >> 1) & 1) + ((w >> 2) & 1);
-                const int y = ((w >> 3) & 1) + ((w >> 4) & 1) + ((w >> 5) & 1);
-                f[4 * i + c] = red(x - y + MQ);
-            }
-        }
-    }
+    for (int m = 0; m < 8; m++) v[m] = f[eb(m)];
+    layer(4, 8, 1, eb);  // length 128
+    layer(2, 7, 2, eb);
+    layer(1, 6, 4, eb);
+#pragma unroll
+    for (int m = 0; m < 8; m++) f[eb(m)] = (uint16_t)v[m];
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < 8; m++) v[m] = f[ec(m)];
+    layer(4, 5, 8, ec);  // length 16
+    layer(2, 4, 16, ec);
+    layer(1, 3, 32, ec);
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < 8; m++) f[ec(m)] = (uint16_t)v[m];
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < 8; m++) v[m] = f[ed(m)];
+    layer(2, 2, 64, ed);  // length 2
+#pragma unroll
+    for (int m = 0; m < 8; m++) f[ed(m)] = (uint16_t)v[m];
 }
 
-__global__ void __launch_bounds__(128) k_dataset(int k, uint4 key_lo, uint4 key_hi, uint64_t first, uint64_t count,
-                                                 uint8_t* __restrict__ out) {
-    const uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (r >= count) return;
-    const int pk_len = 384 * k + 32;
-    uint8_t* rec = out + r * (uint64_t)(32 + pk_len);
-    uint8_t* pk = rec + 32;
-    // record seed: ChaCha20 block number first + r
-    const uint32_t key[8] = {key_lo.x, key_lo.y, key_lo.z, key_lo.w, key_hi.x, key_hi.y, key_hi.z, key_hi.w};
-    uint8_t seed64[64];
-    chacha20_block(key, first + r, seed64);
-    // K-PKE.KeyGen (FIPS 203 Algorithm 13): (rho, sigma) = SHA3-512(d || k)
-    uint8_t rho[32], sigma[32];
+template <int K>
+__global__ void __launch_bounds__(Keys<K>::THREADS, 4)
+    k_dataset_keys(uint4 key_lo, uint4 key_hi, uint64_t first, uint64_t count, uint8_t* __restrict__ out, bool words) {
+    using C = Keys<K>;
+    extern __shared__ __align__(16) uint8_t ds_smem[];
+    C& sm = *reinterpret_cast<C*>(ds_smem);
+    const int t = threadIdx.x, lane = t & 31;
+    const uint64_t rec0 = (uint64_t)blockIdx.x * C::R;
+    const int live = (int)min((uint64_t)C::R, count - rec0);
+    if (t < live) {
+        // record seed: ChaCha20 block number first + record; its first half is d
+        const uint32_t key[8] = {key_lo.x, key_lo.y, key_lo.z, key_lo.w, key_hi.x, key_hi.y, key_hi.z, key_hi.w};
+        uint32_t blk[16];
+        chacha20_block(key, first + rec0 + t, blk);
+        // K-PKE.KeyGen (FIPS 203 Algorithm 13): (rho, sigma) = SHA3-512(d || k)
+        uint64_t a[25];
+#pragma unroll
+        for (int i = 0; i < 25; i++) a[i] = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) a[i] = (uint64_t)blk[2 * i] | ((uint64_t)blk[2 * i + 1] << 32);
+        a[4] = (uint64_t)K | (0x06ull << 8);
+        a[8] = 0x80ull << 56;  // byte 71, the last of the 72-byte rate
+        keccakf(a);
+#pragma unroll
+        for (int i = 0; i < 8; i++) sm.seed[t][i] = a[i];
+    }
+    __syncthreads();
     {
-        Sponge sp;
-        sp.init(72);
-        for (int i = 0; i < 32; i++) sp.absorb_byte(seed64[i]);
-        sp.absorb_byte((uint8_t)k);
-        sp.finish(0x06);
-        for (int i = 0; i < 32; i++) rho[i] = sp.squeeze_byte();
-        for (int i = 0; i < 32; i++) sigma[i] = sp.squeeze_byte();
-    }
-    const int eta1 = k == 2 ? 3 : 2;
-    int16_t s[4][256], t[256];
-    for (int i = 0; i < k; i++) {
-        sample_cbd(sigma, i, eta1, s[i]);
-        mlkem_ntt(s[i]);
-    }
-    for (int i = 0; i < k; i++) {
-        sample_cbd(sigma, k + i, eta1, t);  // e[i]
-        mlkem_ntt(t);
-        for (int j = 0; j < k; j++) {
-            // A_hat[i][j] = SampleNTT(SHAKE128(rho || j || i)) (Algorithm 7), consumed pairwise by
-            // the base-case products (Algorithms 11, 12) as it is sampled
-            Sponge sp;
-            sp.init(168);
-            for (int b = 0; b < 32; b++) sp.absorb_byte(rho[b]);
-            sp.absorb_byte((uint8_t)j);
-            sp.absorb_byte((uint8_t)i);
-            sp.finish(0x1F);
-            int have = 0, pend = 0;
-            while (have < 256) {
-                const int c0 = sp.squeeze_byte(), c1 = sp.squeeze_byte(), c2 = sp.squeeze_byte();
-                const int dv[2] = {c0 + 256 * (c1 & 15), (c1 >> 4) + 16 * c2};
+        const bool matrix = t < 32 * C::MW;
+        const int u = matrix ? t : t - 32 * C::MW, per = matrix ? K * K : 2 * K;
+        const int rec = u / per, st = matrix ? u % per : K * K + u % per;
+        if (rec < live) {
+            uint16_t* p = sm.poly[rec][st];
+            uint64_t a[25];
 #pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    if (dv[u] >= MQ || have >= 256) continue;
-                    if (have & 1) {  // coefficients 2p, 2p + 1 complete: add A_p * s_j,p
-                        const int p = have >> 1, a0 = pend, a1 = dv[u];
-                        const int b0 = s[j][2 * p], b1 = s[j][2 * p + 1];
-                        t[2 * p] = red(t[2 * p] + a0 * b0 % MQ + (a1 * b1 % MQ) * c_gamma[p] % MQ);
-                        t[2 * p + 1] = red(t[2 * p + 1] + a0 * b1 % MQ + a1 * b0 % MQ);
-                    } else {
-                        pend = dv[u];
+            for (int i = 0; i < 25; i++) a[i] = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = sm.seed[rec][matrix ? i : 4 + i];
+            if (matrix) {  // SampleNTT(SHAKE128(rho || j || i)) (Algorithm 7), rate 168
+                a[4] = (uint64_t)(st % K) | ((uint64_t)(st / K) << 8) | (0x1Full << 16);
+                a[20] = 0x80ull << 56;
+            } else {       // SamplePolyCBD(SHAKE256(sigma || n)) (Algorithm 8), rate 136
+                a[4] = (uint64_t)(st - K * K) | (0x1Full << 8);
+                a[16] = 0x80ull << 56;
+            }
+            int have = 0;
+            while (have < 256) {
+                keccakf(a);
+                if (matrix) {  // 21 words = 56 triples of bytes, two 12-bit candidates each
+#pragma unroll
+                    for (int g = 0; g < 7; g++) {
+                        const uint64_t w0 = a[3 * g], w1 = a[3 * g + 1], w2 = a[3 * g + 2];
+#pragma unroll
+                        for (int c = 0; c < 16; c++) {
+                            constexpr int B = 12;
+                            const int bit = B * c, w = bit >> 6, sh = bit & 63;
+                            const uint64_t lo = w == 0 ? w0 : (w == 1 ? w1 : w2), hi = w == 0 ? w1 : w2;
+                            const uint32_t v =
+                                (uint32_t)(sh <= 52 ? lo >> sh : (lo >> sh) | (hi << (64 - sh))) & 0xFFFu;
+                            if (v < MQ && have < 256) p[have++] = (uint16_t)v;
+                        }
                     }
-                    have++;
+                } else if (C::ETA1 == 2) {  // 16 words, a nibble per coefficient
+#pragma unroll
+                    for (int w = 0; w < 16; w++) {
+                        const uint64_t x = (a[w] & 0x5555555555555555ull) + ((a[w] >> 1) & 0x5555555555555555ull);
+#pragma unroll
+                        for (int c = 0; c < 16; c++) {
+                            const uint32_t n = (uint32_t)(x >> (4 * c)) & 15u;
+                            const uint32_t d = (n & 3u) + MQ - (n >> 2);
+                            p[16 * w + c] = (uint16_t)min(d, d - MQ);
+                        }
+                    }
+                    have = 256;
+                } else {  // eta 3: six bits per coefficient; 136 bytes of the first block, 56 of the second
+                    // coefficient c takes bits [6 c, 6 c + 6): 1088 bits of a block hold 181 and 2 bits
+                    const int c0 = have;
+                    auto put = [&](int c, uint32_t s6) {
+                        const uint32_t x = (s6 & 1) + ((s6 >> 1) & 1) + ((s6 >> 2) & 1);
+                        const uint32_t y = ((s6 >> 3) & 1) + ((s6 >> 4) & 1) + ((s6 >> 5) & 1);
+                        const uint32_t d = x + MQ - y;
+                        p[c] = (uint16_t)min(d, d - MQ);
+                    };
+                    if (c0 == 0) {
+#pragma unroll
+                        for (int c = 0; c < 181; c++) {
+                            const int bit = 6 * c, w = bit >> 6, sh = bit & 63;
+                            const uint64_t hi = a[w + 1 < 17 ? w + 1 : 16];
+                            put(c, (uint32_t)(sh <= 58 ? a[w] >> sh : (a[w] >> sh) | (hi << (64 - sh))) & 63u);
+                        }
+                        p[181] = (uint16_t)(a[16] >> 62);  // the two bits that the next block completes
+                        have = 181;
+                    } else {
+                        put(181, ((uint32_t)p[181] | ((uint32_t)a[0] << 2)) & 63u);
+#pragma unroll
+                        for (int c = 182; c < 256; c++) {
+                            const int bit = 6 * c - 1088, w = bit >> 6, sh = bit & 63;
+                            put(c, (uint32_t)(sh <= 58 ? a[w] >> sh : (a[w] >> sh) | (a[w + 1] << (64 - sh))) & 63u);
+                        }
+                        have = 256;
+                    }
                 }
             }
         }
-        for (int p = 0; p < 128; p++) {  // ByteEncode_12 (Algorithm 5)
-            const int c0 = t[2 * p], c1 = t[2 * p + 1];
-            pk[384 * i + 3 * p] = (uint8_t)c0;
-            pk[384 * i + 3 * p + 1] = (uint8_t)((c0 >> 8) | ((c1 & 15) << 4));
-            pk[384 * i + 3 * p + 2] = (uint8_t)(c1 >> 4);
+    }
+    __syncthreads();
+    for (int i = t >> 5; i < live * 2 * K; i += C::THREADS / 32)  // NTT of every s and e, a warp each
+        mlkem_ntt_warp(sm.poly[i / (2 * K)][K * K + i % (2 * K)], lane);
+    __syncthreads();
+    // t_i = sum_j A_ij s_j + e_i (base-case products, Algorithms 11 and 12), four coefficient
+    // pairs per thread, and ByteEncode_12 (Algorithm 5) of them: 12 bytes
+    for (int i = t; i < live * K * 32; i += C::THREADS) {
+        const int rec = i / (K * 32), row = i / 32 % K, p0 = (i % 32) * 4;
+        uint32_t o[3] = {0, 0, 0};
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int p = p0 + u;
+            const uint32_t gm = d_mlkem.gamma[p];
+            const uint16_t* e = sm.poly[rec][K * K + K + row];
+            uint32_t c0 = e[2 * p], c1 = e[2 * p + 1];
+#pragma unroll
+            for (int j = 0; j < K; j++) {
+                const uint16_t *A = sm.poly[rec][row * K + j], *s = sm.poly[rec][K * K + j];
+                const uint32_t a0 = A[2 * p], a1 = A[2 * p + 1], b0 = s[2 * p], b1 = s[2 * p + 1];
+                c0 += a0 * b0 + modq12(a1 * b1) * gm;  // each below q^2, at most 8 q^2 + q
+                c1 += a0 * b1 + a1 * b0;
+            }
+            const uint32_t w = modq12(c0) | (modq12(c1) << 12);  // 24 bits
+            if (u == 0) o[0] = w;
+            else if (u == 1) o[0] |= w << 24, o[1] = w >> 8;
+            else if (u == 2) o[1] |= w << 16, o[2] = w >> 16;
+            else o[2] |= w << 8;
+        }
+        uint8_t* dst = out + (rec0 + rec) * (uint64_t)C::REC + 32 + 384 * row + 3 * p0;
+        if (words) {
+#pragma unroll
+            for (int w = 0; w < 3; w++) reinterpret_cast<uint32_t*>(dst)[w] = o[w];
+        } else {
+            for (int b = 0; b < 12; b++) dst[b] = (uint8_t)(o[b >> 2] >> (8 * (b & 3)));
         }
     }
-    for (int b = 0; b < 32; b++) pk[384 * k + b] = rho[b];
-    // id = SHA3-256("pq-key:v1:" || kem_name || pk)
-    {
-        const char* name = k == 2 ? "ml-kem-512" : (k == 3 ? "ml-kem-768" : "ml-kem-1024");
-        const char* dom = "pq-key:v1:";
-        Sponge sp;
-        sp.init(136);
-        for (int i = 0; i < 10; i++) sp.absorb_byte((uint8_t)dom[i]);
-        for (int i = 0; name[i]; i++) sp.absorb_byte((uint8_t)name[i]);
-        for (int i = 0; i < pk_len; i++) sp.absorb_byte(pk[i]);
-        sp.finish(0x06);
-        for (int i = 0; i < 32; i++) rec[i] = sp.squeeze_byte();
+    for (int i = t; i < live * 32; i += C::THREADS) {
+        const int rec = i >> 5, b = i & 31;
+        out[(rec0 + rec) * (uint64_t)C::REC + 32 + 384 * K + b] = (uint8_t)(sm.seed[rec][b >> 3] >> (8 * (b & 7)));
     }
 }
 
-// host: FIPS 202 Algorithm 5, bit i of r holds R[i]
-int rc_bit(int t) {
-    if (t % 255 == 0) return 1;
-    unsigned r = 1;
-    for (int i = 1; i <= t % 255; i++) {
-        r <<= 1;
-        r ^= ((r >> 8) & 1) * 0x71u;
-        r &= 0xFF;
+// id = SHA3-256("pq-key:v1:" || kem_name || pk), one record per thread.  The prefix is 16 bytes
+// and PART more (4 for "-512" and "-768", 5 for "-1024"), so message word 2 + n is made of pk words
+// n - 1 and n; `words`: the records are 8-byte aligned.
+template <int K>
+__global__ void __launch_bounds__(128) k_dataset_ids(uint64_t count, uint8_t* __restrict__ out, bool words) {
+    constexpr int PK = 384 * K + 32, REC = 32 + PK, PART = K == 4 ? 5 : 4;
+    constexpr int PW = PK / 8;                       // pk words
+    constexpr int MSG = 16 + PART + PK;              // message bytes
+    constexpr int BLOCKS = MSG / 136 + 1;            // padding takes at least one byte
+    const uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (r >= count) return;
+    uint8_t* rec = out + r * (uint64_t)REC;
+    const uint8_t* pk = rec + 32;
+    auto word = [&](int n) -> uint64_t {
+        if (words) return reinterpret_cast<const uint64_t*>(pk)[n];
+        uint64_t v = 0;
+        for (int b = 0; b < 8; b++) v |= (uint64_t)pk[8 * n + b] << (8 * b);
+        return v;
+    };
+    auto chars = [](const char* s, int n) {
+        uint64_t v = 0;
+        for (int b = 0; b < n; b++) v |= (uint64_t)(uint8_t)s[b] << (8 * b);
+        return v;
+    };
+    const char* tail = K == 2 ? "-512" : (K == 3 ? "-768" : "-1024");
+    uint64_t carry = chars(tail, PART), a[25], m[17];
+    int n = 0;  // next pk word
+    // the next block's 17 message words, loaded while the previous block is permuted
+    auto load = [&](int blk) {
+#pragma unroll
+        for (int i = 0; i < 17; i++) {
+            if (i < 2 && blk == 0) m[i] = i ? chars(":ml-kem", 7) << 8 | '1' : chars("pq-key:v", 8);
+            else m[i] = n < PW ? word(n++) : 0;
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < 25; i++) a[i] = 0;
+    load(0);
+    int absorbed = 0;  // pk words absorbed
+#pragma unroll 1
+    for (int blk = 0; blk < BLOCKS; blk++) {
+#pragma unroll
+        for (int i = 0; i < 17; i++) {
+            uint64_t x = m[i];
+            if (i >= 2 || blk) {
+                if (absorbed < PW) {
+                    x = carry | (m[i] << (8 * PART));
+                    carry = m[i] >> (64 - 8 * PART);
+                } else {
+                    x = absorbed == PW ? carry | (0x06ull << (8 * PART)) : 0;  // the last bytes and the domain byte
+                }
+                absorbed++;
+            }
+            if (i == 16 && blk == BLOCKS - 1) x ^= 0x80ull << 56;
+            a[i] ^= x;
+        }
+        if (blk + 1 < BLOCKS) load(blk + 1);
+        keccakf(a);
     }
-    return r & 1;
+    if (words) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) reinterpret_cast<uint64_t*>(rec)[i] = a[i];
+    } else {
+        for (int b = 0; b < 32; b++) {
+            uint64_t v = a[0];
+            if (b >= 8) v = b >= 24 ? a[3] : (b >= 16 ? a[2] : a[1]);
+            rec[b] = (uint8_t)(v >> (8 * (b & 7)));
+        }
+    }
 }
 
-int brv7(int x) {
-    int r = 0;
-    for (int i = 0; i < 7; i++) r |= ((x >> i) & 1) << (6 - i);
-    return r;
-}
-
-int pow17(int e) {
-    int64_t r = 1, b = 17;
-    while (e) {
-        if (e & 1) r = r * b % MQ;
-        b = b * b % MQ;
-        e >>= 1;
-    }
-    return (int)r;
-}
-
-cudaError_t load_dataset_constants() {
-    uint64_t rc[24];
-    for (int ir = 0; ir < 24; ir++) {
-        rc[ir] = 0;
-        for (int j = 0; j <= 6; j++)
-            if (rc_bit(j + 7 * ir)) rc[ir] |= 1ull << ((1 << j) - 1);
-    }
-    int16_t zeta[128], gamma[128];
-    for (int i = 0; i < 128; i++) {
-        zeta[i] = (int16_t)pow17(brv7(i));
-        gamma[i] = (int16_t)pow17(2 * brv7(i) + 1);
-    }
-    cudaError_t e = cudaMemcpyToSymbol(c_keccak_rc, rc, sizeof(rc));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_zeta, zeta, sizeof(zeta));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gamma, gamma, sizeof(gamma));
-    return e;
+template <int K>
+cudaError_t launch_dataset(const uint32_t (&key)[8], uint64_t first, uint64_t count, uint8_t* d_records,
+                           cudaStream_t st) {
+    const uint4 lo = make_uint4(key[0], key[1], key[2], key[3]), hi = make_uint4(key[4], key[5], key[6], key[7]);
+    const int smem = (int)sizeof(Keys<K>);
+    cudaError_t e = cudaFuncSetAttribute(k_dataset_keys<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const bool words = reinterpret_cast<uintptr_t>(d_records) % 8 == 0;
+    k_dataset_keys<K><<<(unsigned)((count + Keys<K>::R - 1) / Keys<K>::R), Keys<K>::THREADS, smem, st>>>(lo, hi, first, count,
+                                                                                                    d_records, words);
+    k_dataset_ids<K><<<(unsigned)((count + 127) / 128), 128, 0, st>>>(count, d_records, words);
+    return cudaGetLastError();
 }
 
 // rand_core SeedableRng::seed_from_u64: PCG32 output words, little endian
@@ -356,18 +485,18 @@ extern "C" int ipr_dataset_generate(int device, int kem, uint64_t seed, uint64_t
     }
     int st = ipr::cuda_status(cudaSetDevice(device));
     if (st) return st;
-    if ((st = ipr::cuda_status(ipr::load_dataset_constants()))) return st;
-    uint32_t key[8];
-    ipr::seed_from_u64(seed, key);
-    const uint4 lo = make_uint4(key[0], key[1], key[2], key[3]), hi = make_uint4(key[4], key[5], key[6], key[7]);
-    const uint64_t blocks = (count + 127) / 128;
+    const uint64_t blocks = (count + 3) / 4;
     if (blocks > 0x7fffffffull) {
         ipr::set_last_error("ipr_dataset_generate: count too large for one call");
         return IPR_E_ARGS;
     }
-    ipr::k_dataset<<<(unsigned)blocks, 128, 0, static_cast<cudaStream_t>(stream)>>>(k, lo, hi, first, count,
-                                                                                   d_records);
-    return ipr::cuda_status(cudaGetLastError());
+    uint32_t key[8];
+    ipr::seed_from_u64(seed, key);
+    auto cs = static_cast<cudaStream_t>(stream);
+    const cudaError_t e = k == 2   ? ipr::launch_dataset<2>(key, first, count, d_records, cs)
+                          : k == 3 ? ipr::launch_dataset<3>(key, first, count, d_records, cs)
+                                   : ipr::launch_dataset<4>(key, first, count, d_records, cs);
+    return ipr::cuda_status(e);
 }
 
 // the same records into host memory: a device buffer of one batch (at most 65,536 records)

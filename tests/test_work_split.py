@@ -123,3 +123,21 @@ def test_collapse_with_given_rows_matches_oracle(pkg, orc):
             _free(p)
     for name, w, g in zip(("a_hat", "bold_t", "bold_t_bar", "bold_t_hat"), (a_hat, bt, btb, bth), got):
         assert np.array_equal(np.asarray(w).reshape(-1), g), name
+
+
+@pytest.mark.parametrize("kem,counts", [("ml-kem-512", (1, 15, 16, 17)), ("ml-kem-768", (1, 6, 7, 8, 129)),
+                                        ("ml-kem-1024", (1, 3, 4, 5))])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_dataset_tiles(pkg, orc, kem, counts, shift):
+    """a CTA's records less one, all, one more; shift 1: records that are not word-aligned"""
+    import torch
+    gen = pkg.DatasetGenerator(kem, 1000).with_seed(11)
+    for n in counts:
+        d = torch.full((n * gen.record_size + 16,), 7, dtype=torch.uint8, device="cuda")
+        gen.generate_device(d.data_ptr() + shift, first=3, count=n)
+        got = d.cpu().numpy()
+        rows = got[shift:shift + n * gen.record_size].reshape(n, -1)
+        for i in {0, n // 2, n - 1}:
+            rid, pk = orc.dataset_record(kem, 11, 3 + i)
+            assert rows[i].tobytes() == rid + pk
+        assert (got[:shift] == 7).all() and (got[shift + rows.size:] == 7).all()
