@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(F4_THREADS, STAGE ? 2 : 3)
 // 8 coefficients of layout A).  A step is a chain of dependent transforms, so with few chains
 // the time is its latency: here it holds one forward batch and one single inverse transform
 // where k_fold4 runs four and four, and each CTA has an SM's schedulers for itself.
-// 31 steps of up to 32 chains: 174 us (5.6 us a step), against 482 us for k_fold4; from about
+// 31 steps of up to 32 chains: 167 us (5.4 us a step), against 474 us for k_fold4; from about
 // 0.4 chains per SM on it is bound by issue like k_fold4, at a fifth more work per chain (both
 // limbs' CTAs compose s), so the server picks the form by the number of chains.
 // Shared memory: exchange buffer 24 KB, bodies and row 0 / S staged by cp.async 32 KB, the two
@@ -539,7 +539,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
     };
     // pr -> x: inverse transform, residues of the other limb, CRT, + packed row
     auto to_s = [&]() {
-        inverse_one(pr, t, xbuf, 1, iw, q);
+        inverse_one<true>(pr, t, xbuf, 1, iw, q);
 #pragma unroll
         for (int m = 0; m < EPT; m++) st_peer(ex2 + m * 256 + t, rank ^ 1, pr[m]);
         umma::cluster_sync();
@@ -579,7 +579,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
         for (int m = 0; m < EPT; m++)
 #pragma unroll
             for (int k = 0; k < 3; k++) v[k][m] = (uint32_t)((x[m] >> (k * GADGET_BITS)) & mask);
-        forward_digits<3>(v, t, xbuf, 1, fw, q);
+        forward_digits<3, true>(v, t, xbuf, 1, fw, q);
         load_pk(j);
         cp_wait<0>();
         uint32_t acc0[EPT], acc1[EPT];  // digit sum (< 6q), Montgomery-reduced product (< 2q)

@@ -18,6 +18,7 @@
 #include "host_math.hpp"
 #include "ipr_b200.h"
 #include "ipr_device.cuh"
+#include "ntt_lazy.cuh"
 #include "ntt_regs.cuh"
 #include "umma.cuh"
 
@@ -26,56 +27,79 @@ void set_last_error(const char* msg);
 
 namespace {
 
-constexpr int M_POLYS = 4;  // polynomials per 256-thread CTA (one twiddle load feeds 4 butterflies)
+// N^-1 mod q and its Shoup companion
+struct LimbScale {
+    uint32_t w, wp;
+};
 
-// One CTA of 256 threads per M_POLYS polynomials.  Global memory is read and written in
-// natural order (coalesced 8-byte accesses); the register layouts the transforms start
-// from and end in are reached through shared memory.
-template <bool INVERSE>
-__global__ void __launch_bounds__(256) k_ntt_limb(uint64_t* __restrict__ polys, int64_t count, uint32_t q,
-                                                  const uint32_t* __restrict__ w, const uint32_t* __restrict__ wp) {
-    __shared__ uint32_t xbuf[M_POLYS * N];
+// 32 bytes of four 64-bit words whose high halves are zero
+__device__ __forceinline__ void ld_words4(const uint64_t* p, uint32_t (&v)[4]) {
+    asm volatile("{\n\t.reg .b32 h0, h1, h2, h3;\n\tld.global.v8.b32 {%0,h0,%1,h1,%2,h2,%3,h3}, [%4];\n\t}\n"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "l"(p));
+}
+__device__ __forceinline__ void st_words4(uint64_t* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%5,%2,%5,%3,%5,%4,%5};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(0)
+                 : "memory");
+}
+
+// One CTA of 256 threads per polynomial, lazily reduced transforms (ntt_lazy.cuh).  The
+// coefficient side is read or written in layout A (coalesced 8-byte accesses), the NTT side in
+// layout D, where a thread's 8 consecutive words are two whole 32-byte sectors (WIDE: 32-byte
+// aligned buffers; 8-byte accesses otherwise), so neither side passes through shared memory.
+// Bound by HBM and, nearly as much, by the shared-memory exchanges; two or four polynomials per
+// CTA share their twiddles but fill the last wave worse.  4096 / 1501 polynomials, out of
+// L2: 28.2 / 13.8 us forward, 28.8 / 14.4 us inverse (4.7 TB/s), against 34 / 21 us for the
+// canonical butterflies on four polynomials with both sides staged.
+template <bool INVERSE, bool WIDE>
+__global__ void __launch_bounds__(256, 6)
+    k_ntt_limb(uint64_t* __restrict__ polys, uint32_t q, const uint2* __restrict__ tw, LimbScale ni) {
+    __shared__ __align__(16) uint32_t xbuf[N];
     const int t = threadIdx.x;
-    const int64_t p0 = (int64_t)blockIdx.x * M_POLYS;
-    uint32_t v[M_POLYS][nttr::EPT];
+    uint64_t* poly = polys + (int64_t)blockIdx.x * N;
+    uint32_t v[1][nttr::EPT];
+    if (INVERSE && WIDE) {
 #pragma unroll
-    for (int p = 0; p < M_POLYS; p++) {
-        const bool live = p0 + p < count;
-        const uint64_t* src = polys + (p0 + p) * N;
+        for (int h = 0; h < 2; h++) {
+            uint32_t w[4];
+            ld_words4(poly + 8 * t + 4 * h, w);
 #pragma unroll
-        for (int m = 0; m < nttr::EPT; m++) {
-            const uint32_t x = live ? (uint32_t)src[nttr::eA(t, m)] : 0u;
-            if (INVERSE) xbuf[p * N + nttr::eA(t, m)] = x;  // to layout D below
-            else v[p][m] = x;
+            for (int i = 0; i < 4; i++) v[0][4 * h + i] = w[i];
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < nttr::EPT; m++) v[0][m] = (uint32_t)poly[INVERSE ? nttr::eD(t, m) : nttr::eA(t, m)];
+    }
+#pragma unroll
+    for (int m = 0; m < nttr::EPT; m++) v[0][m] = nttr::canon(v[0][m], q);  // any input below 4q
+    if (INVERSE) {
+        nttl::inverse_polys<1, true>(v, t, xbuf, 1, tw, q);
+#pragma unroll
+        for (int m = 0; m < nttr::EPT; m++) poly[nttr::eA(t, m)] = nttl::mul_canon(v[0][m], ni.w, ni.wp, q);
+    } else {
+        nttl::forward_digits<1, true>(v, t, xbuf, 1, tw, q);  // inputs below q: below 15 q through stage 6
+#pragma unroll
+        for (int m = 0; m < nttr::EPT; m++) v[0][m] = nttr::csub(v[0][m], q);
+        uint64_t* dst = poly + 8 * t;
+        if (WIDE) {
+            st_words4(dst, v[0][0], v[0][1], v[0][2], v[0][3]);
+            st_words4(dst + 4, v[0][4], v[0][5], v[0][6], v[0][7]);
+        } else {
+#pragma unroll
+            for (int m = 0; m < nttr::EPT; m++) dst[m] = v[0][m];
         }
     }
-    if (INVERSE) {
-        __syncthreads();
-#pragma unroll
-        for (int p = 0; p < M_POLYS; p++)
-#pragma unroll
-            for (int m = 0; m < nttr::EPT; m++) v[p][m] = xbuf[p * N + nttr::eD(t, m)];
-        __syncthreads();
-        nttr::inverse<M_POLYS>(v, t, xbuf, 1, w, wp, q);  // ends in layout A
-    } else {
-        nttr::forward<M_POLYS>(v, t, xbuf, 1, w, wp, q);  // ends in layout D
-        __syncthreads();
-#pragma unroll
-        for (int p = 0; p < M_POLYS; p++)
-#pragma unroll
-            for (int m = 0; m < nttr::EPT; m++) xbuf[p * N + nttr::eD(t, m)] = v[p][m];
-        __syncthreads();
-#pragma unroll
-        for (int p = 0; p < M_POLYS; p++)
-#pragma unroll
-            for (int m = 0; m < nttr::EPT; m++) v[p][m] = xbuf[p * N + nttr::eA(t, m)];
-    }
-#pragma unroll
-    for (int p = 0; p < M_POLYS; p++) {
-        if (p0 + p >= count) break;
-        uint64_t* dst = polys + (p0 + p) * N;
-#pragma unroll
-        for (int m = 0; m < nttr::EPT; m++) dst[nttr::eA(t, m)] = v[p][m];
+}
+
+// count <= 2^36: launches of at most 2^30 polynomials
+template <bool INVERSE>
+void launch_ntt_limb(uint64_t* polys, int64_t count, uint32_t q, const uint2* tw, LimbScale ni, cudaStream_t st) {
+    constexpr int64_t MOST = 1ll << 30;
+    for (int64_t p0 = 0; p0 < count; p0 += MOST) {
+        const unsigned blocks = (unsigned)std::min(MOST, count - p0);
+        uint64_t* d = polys + p0 * N;
+        if (reinterpret_cast<uintptr_t>(d) % 32 == 0) k_ntt_limb<INVERSE, true><<<blocks, 256, 0, st>>>(d, q, tw, ni);
+        else k_ntt_limb<INVERSE, false><<<blocks, 256, 0, st>>>(d, q, tw, ni);
     }
 }
 
@@ -111,22 +135,21 @@ __global__ void k_wait_selftest(uint64_t limit_ns, int* out) {
     if (threadIdx.x == 0) *out = done ? 1 : 0;
 }
 
-// per-device NTT tables (fw, fwp, iw, iwp: [4][2 limbs][N] u32), built on first use
+// per-device NTT tables (forward and plain inverse twiddles interleaved with their Shoup companions:
+// [2][2 limbs][N] pairs), built on first use
 std::mutex g_mu;
-std::vector<uint32_t*> g_tables;
+std::vector<uint2*> g_tables;
 
-int tables_for(int device, const uint32_t** out) {
+int tables_for(int device, const uint2** out) {
     std::lock_guard<std::mutex> lk(g_mu);
     if ((int)g_tables.size() <= device) g_tables.resize(device + 1, nullptr);
-    uint32_t*& d = g_tables[device];
+    uint2*& d = g_tables[device];
     if (!d) {
         HostParams hp;
         host_params_init(hp);
         std::vector<uint32_t> h(8 * N);
-        std::copy(hp.fw.begin(), hp.fw.end(), h.begin());
-        std::copy(hp.fwp.begin(), hp.fwp.end(), h.begin() + 2 * N);
-        std::copy(hp.iw.begin(), hp.iw.end(), h.begin() + 4 * N);
-        std::copy(hp.iwp.begin(), hp.iwp.end(), h.begin() + 6 * N);
+        std::copy(hp.fwi.begin(), hp.fwi.end(), h.begin());
+        std::copy(hp.iwi.begin(), hp.iwi.end(), h.begin() + 4 * N);
         cudaError_t e = cudaMalloc(&d, h.size() * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMemcpy(d, h.data(), h.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
@@ -159,16 +182,17 @@ int ipr_ntt_batch(int device, uint64_t* d_polys, uint64_t count, int limb, int i
     if (count == 0) return IPR_OK;
     int st = ipr::cuda_status(cudaSetDevice(device));
     if (st) return st;
-    const uint32_t* tb;
+    const uint2* tb;
     if ((st = ipr::tables_for(device, &tb))) return st;
     const int n = ipr::N;
     const uint32_t q = limb ? ipr::Q1 : ipr::Q0;
-    const uint32_t* w = tb + (inverse ? 4 * n : 0) + limb * n;
-    const uint32_t* wp = tb + (inverse ? 6 * n : 2 * n) + limb * n;
-    const unsigned blocks = (unsigned)((count + ipr::M_POLYS - 1) / ipr::M_POLYS);
+    const uint2* tw = tb + (inverse ? 2 * n : 0) + limb * n;
+    const uint32_t w = q - (q - 1) / n;  // N^-1 mod q
+    const ipr::LimbScale ni{w, (uint32_t)(((uint64_t)w << 32) / q)};
     auto cs = static_cast<cudaStream_t>(stream);
-    if (inverse) ipr::k_ntt_limb<true><<<blocks, 256, 0, cs>>>(d_polys, (int64_t)count, q, w, wp);
-    else ipr::k_ntt_limb<false><<<blocks, 256, 0, cs>>>(d_polys, (int64_t)count, q, w, wp);
+    const int64_t c = (int64_t)count;
+    if (inverse) ipr::launch_ntt_limb<true>(d_polys, c, q, tw, ni, cs);
+    else ipr::launch_ntt_limb<false>(d_polys, c, q, tw, ni, cs);
     return ipr::cuda_status(cudaGetLastError());
 }
 

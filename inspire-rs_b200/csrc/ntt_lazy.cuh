@@ -48,15 +48,48 @@ __device__ __forceinline__ int tw_idx(int mm, int hi, int k) {
     return (1 << mm) + (hi >> (11 - mm)) + ((k * RS) >> (11 - mm));
 }
 
-template <int P, int MODE, int RS>
-__device__ __forceinline__ void fstage(uint32_t (&v)[P][EPT], int mm, int dd, int hi, const uint2* __restrict__ tw,
-                                       uint32_t q) {
+// the consecutive twiddles of a stage with register distance dd: 4 / dd of them (elements k that
+// share k / (2 dd) share one), in one 8-, 16- or 32-byte load.  The first index is a multiple
+// of their number, so the load is aligned.  HOIST lets the compiler move the loads above the
+// exchanges' barriers: faster where registers are free (the four-CTA fold 181 -> 167 us, the
+// batched NTT), slower where they are not (the collapse 5.21 -> 5.41 ms, two chains per SM 472 ->
+// 507 us).
+struct Tw4 {
+    uint2 w[4];
+};
+template <int DD, int RS, bool HOIST>
+__device__ __forceinline__ Tw4 load_tw(const uint2* __restrict__ tw, int mm, int hi) {
+    const uint2* p = tw + tw_idx<RS>(mm, hi, 0);
+    Tw4 r;
+    if constexpr (DD == 4) {
+        r.w[0] = __ldg(p);
+    } else if constexpr (DD == 2) {
+        const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
+        r.w[0] = make_uint2(a.x, a.y);
+        r.w[1] = make_uint2(a.z, a.w);
+    } else {
+        if constexpr (HOIST)
+            asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                : "=r"(r.w[0].x), "=r"(r.w[0].y), "=r"(r.w[1].x), "=r"(r.w[1].y), "=r"(r.w[2].x), "=r"(r.w[2].y),
+                  "=r"(r.w[3].x), "=r"(r.w[3].y)
+                : "l"(p));
+        else
+            asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                         : "=r"(r.w[0].x), "=r"(r.w[0].y), "=r"(r.w[1].x), "=r"(r.w[1].y), "=r"(r.w[2].x),
+                           "=r"(r.w[2].y), "=r"(r.w[3].x), "=r"(r.w[3].y)
+                         : "l"(p));
+    }
+    return r;
+}
+
+template <int P, int MODE, int DD, int RS, bool HOIST>
+__device__ __forceinline__ void fstage(uint32_t (&v)[P][EPT], int mm, int hi, const uint2* __restrict__ tw, uint32_t q) {
+    const Tw4 w = load_tw<DD, RS, HOIST>(tw, mm, hi);
 #pragma unroll
     for (int k = 0; k < EPT; k++) {
-        if (k & dd) continue;
-        const uint2 w = __ldg(tw + tw_idx<RS>(mm, hi, k));
+        if (k & DD) continue;
 #pragma unroll
-        for (int p = 0; p < P; p++) fwd_b<MODE>(v[p][k], v[p][k + dd], w.x, w.y, q);
+        for (int p = 0; p < P; p++) fwd_b<MODE>(v[p][k], v[p][k + DD], w.w[k / (2 * DD)].x, w.w[k / (2 * DD)].y, q);
     }
 }
 
@@ -104,26 +137,26 @@ __device__ __forceinline__ void xchg_b2a(uint32_t (&v)[P][EPT], int t, uint32_t*
 // in [0, 2q); xbuf holds XP >= P polynomials of this team.  Bounds: after stage s <= 6 every
 // value is below 2^19 + 2q (s + 1) <= 2^19 + 14q; stage 7 reduces x first (outputs < 4q);
 // stages 8..10 add 2q each (< 10q < 2^32); one reduction at the end.
-template <int P>
+template <int P, bool HOIST = false>
 __device__ __forceinline__ void forward_digits(uint32_t (&v)[P][EPT], int t, uint32_t* xbuf, int bar,
                                                const uint2* __restrict__ tw, uint32_t q) {
     const int l = t & 31, w = t >> 5;
     uint32_t* wb = xbuf + w * 256;
     const int hb = 256 * w, hc = 256 * w + 32 * (l >> 2), hd = 256 * w + 8 * l;
-    fstage<P, 0, 256>(v, 0, 4, 0, tw, q);
-    fstage<P, 0, 256>(v, 1, 2, 0, tw, q);
-    fstage<P, 0, 256>(v, 2, 1, 0, tw, q);
+    fstage<P, 0, 4, 256, HOIST>(v, 0, 0, tw, q);
+    fstage<P, 0, 2, 256, HOIST>(v, 1, 0, tw, q);
+    fstage<P, 0, 1, 256, HOIST>(v, 2, 0, tw, q);
     xchg_a2b<P>(v, t, xbuf, bar);
-    fstage<P, 0, 32>(v, 3, 4, hb, tw, q);
-    fstage<P, 0, 32>(v, 4, 2, hb, tw, q);
-    fstage<P, 0, 32>(v, 5, 1, hb, tw, q);
+    fstage<P, 0, 4, 32, HOIST>(v, 3, hb, tw, q);
+    fstage<P, 0, 2, 32, HOIST>(v, 4, hb, tw, q);
+    fstage<P, 0, 1, 32, HOIST>(v, 5, hb, tw, q);
     nttr::b_to_c<P>(v, l, wb);
-    fstage<P, 0, 4>(v, 6, 4, hc, tw, q);
-    fstage<P, 1, 4>(v, 7, 2, hc, tw, q);
-    fstage<P, 0, 4>(v, 8, 1, hc, tw, q);
+    fstage<P, 0, 4, 4, HOIST>(v, 6, hc, tw, q);
+    fstage<P, 1, 2, 4, HOIST>(v, 7, hc, tw, q);
+    fstage<P, 0, 1, 4, HOIST>(v, 8, hc, tw, q);
     nttr::c_to_d<P>(v, l, wb);
-    fstage<P, 0, 1>(v, 9, 2, hd, tw, q);
-    fstage<P, 0, 1>(v, 10, 1, hd, tw, q);
+    fstage<P, 0, 2, 1, HOIST>(v, 9, hd, tw, q);
+    fstage<P, 0, 1, 1, HOIST>(v, 10, hd, tw, q);
 #pragma unroll
     for (int p = 0; p < P; p++)
 #pragma unroll
@@ -142,17 +175,18 @@ __device__ __forceinline__ void inv_b(uint32_t& x, uint32_t& y, uint32_t w, uint
 }
 
 // one inverse stage over 2 * PL polynomials: [0, PL) of limb 0, [PL, 2 PL) of limb 1
-template <int PL, int OFF, bool RED, int RS>
-__device__ __forceinline__ void istage(uint32_t (&v)[2 * PL][EPT], int mm, int dd, int hi, const uint2* __restrict__ iw) {
+template <int PL, int OFF, bool RED, int DD, int RS>
+__device__ __forceinline__ void istage(uint32_t (&v)[2 * PL][EPT], int mm, int hi, const uint2* __restrict__ iw) {
 #pragma unroll
-    for (int k = 0; k < EPT; k++) {
-        if (k & dd) continue;
-        const int idx = tw_idx<RS>(mm, hi, k);
-        const uint2 w0 = __ldg(iw + idx), w1 = __ldg(iw + N + idx);
+    for (int l = 0; l < 2; l++) {
+        const Tw4 w = load_tw<DD, RS, false>(iw + l * N, mm, hi);
 #pragma unroll
-        for (int p = 0; p < PL; p++) inv_b<OFF, RED>(v[p][k], v[p][k + dd], w0.x, w0.y, Q0);
+        for (int k = 0; k < EPT; k++) {
+            if (k & DD) continue;
+            const uint2 x = w.w[k / (2 * DD)];
 #pragma unroll
-        for (int p = PL; p < 2 * PL; p++) inv_b<OFF, RED>(v[p][k], v[p][k + dd], w1.x, w1.y, Q1);
+            for (int p = l * PL; p < (l + 1) * PL; p++) inv_b<OFF, RED>(v[p][k], v[p][k + DD], x.x, x.y, l ? Q1 : Q0);
+        }
     }
 }
 
@@ -165,20 +199,20 @@ __device__ __forceinline__ void inverse_limbs(uint32_t (&v)[2 * PL][EPT], int t,
     const int l = t & 31, w = t >> 5;
     uint32_t* wb = xbuf + w * 256;
     const int hb = 256 * w, hc = 256 * w + 32 * (l >> 2), hd = 256 * w + 8 * l;
-    istage<PL, 1, false, 1>(v, 10, 1, hd, iw);
-    istage<PL, 2, false, 1>(v, 9, 2, hd, iw);
+    istage<PL, 1, false, 1, 1>(v, 10, hd, iw);
+    istage<PL, 2, false, 2, 1>(v, 9, hd, iw);
     nttr::d_to_c<2 * PL, XB>(v, l, wb);
-    istage<PL, 4, false, 4>(v, 8, 1, hc, iw);
-    istage<PL, 8, true, 4>(v, 7, 2, hc, iw);
-    istage<PL, 2, false, 4>(v, 6, 4, hc, iw);
+    istage<PL, 4, false, 1, 4>(v, 8, hc, iw);
+    istage<PL, 8, true, 2, 4>(v, 7, hc, iw);
+    istage<PL, 2, false, 4, 4>(v, 6, hc, iw);
     nttr::c_to_b<2 * PL, XB>(v, l, wb);
-    istage<PL, 4, false, 32>(v, 5, 1, hb, iw);
-    istage<PL, 8, true, 32>(v, 4, 2, hb, iw);
-    istage<PL, 2, false, 32>(v, 3, 4, hb, iw);
+    istage<PL, 4, false, 1, 32>(v, 5, hb, iw);
+    istage<PL, 8, true, 2, 32>(v, 4, hb, iw);
+    istage<PL, 2, false, 4, 32>(v, 3, hb, iw);
     xchg_b2a<2 * PL, XB>(v, t, xbuf, bar);
-    istage<PL, 4, false, 256>(v, 2, 1, 0, iw);
-    istage<PL, 8, true, 256>(v, 1, 2, 0, iw);
-    istage<PL, 2, false, 256>(v, 0, 4, 0, iw);
+    istage<PL, 4, false, 1, 256>(v, 2, 0, iw);
+    istage<PL, 8, true, 2, 256>(v, 1, 0, iw);
+    istage<PL, 2, false, 4, 256>(v, 0, 0, iw);
 #pragma unroll
     for (int p = 0; p < 2 * PL; p++)
 #pragma unroll
@@ -188,42 +222,50 @@ __device__ __forceinline__ void inverse_limbs(uint32_t (&v)[2 * PL][EPT], int t,
         }
 }
 
-// one inverse stage of a single polynomial
-template <int OFF, bool RED, int RS>
-__device__ __forceinline__ void istage_one(uint32_t (&v)[EPT], int mm, int dd, int hi, const uint2* __restrict__ iw,
-                                           uint32_t q) {
+// one inverse stage of P polynomials of one limb
+template <int P, int OFF, bool RED, int DD, int RS, bool HOIST>
+__device__ __forceinline__ void istage_limb(uint32_t (&v)[P][EPT], int mm, int hi, const uint2* __restrict__ iw,
+                                            uint32_t q) {
+    const Tw4 w = load_tw<DD, RS, HOIST>(iw, mm, hi);
 #pragma unroll
     for (int k = 0; k < EPT; k++) {
-        if (k & dd) continue;
-        const uint2 w = __ldg(iw + tw_idx<RS>(mm, hi, k));
-        inv_b<OFF, RED>(v[k], v[k + dd], w.x, w.y, q);
+        if (k & DD) continue;
+#pragma unroll
+        for (int p = 0; p < P; p++) inv_b<OFF, RED>(v[p][k], v[p][k + DD], w.w[k / (2 * DD)].x, w.w[k / (2 * DD)].y, q);
     }
 }
 
-// N * INTT of one canonical polynomial of one limb (iw: that limb's table): layout D in, layout
+// N * INTT of P canonical polynomials of one limb (iw: that limb's table): layout D in, layout
 // A canonical out; the bounds of inverse_limbs
-__device__ __forceinline__ void inverse_one(uint32_t (&v)[EPT], int t, uint32_t* xbuf, int bar,
-                                            const uint2* __restrict__ iw, uint32_t q) {
+template <int P, bool HOIST = false>
+__device__ __forceinline__ void inverse_polys(uint32_t (&v)[P][EPT], int t, uint32_t* xbuf, int bar,
+                                              const uint2* __restrict__ iw, uint32_t q) {
     const int l = t & 31, w = t >> 5;
     uint32_t* wb = xbuf + w * 256;
     const int hb = 256 * w, hc = 256 * w + 32 * (l >> 2), hd = 256 * w + 8 * l;
-    uint32_t (&p)[1][EPT] = reinterpret_cast<uint32_t (&)[1][EPT]>(v);
-    istage_one<1, false, 1>(v, 10, 1, hd, iw, q);
-    istage_one<2, false, 1>(v, 9, 2, hd, iw, q);
-    nttr::d_to_c<1>(p, l, wb);
-    istage_one<4, false, 4>(v, 8, 1, hc, iw, q);
-    istage_one<8, true, 4>(v, 7, 2, hc, iw, q);
-    istage_one<2, false, 4>(v, 6, 4, hc, iw, q);
-    nttr::c_to_b<1>(p, l, wb);
-    istage_one<4, false, 32>(v, 5, 1, hb, iw, q);
-    istage_one<8, true, 32>(v, 4, 2, hb, iw, q);
-    istage_one<2, false, 32>(v, 3, 4, hb, iw, q);
-    xchg_b2a<1>(p, t, xbuf, bar);
-    istage_one<4, false, 256>(v, 2, 1, 0, iw, q);
-    istage_one<8, true, 256>(v, 1, 2, 0, iw, q);
-    istage_one<2, false, 256>(v, 0, 4, 0, iw, q);
+    istage_limb<P, 1, false, 1, 1, HOIST>(v, 10, hd, iw, q);
+    istage_limb<P, 2, false, 2, 1, HOIST>(v, 9, hd, iw, q);
+    nttr::d_to_c<P>(v, l, wb);
+    istage_limb<P, 4, false, 1, 4, HOIST>(v, 8, hc, iw, q);
+    istage_limb<P, 8, true, 2, 4, HOIST>(v, 7, hc, iw, q);
+    istage_limb<P, 2, false, 4, 4, HOIST>(v, 6, hc, iw, q);
+    nttr::c_to_b<P>(v, l, wb);
+    istage_limb<P, 4, false, 1, 32, HOIST>(v, 5, hb, iw, q);
+    istage_limb<P, 8, true, 2, 32, HOIST>(v, 4, hb, iw, q);
+    istage_limb<P, 2, false, 4, 32, HOIST>(v, 3, hb, iw, q);
+    xchg_b2a<P>(v, t, xbuf, bar);
+    istage_limb<P, 4, false, 1, 256, HOIST>(v, 2, 0, iw, q);
+    istage_limb<P, 8, true, 2, 256, HOIST>(v, 1, 0, iw, q);
+    istage_limb<P, 2, false, 4, 256, HOIST>(v, 0, 0, iw, q);
 #pragma unroll
-    for (int k = 0; k < EPT; k++) v[k] = csub(csub(v[k], 2 * q), q);
+    for (int p = 0; p < P; p++)
+#pragma unroll
+        for (int k = 0; k < EPT; k++) v[p][k] = csub(csub(v[p][k], 2 * q), q);
+}
+template <bool HOIST = false>
+__device__ __forceinline__ void inverse_one(uint32_t (&v)[EPT], int t, uint32_t* xbuf, int bar,
+                                            const uint2* __restrict__ iw, uint32_t q) {
+    inverse_polys<1, HOIST>(reinterpret_cast<uint32_t (&)[1][EPT]>(v), t, xbuf, bar, iw, q);
 }
 
 // the 8 consecutive words of layout D held by thread t (two 16-byte loads)

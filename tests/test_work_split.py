@@ -141,3 +141,27 @@ def test_dataset_tiles(pkg, orc, kem, counts, shift):
             rid, pk = orc.dataset_record(kem, 11, 3 + i)
             assert rows[i].tobytes() == rid + pk
         assert (got[:shift] == 7).all() and (got[shift + rows.size:] == 7).all()
+
+
+@pytest.mark.parametrize("count", [1, 2, 149])
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_ntt_of_any_word_alignment(pkg, orc, count, shift):
+    """buffers at 0, 8 and 16 bytes past a 32-byte boundary, forward and back"""
+    import numpy as np
+    import torch
+    rng = np.random.default_rng(count + shift)
+    for limb, q in enumerate((268369921, 249561089)):
+        polys = rng.integers(0, q, (count, N), dtype=np.uint64)
+        polys[0, :3] = (0, q - 1, 1)
+        d = torch.full((count * N + 8,), 5, dtype=torch.int64, device="cuda")
+        body = d[shift:shift + count * N]
+        body.copy_(torch.from_numpy(polys.reshape(-1).view(np.int64)))
+        pkg.ntt_batch(body.data_ptr(), count, limb)
+        got = body.cpu().numpy().view(np.uint64).reshape(count, N)
+        for i in {0, count - 1}:
+            both = np.zeros((2, N), dtype=np.uint64)
+            both[limb] = polys[i]
+            assert np.array_equal(got[i], orc.ntt_forward(both)[limb])
+        pkg.ntt_batch(body.data_ptr(), count, limb, inverse=True)
+        assert np.array_equal(body.cpu().numpy().view(np.uint64).reshape(count, N), polys)
+        assert (d[:shift] == 5).all() and (d[shift + count * N:] == 5).all()
