@@ -75,14 +75,20 @@ void destroy_graphs(ipr_server* s) {
 constexpr unsigned kQbPadRows = 256;
 unsigned qb_rows(unsigned nq) { return 7 * nq + kQbPadRows; }
 
-// the GEMM's tile height: the smallest multiple of 16 that holds all nq queries, at most 224
-// (32 queries), lowered under the server option's cap to a multiple of 112 (16 queries, no
-// unused rows) when the cap allows one, else to a multiple of 16
+// the GEMM's tile height: the queries go to the fewest tiles of at most 224 rows (32 queries;
+// under the server option's cap the largest multiple of 112 = 16 queries within it, or of 16
+// below that), and every tile is the smallest multiple of 16 that holds an even share of them,
+// so that no tile is mostly unused rows (40 queries: two tiles of 144, not of 224)
 int g1_nt(const ipr_server* s, unsigned nq) {
-    int nt = (int)(7 * nq + 15) / 16 * 16;
-    if (nt > 224) nt = 224;
-    if (s->g1_tile && s->g1_tile < nt) nt = s->g1_tile >= 112 ? s->g1_tile / 112 * 112 : s->g1_tile / 16 * 16;
-    return nt < 16 ? 16 : nt;
+    int most = 224;
+    if (s->g1_tile && s->g1_tile < most) most = s->g1_tile >= 112 ? s->g1_tile / 112 * 112 : s->g1_tile / 16 * 16;
+    if (most < 16) most = 16;
+    const int one = (int)(7 * nq + 15) / 16 * 16;  // a single tile of up to the cap itself
+    if (one <= (s->g1_tile && s->g1_tile < 224 ? s->g1_tile : 224)) return one;
+    const unsigned per = most / 7, tiles = (nq + per - 1) / per;
+    const unsigned share = (nq + tiles - 1) / tiles;
+    const int nt = (int)(7 * share + 15) / 16 * 16;
+    return nt < most ? nt : most;
 }
 int g1_tiles(unsigned nq, int nt) { return (int)((nq + nt / 7 - 1) / (nt / 7)); }
 
@@ -126,21 +132,21 @@ int ensure_scratch(ipr_server* s, unsigned nq) {
 
 // The one-chain fold's form for `chains` chains, by predicted time.  Chains run in rounds of
 // (chains per SM x SMs).  In hundredths of a round of two chains per SM staging the RGSW bodies
-// in shared memory (820 us for 31 steps):
-//   two per SM, staged       100 a round, 60 for a last round of at most one chain per SM (482 us)
+// in shared memory (830 us for 31 steps):
+//   two per SM, staged       100 a round, 57 for a last round of at most one chain per SM (474 us)
 //   three per SM, bodies from L2 (more warps to hide latency, 80 registers)  122 a round
-//   four CTAs per chain      21 (174 us) while the chip is not full, then 76 per chain and SM
-// Measured at 148 SMs (us, staged form / four CTAs per chain): 32 chains 482 / 175, 64 482 / 285,
-// 96 482 / 411, 120 492 / 520, 162 808 / 671, 240 819 / 955, 384 1313 / 1586; 1,408 chains (64 payloads at
+//   four CTAs per chain      20 (167 us) while the chip is not full, then 72 per chain and SM
+// Measured at 148 SMs (us, staged form / four CTAs per chain): 32 chains 474 / 167, 64 474 / 274,
+// 96 474 / 384, 120 474 / 477, 162 830 / 615, 240 833 / 940, 384 1300 / 1442; 1,408 chains (64 payloads at
 // 1M) take 4 rounds of three per SM against 5 of two.  Forms 4 / 5 force one occupancy.
 ipr::FoldForm fold_form(const ipr_server* s, int chains) {
     if (s->fold_mode == 4) return ipr::FoldForm::kThreePerSm;
     if (s->fold_mode == 5) return ipr::FoldForm::kStaged;
     const int64_t sm = s->sm_count > 0 ? s->sm_count : 1;
     const int64_t rest = chains % (2 * sm);
-    const int64_t staged = chains / (2 * sm) * 100 + (rest == 0 ? 0 : (rest <= sm ? 60 : 100));
+    const int64_t staged = chains / (2 * sm) * 100 + (rest == 0 ? 0 : (rest <= sm ? 57 : 100));
     const int64_t three = (chains + 3 * sm - 1) / (3 * sm) * 122;
-    const int64_t cluster = chains * 76 / sm > 21 ? chains * 76 / sm : 21;
+    const int64_t cluster = chains * 72 / sm > 20 ? chains * 72 / sm : 20;
     if (cluster < staged && cluster < three) return ipr::FoldForm::kCluster;
     return three >= staged ? ipr::FoldForm::kStaged : ipr::FoldForm::kThreePerSm;
 }
