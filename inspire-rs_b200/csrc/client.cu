@@ -37,9 +37,12 @@
 #include "host_math.hpp"
 #include "ipr_b200.h"
 #include "ipr_device.cuh"
+#include "ntt_lazy.cuh"
 
 namespace ipr {
 void set_last_error(const char* msg);
+// [forward, inverse without N^-1][2 limbs][N] twiddles interleaved with their companions, device memory (micro.cu)
+int ntt_tables(int device, const uint2** out);
 }
 
 namespace {
@@ -58,6 +61,8 @@ using ipr::N;
 using ipr::Q0;
 using ipr::Q1;
 using ipr::QQ;
+namespace nttr = ipr::nttr;
+namespace nttl = ipr::nttl;
 
 constexpr int KEY_POLYS = 6;     // y_0..2, z_0..2
 constexpr int GSW_COLS = 6;      // 2 t_gsw
@@ -99,9 +104,9 @@ __device__ __forceinline__ int cbd_sample(const uint32_t* key, uint64_t stream, 
     return (__popc(w[0]) + __popc(w[1]) + __popc(w[2] & m)) - (__popc(w[3]) + __popc(w[4]) + __popc(w[5] & m));
 }
 
+// v mod q for |v| < 2^40
 __device__ __forceinline__ uint32_t signed_mod(int64_t v, uint32_t q) {
-    int64_t r = v % (int64_t)q;
-    return (uint32_t)(r < 0 ? r + q : r);
+    return ipr::mod64((uint64_t)(v + ((int64_t)q << 13)), q, q == Q0 ? ipr::BR0 : ipr::BR1);
 }
 
 __device__ __forceinline__ uint32_t addmod(uint32_t a, uint32_t b, uint32_t q) {
@@ -113,16 +118,9 @@ __device__ __forceinline__ uint32_t mulmod32(uint32_t a, uint32_t b, uint32_t q,
     return ipr::mod64((uint64_t)a * b, q, br);
 }
 
-// rescale (src/core/arith.rs:436-452): round(a * out / inp) with the input centred in
-// (-inp/2, inp/2] and the result taken mod out
-__device__ __forceinline__ uint64_t rescale_any(uint64_t a, uint64_t inp, uint64_t out) {
-    const uint64_t av = a % inp, half = inp / 2;
-    const bool neg = av >= half;
-    const uint64_t u = neg ? inp - av : av;
-    const unsigned __int128 num = (unsigned __int128)u * out + half;
-    const uint64_t r = (uint64_t)(num / inp), rm = r % out;
-    return neg ? (rm ? out - rm : 0) : rm;
-}
+struct Targets {  // per sub-query: first-dimension row, sub-column
+    uint32_t row[255], sub[255];
+};
 
 struct BuildArgs {
     const uint32_t* key;        // [8] ChaCha key (the client seed)
@@ -132,42 +130,46 @@ struct BuildArgs {
     const int8_t* s;            // [N] secret key
     const int8_t* tau;          // [2][N] tau_5(s), tau_{2N-1}(s)
     const uint32_t* sa_row;     // [rpolys][2][N] raw residues of s * a_r
-    const int64_t* targets;     // [n][2] (row, sub-column)
-    uint64_t* limb0;            // [6 + 6n][N] residues to transform, limb 0
-    uint64_t* limb1;
-    uint64_t* fields;           // 56-bit wire fields of the payload
+    int64_t* vals;              // [6 + 6n][N] coefficients to transform: noise + message
+    uint8_t* out;               // the payload: 1 count byte, then 7-byte little-endian fields
 };
+
+__device__ __forceinline__ void put_field(uint8_t* out, int64_t field, uint32_t v0, uint32_t v1) {
+    const uint64_t v = (uint64_t)v0 | ((uint64_t)v1 << 28);
+    uint8_t* p = out + 1 + 7 * field;
+#pragma unroll
+    for (int b = 0; b < 7; b++) p[b] = (uint8_t)(v >> (8 * b));
+}
 
 // One thread per noise coefficient.  Noise polys: the 6 keys, then per sub-query its
 // rpolys row polys and its 6 RGSW columns in the order 1, 0, 3, 2, 5, 4 (the reference
-// encrypts sigma_j before s * sigma_j).
-__global__ void k_client_build(BuildArgs a) {
+// encrypts sigma_j before s * sigma_j).  Row polys need no transform: their fields are final.
+__global__ void k_client_build(BuildArgs a, const __grid_constant__ Targets tg) {
     __shared__ uint32_t key[8];
     if (threadIdx.x < 8) key[threadIdx.x] = a.key[threadIdx.x];
     __syncthreads();
     const int per_q = a.rpolys + GSW_COLS;
     const int64_t total = (int64_t)(KEY_POLYS + a.n * per_q) * N;
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.out[0] = (uint8_t)a.n;
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total;
          g += (int64_t)gridDim.x * blockDim.x) {
         const int p = (int)(g / N), i = (int)(g % N);
         const int e = cbd_sample(key, a.stream, (uint64_t)g);
         int64_t term = 0;  // message term of coefficient i (a small multiple of a gadget power)
-        int64_t dst = -1;  // transformed poly index, or -1 for a row poly
-        int64_t field = -1;
+        int64_t dst = -1;  // transformed poly index
         if (p < KEY_POLYS) {
             const int which = p / 3, k = p % 3;
             term = (int64_t)a.tau[which * N + i] * ((int64_t)1 << (ipr::GADGET_BITS * k));
             dst = p;
         } else {
             const int q = (p - KEY_POLYS) / per_q, r = (p - KEY_POLYS) % per_q;
-            const int64_t row = a.targets[2 * q], sub = a.targets[2 * q + 1];
+            const int64_t row = tg.row[q], sub = tg.sub[q];
             if (r < a.rpolys) {
                 const uint64_t m = (r == row / N && i == row % N) ? QQ / ipr::PT : 0;
                 const uint32_t* sa = a.sa_row + (int64_t)r * 2 * N;
                 const uint32_t v0 = addmod(addmod(sa[i], signed_mod(e, Q0), Q0), (uint32_t)(m % Q0), Q0);
                 const uint32_t v1 = addmod(addmod(sa[N + i], signed_mod(e, Q1), Q1), (uint32_t)(m % Q1), Q1);
-                field = KEY_POLYS * N + (int64_t)q * (a.db_rows + GSW_COLS * N) + (int64_t)r * N + i;
-                a.fields[field] = (uint64_t)v0 | ((uint64_t)v1 << 28);
+                put_field(a.out, KEY_POLYS * N + (int64_t)q * (a.db_rows + GSW_COLS * N) + (int64_t)r * N + i, v0, v1);
                 continue;
             }
             const int col = (r - a.rpolys) ^ 1, j = col >> 1;
@@ -182,97 +184,91 @@ __global__ void k_client_build(BuildArgs a) {
             }
             dst = KEY_POLYS + (int64_t)q * GSW_COLS + col;
         }
-        a.limb0[dst * N + i] = signed_mod((int64_t)e + term, Q0);
-        a.limb1[dst * N + i] = signed_mod((int64_t)e + term, Q1);
+        a.vals[dst * N + i] = (int64_t)e + term;
     }
 }
 
-// fields of the transformed polys: keys y_k / z_k (+ -s * mask), RGSW bodies (+ s * a)
-__global__ void k_client_finish(const uint64_t* __restrict__ limb0, const uint64_t* __restrict__ limb1, int n,
-                                int64_t db_rows, const uint32_t* __restrict__ neg_sm,
-                                const uint32_t* __restrict__ sa_gsw, uint64_t* __restrict__ fields) {
-    const int64_t total = (int64_t)(KEY_POLYS + GSW_COLS * n) * N;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int pp = (int)(t / N), z = (int)(t % N);
-        const uint32_t* add;
-        int64_t field;
-        if (pp < KEY_POLYS) {
-            const int which = pp / 3, k = pp % 3;
-            add = neg_sm + ((int64_t)(which * 3 + k) * 2) * N;
-            field = 2 * ((int64_t)k * N + z) + which;  // y and z interleaved per (column, slot)
-        } else {
-            const int q = (pp - KEY_POLYS) / GSW_COLS, c = (pp - KEY_POLYS) % GSW_COLS;
-            add = sa_gsw;
-            field = KEY_POLYS * N + (int64_t)q * (db_rows + GSW_COLS * N) + db_rows + (int64_t)c * N + z;
-        }
-        const uint32_t v0 = addmod((uint32_t)limb0[t], add[z], Q0);
-        const uint32_t v1 = addmod((uint32_t)limb1[t], add[N + z], Q1);
-        fields[field] = (uint64_t)v0 | ((uint64_t)v1 << 28);
-    }
-}
-
-// 1 count byte, then every field as 7 little-endian bytes
-__global__ void k_client_serialize(const uint64_t* __restrict__ fields, int64_t nfields, int n,
-                                   uint8_t* __restrict__ out) {
-    const int64_t f0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (f0 == 0) out[0] = (uint8_t)n;
-    for (int64_t f = f0; f < nfields; f += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t v = fields[f];
+// One CTA per transformed poly, one limb per 256 threads: NTT, plus -s * mask (keys y_k / z_k) or
+// s * a (RGSW bodies), and the poly's wire fields.  A payload was five launches (noise, one NTT
+// per limb, masks, serialisation) and is two.
+__global__ void __launch_bounds__(512) k_client_transform(const int64_t* __restrict__ vals, int64_t db_rows,
+                                                          const uint2* __restrict__ tw,
+                                                          const uint32_t* __restrict__ neg_sm,
+                                                          const uint32_t* __restrict__ sa_gsw,
+                                                          uint8_t* __restrict__ out) {
+    __shared__ __align__(16) uint32_t xbuf[2][N];
+    __shared__ uint32_t res[2][N];
+    const int l = threadIdx.x >> 8, t = threadIdx.x & 255;
+    const int pp = blockIdx.x;
+    const uint32_t q = l ? Q1 : Q0;
+    uint32_t v[1][nttr::EPT];
 #pragma unroll
-        for (int b = 0; b < 7; b++) out[1 + 7 * f + b] = (uint8_t)(v >> (8 * b));
+    for (int m = 0; m < nttr::EPT; m++) v[0][m] = signed_mod(vals[(int64_t)pp * N + nttr::eA(t, m)], q);
+    nttl::forward_digits<1, true>(v, t, xbuf[l], 1 + l, tw + l * N, q);  // inputs below q: below 15 q through stage 6
+    const uint32_t* add = (pp < KEY_POLYS ? neg_sm + (int64_t)pp * 2 * N : sa_gsw) + l * N;
+#pragma unroll
+    for (int m = 0; m < nttr::EPT; m++) {
+        const int z = nttr::eD(t, m);
+        res[l][z] = addmod(nttr::csub(v[0][m], q), add[z], q);
+    }
+    __syncthreads();
+    for (int z = threadIdx.x; z < N; z += 512) {
+        int64_t field;
+        if (pp < KEY_POLYS) field = 2 * ((int64_t)(pp % 3) * N + z) + pp / 3;  // y and z interleaved per (column, slot)
+        else {
+            const int qi = (pp - KEY_POLYS) / GSW_COLS, c = (pp - KEY_POLYS) % GSW_COLS;
+            field = KEY_POLYS * N + (int64_t)qi * (db_rows + GSW_COLS * N) + db_rows + (int64_t)c * N + z;
+        }
+        put_field(out, field, res[0][z], res[1][z]);
     }
 }
 
-__device__ __forceinline__ uint64_t read_bits_dev(const uint8_t* buf, int64_t bit, int nbits) {
-    const int64_t byte = bit >> 3;
-    const int sh = (int)(bit & 7), nbytes = (sh + nbits + 7) >> 3;  // at most 5 bytes, all inside the field
-    uint64_t v = 0;
-    for (int b = 0; b < nbytes; b++) v |= (uint64_t)buf[byte + b] << (8 * b);
-    return (v >> sh) & ((1ull << nbits) - 1);
+// field i of NB-bit little-endian fields packed from a 4-byte aligned base
+template <int NB>
+__device__ __forceinline__ uint32_t packed_field(const uint32_t* __restrict__ base, int i) {
+    const int bit = NB * i, w = bit >> 5, sh = bit & 31;
+    const uint32_t lo = __ldg(base + w), hi = sh + NB > 32 ? __ldg(base + w + 1) : 0;
+    return __funnelshift_r(lo, hi, sh) & ((1u << NB) - 1);
 }
 
-// recover_how_many: result r's row 0 (28-bit fields, rescaled from q'_2) goes to the limb
-// arrays for the transform, row 1 (20-bit fields, from q'_1) is kept as residues
-__global__ void k_client_unpack(const uint8_t* __restrict__ resp, const int64_t* __restrict__ offsets, int nres,
-                                uint64_t* __restrict__ limb0, uint64_t* __restrict__ limb1,
-                                uint32_t* __restrict__ row1) {
-    const int64_t total = (int64_t)nres * N;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(t / N), i = (int)(t % N);
-        const uint8_t* c = resp + offsets[r];
-        const uint64_t v0 = rescale_any(read_bits_dev(c, 28LL * i, 28), ipr::QP2, QQ);
-        const uint64_t v1 = rescale_any(read_bits_dev(c, 28LL * N + 20LL * i, 20), ipr::QP1, QQ);
-        limb0[t] = v0 % Q0;
-        limb1[t] = v0 % Q1;
-        row1[(int64_t)r * 2 * N + i] = (uint32_t)(v1 % Q0);
-        row1[(int64_t)r * 2 * N + N + i] = (uint32_t)(v1 % Q1);
+// Decryption of one result per CTA: recover_how_many, s * row0 + row1, CRT, rescale to 65535.
+// Row 0 is rescaled from q'_2 = q0 to q = q0 q1, which is the product with q1 exactly (centred), so its
+// residue mod q1 is 0 and only limb 0 is transformed.  Row 1 comes from q'_1 = 2^20:
+// floor((u q + 2^19) / 2^20).  A response was seven launches and is one.
+__global__ void __launch_bounds__(256) k_client_decrypt(const uint8_t* __restrict__ resp, int c_groups,
+                                                        const uint2* __restrict__ tw, const uint32_t* __restrict__ s_ntt,
+                                                        uint32_t ninv, uint32_t ninvp, uint16_t* __restrict__ out) {
+    __shared__ __align__(16) uint32_t xbuf[N];
+    const int t = threadIdx.x, r = blockIdx.x;
+    // framing: u32 count, then per sub-query u32 length and c_groups results
+    const int64_t off = 4 + (int64_t)(r / c_groups) * (4 + (int64_t)c_groups * ipr::RESULT_BYTES) + 4 +
+                        (int64_t)(r % c_groups) * ipr::RESULT_BYTES;
+    const uint32_t* base = reinterpret_cast<const uint32_t*>(resp + off);
+    uint32_t v[1][nttr::EPT];
+#pragma unroll
+    for (int m = 0; m < nttr::EPT; m++) {
+        uint32_t a = packed_field<28>(base, nttr::eA(t, m));
+        if (a >= Q0) a -= Q0;
+        const bool neg = a >= Q0 / 2;
+        const uint32_t x = mulmod32(neg ? Q0 - a : a, Q1 % Q0, Q0, ipr::BR0);  // |row 0| q1 mod q0
+        v[0][m] = neg && x ? Q0 - x : x;
     }
-}
-
-__global__ void k_client_mul_s(uint64_t* __restrict__ limb0, uint64_t* __restrict__ limb1, int nres,
-                               const uint32_t* __restrict__ s_ntt) {
-    const int64_t total = (int64_t)nres * N;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int z = (int)(t % N);
-        limb0[t] = mulmod32((uint32_t)limb0[t], s_ntt[z], Q0, ipr::BR0);
-        limb1[t] = mulmod32((uint32_t)limb1[t], s_ntt[N + z], Q1, ipr::BR1);
-    }
-}
-
-// s * row0 (back in coefficients) + row1, CRT to [0, q), rescale to 65535
-__global__ void k_client_decode(const uint64_t* __restrict__ limb0, const uint64_t* __restrict__ limb1,
-                                const uint32_t* __restrict__ row1, int nres, uint16_t* __restrict__ out) {
-    const int64_t total = (int64_t)nres * N;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(t / N), i = (int)(t % N);
-        const uint32_t d0 = addmod((uint32_t)limb0[t], row1[(int64_t)r * 2 * N + i], Q0);
-        const uint32_t d1 = addmod((uint32_t)limb1[t], row1[(int64_t)r * 2 * N + N + i], Q1);
-        const uint64_t raw = ipr::crt2(d0, d1, ipr::Q0INV, ipr::BR1);
-        out[t] = (uint16_t)rescale_any(raw, QQ, ipr::PT);
+    nttl::forward_digits<1, true>(v, t, xbuf, 1, tw, Q0);
+#pragma unroll
+    for (int m = 0; m < nttr::EPT; m++) v[0][m] = mulmod32(v[0][m], __ldg(s_ntt + nttr::eD(t, m)), Q0, ipr::BR0);
+    nttl::inverse_polys<1, true>(v, t, xbuf, 1, tw + 2 * N, Q0);
+#pragma unroll
+    for (int m = 0; m < nttr::EPT; m++) {
+        const int i = nttr::eA(t, m);
+        const uint32_t b = packed_field<20>(base + 28 * N / 32, i);
+        const bool neg = b >= (1u << 19);
+        const uint64_t u = neg ? (1u << 20) - b : b;
+        const uint64_t lo = u * QQ, hi = __umul64hi(u, QQ), num = lo + (1u << 19);
+        const uint64_t x = (num >> 20) | ((hi + (num < lo)) << 44);  // < q
+        const uint64_t row1 = neg && x ? QQ - x : x;
+        const uint32_t d0 = addmod(nttl::mul_canon(v[0][m], ninv, ninvp, Q0), ipr::mod64(row1, Q0, ipr::BR0), Q0);
+        const uint32_t d1 = ipr::mod64(row1, Q1, ipr::BR1);
+        out[(int64_t)r * N + i] = (uint16_t)ipr::rescale_pt(ipr::crt2m(d0, d1));
     }
 }
 
@@ -296,17 +292,12 @@ struct ipr_client {
     uint32_t* d_sa_row = nullptr; // [rpolys][2][N]
     uint32_t* d_sa_gsw = nullptr; // [2][N]
     uint32_t* d_neg_sm = nullptr; // [2][3][2][N]
+    const uint2* d_tw = nullptr;  // NTT tables of the device
     // scratch, grown on demand
-    uint64_t* d_limb[2] = {nullptr, nullptr};
-    size_t limb_polys = 0;
-    uint64_t* d_fields = nullptr;
-    size_t fields_cap = 0;
+    int64_t* d_polys = nullptr;   // coefficients to transform
+    size_t polys_cap = 0;
     uint8_t* d_bytes = nullptr;   // query bytes out / response bytes in
     size_t bytes_cap = 0;
-    int64_t* d_aux = nullptr;     // targets / result offsets
-    size_t aux_cap = 0;
-    uint32_t* d_row1 = nullptr;
-    size_t row1_cap = 0;
     uint16_t* d_vals = nullptr;
     size_t vals_cap = 0;
 };
@@ -324,22 +315,6 @@ int grow(T*& p, size_t& cap, size_t need) {
         return fail(IPR_E_OOM, "client scratch of %zu bytes", need * sizeof(T));
     }
     cap = need;
-    return IPR_OK;
-}
-
-int ensure_limbs(ipr_client* c, size_t polys) {
-    if (polys <= c->limb_polys && c->d_limb[0]) return IPR_OK;
-    for (auto& p : c->d_limb) {
-        if (p) cudaFree(p);
-        p = nullptr;
-    }
-    c->limb_polys = 0;
-    for (auto& p : c->d_limb)
-        if (cudaMalloc(&p, polys * N * sizeof(uint64_t)) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(IPR_E_OOM, "client transform buffers");
-        }
-    c->limb_polys = polys;
     return IPR_OK;
 }
 
@@ -464,7 +439,8 @@ int ipr_client_create(int device, const ipr_plan* plan, const uint8_t seed[32], 
         (st = upload(&c->d_tau, tau, c->stream)) || (st = upload(&c->d_s_ntt, s_ntt, c->stream)) ||
         (st = upload(&c->d_sa_row, sa_row, c->stream)) || (st = upload(&c->d_sa_gsw, sa_gsw, c->stream)) ||
         (st = upload(&c->d_neg_sm, neg_sm, c->stream)) ||
-        (st = cuda_ok(cudaStreamSynchronize(c->stream), "client setup")))
+        (st = cuda_ok(cudaStreamSynchronize(c->stream), "client setup")) ||
+        (st = ipr::ntt_tables(device, &c->d_tw)))
         return bail(st);
     *out = c;
     return IPR_OK;
@@ -476,36 +452,24 @@ int ipr_client_query(ipr_client* c, uint64_t nonce, unsigned n, const uint64_t* 
     const uint64_t need = ipr::query_bytes(c->plan.db_rows, n);
     if (out_len) *out_len = need;
     if (!out || cap < need) return fail(IPR_E_SPACE, "query needs %llu bytes", (unsigned long long)need);
-    std::vector<int64_t> targets(2 * (size_t)n);
+    Targets tg;
     for (unsigned q = 0; q < n; q++) {
         if (buckets[q] >= c->plan.num_items) return fail(IPR_E_ARGS, "bucket %llu out of range",
                                                              (unsigned long long)buckets[q]);
         const uint64_t col = (buckets[q] % c->per) * c->item_elems;  // build_query_for_index
-        targets[2 * q] = (int64_t)(buckets[q] / c->per);
-        targets[2 * q + 1] = (int64_t)((col % (c->plan.interp * N)) / N);
+        tg.row[q] = (uint32_t)(buckets[q] / c->per);
+        tg.sub[q] = (uint32_t)((col % (c->plan.interp * N)) / N);
     }
     if (cudaSetDevice(c->device) != cudaSuccess) return cuda_ok(cudaGetLastError(), "cudaSetDevice");
-    const int64_t nfields = (int64_t)(need - 1) / 7;
+    const unsigned tp = KEY_POLYS + GSW_COLS * n;
     int st;
-    if ((st = ensure_limbs(c, KEY_POLYS + (size_t)GSW_COLS * n)) ||
-        (st = grow(c->d_aux, c->aux_cap, std::max<size_t>(targets.size(), 1))) ||
-        (st = grow(c->d_fields, c->fields_cap, (size_t)nfields)) || (st = grow(c->d_bytes, c->bytes_cap, need)))
-        return st;
-    if (n && (st = cuda_ok(cudaMemcpyAsync(c->d_aux, targets.data(), targets.size() * sizeof(int64_t),
-                                           cudaMemcpyHostToDevice, c->stream), "targets")))
-        return st;
+    if ((st = grow(c->d_polys, c->polys_cap, (size_t)tp * N)) || (st = grow(c->d_bytes, c->bytes_cap, need))) return st;
     BuildArgs a{c->d_key, 2 + nonce, (int)n, c->rpolys, (int)c->plan.interp, (int64_t)c->plan.db_rows,
-                c->d_s, c->d_tau, c->d_sa_row, c->d_aux, c->d_limb[0], c->d_limb[1], c->d_fields};
+                c->d_s, c->d_tau, c->d_sa_row, c->d_polys, c->d_bytes};
     const int64_t coeffs = (int64_t)(KEY_POLYS + n * (c->rpolys + GSW_COLS)) * N;
-    k_client_build<<<grid_for(coeffs), 256, 0, c->stream>>>(a);
-    if ((st = cuda_ok(cudaGetLastError(), "k_client_build"))) return st;
-    const uint64_t tp = KEY_POLYS + (uint64_t)GSW_COLS * n;
-    for (int l = 0; l < 2; l++)
-        if ((st = ipr_ntt_batch(c->device, c->d_limb[l], tp, l, 0, c->stream))) return st;
-    k_client_finish<<<grid_for((int64_t)tp * N), 256, 0, c->stream>>>(c->d_limb[0], c->d_limb[1], (int)n,
-                                                                       (int64_t)c->plan.db_rows, c->d_neg_sm,
-                                                                       c->d_sa_gsw, c->d_fields);
-    k_client_serialize<<<grid_for(nfields), 256, 0, c->stream>>>(c->d_fields, nfields, (int)n, c->d_bytes);
+    k_client_build<<<grid_for(coeffs), 256, 0, c->stream>>>(a, tg);
+    k_client_transform<<<tp, 512, 0, c->stream>>>(c->d_polys, (int64_t)c->plan.db_rows, c->d_tw, c->d_neg_sm,
+                                                  c->d_sa_gsw, c->d_bytes);
     if ((st = cuda_ok(cudaGetLastError(), "client kernels")) ||
         (st = cuda_ok(cudaMemcpyAsync(out, c->d_bytes, need, cudaMemcpyDeviceToHost, c->stream), "query D2H")) ||
         (st = cuda_ok(cudaStreamSynchronize(c->stream), "client query")))
@@ -526,42 +490,26 @@ int ipr_client_decrypt(ipr_client* c, const uint8_t* response, size_t len, uint1
     uint32_t nq = 0;
     if (!u32(0, &nq)) return fail(IPR_E_FORMAT, "short response");
     const uint64_t per_result = (uint64_t)ipr::RESULT_BYTES, c_groups = c->plan.c;
-    std::vector<int64_t> offsets;
     size_t off = 4;
     for (uint32_t q = 0; q < nq; q++) {
         uint32_t n = 0;
         if (!u32(off, &n) || n != c_groups * per_result || off + 4 + n > len)
             return fail(IPR_E_FORMAT, "response %u: length does not match the plan", q);
-        for (uint64_t w = 0; w < c_groups; w++) offsets.push_back((int64_t)(off + 4 + w * per_result));
         off += 4 + n;
     }
-    const size_t nres = offsets.size(), nvals = nres * N;
+    const size_t nres = (size_t)nq * c_groups, nvals = nres * N;
     if (count) *count = nvals;
     if (!values || cap < nvals) return fail(IPR_E_SPACE, "decryption needs %zu values", nvals);
     if (!nres) return IPR_OK;
     if (cudaSetDevice(c->device) != cudaSuccess) return cuda_ok(cudaGetLastError(), "cudaSetDevice");
     int st;
-    if ((st = ensure_limbs(c, nres)) || (st = grow(c->d_aux, c->aux_cap, nres)) ||
-        (st = grow(c->d_bytes, c->bytes_cap, off)) || (st = grow(c->d_row1, c->row1_cap, nres * 2 * N)) ||
-        (st = grow(c->d_vals, c->vals_cap, nres * N)))
+    if ((st = grow(c->d_bytes, c->bytes_cap, off)) || (st = grow(c->d_vals, c->vals_cap, nres * N))) return st;
+    if ((st = cuda_ok(cudaMemcpyAsync(c->d_bytes, response, off, cudaMemcpyHostToDevice, c->stream), "response")))
         return st;
-    if ((st = cuda_ok(cudaMemcpyAsync(c->d_bytes, response, off, cudaMemcpyHostToDevice, c->stream), "response")) ||
-        (st = cuda_ok(cudaMemcpyAsync(c->d_aux, offsets.data(), nres * sizeof(int64_t), cudaMemcpyHostToDevice,
-                                      c->stream), "offsets")))
-        return st;
-    const int64_t work = (int64_t)nres * N;
-    k_client_unpack<<<grid_for(work), 256, 0, c->stream>>>(c->d_bytes, c->d_aux, (int)nres, c->d_limb[0],
-                                                           c->d_limb[1], c->d_row1);
-    if ((st = cuda_ok(cudaGetLastError(), "k_client_unpack"))) return st;
-    for (int l = 0; l < 2; l++)
-        if ((st = ipr_ntt_batch(c->device, c->d_limb[l], nres, l, 0, c->stream))) return st;
-    k_client_mul_s<<<grid_for(work), 256, 0, c->stream>>>(c->d_limb[0], c->d_limb[1], (int)nres, c->d_s_ntt);
-    if ((st = cuda_ok(cudaGetLastError(), "k_client_mul_s"))) return st;
-    for (int l = 0; l < 2; l++)
-        if ((st = ipr_ntt_batch(c->device, c->d_limb[l], nres, l, 1, c->stream))) return st;
-    k_client_decode<<<grid_for(work), 256, 0, c->stream>>>(c->d_limb[0], c->d_limb[1], c->d_row1, (int)nres,
-                                                           c->d_vals);
-    if ((st = cuda_ok(cudaGetLastError(), "k_client_decode")) ||
+    const uint32_t ninv = Q0 - (Q0 - 1) / N;  // N^-1 mod q0
+    k_client_decrypt<<<(unsigned)nres, 256, 0, c->stream>>>(c->d_bytes, (int)c_groups, c->d_tw, c->d_s_ntt, ninv,
+                                                            (uint32_t)(((uint64_t)ninv << 32) / Q0), c->d_vals);
+    if ((st = cuda_ok(cudaGetLastError(), "k_client_decrypt")) ||
         (st = cuda_ok(cudaMemcpyAsync(values, c->d_vals, nvals * sizeof(uint16_t), cudaMemcpyDeviceToHost,
                                       c->stream), "values D2H")) ||
         (st = cuda_ok(cudaStreamSynchronize(c->stream), "client decrypt")))
@@ -635,8 +583,8 @@ void ipr_client_destroy(ipr_client* c) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    void* ps[] = {c->d_key, c->d_s, c->d_tau, c->d_s_ntt, c->d_sa_row, c->d_sa_gsw, c->d_neg_sm, c->d_limb[0],
-                  c->d_limb[1], c->d_fields, c->d_bytes, c->d_aux, c->d_row1, c->d_vals};
+    void* ps[] = {c->d_key,    c->d_s,      c->d_tau,   c->d_s_ntt, c->d_sa_row,
+                  c->d_sa_gsw, c->d_neg_sm, c->d_polys, c->d_bytes, c->d_vals};
     for (void* p : ps)
         if (p) cudaFree(p);
     if (c->stream) cudaStreamDestroy(c->stream);

@@ -106,6 +106,47 @@ __device__ __forceinline__ uint64_t crt2m(uint32_t x, uint32_t y) {
 }
 
 // ---------------------------------------------------------------------------
+// rescale (src/core/arith.rs:436-452): round(v * out / q) for a canonical v, centred at 0, taken
+// mod out; the modulus switch to q'_2 = q0 and q'_1 = 2^20 and the decoding to 65535.  All are
+// floor((u * out + floor(q / 2)) / q) of u = |v|, without a 128-bit division:
+//   out = q0: floor((u q0 + floor(q0 q1 / 2)) / (q0 q1)) = floor((u + (q1 - 1) / 2) / q1)
+//   out < 2^20 + 1: the quotient from a reciprocal of q is at most 2 too small; the remainder fits 64 bits
+// ---------------------------------------------------------------------------
+constexpr uint64_t INVQ = (uint64_t)(((unsigned __int128)1 << 119) / QQ);  // floor(2^119 / q) < 2^64
+
+template <typename F>
+__device__ __forceinline__ uint32_t rescale_centred(uint64_t v, uint32_t out, F quotient) {
+    const bool neg = v >= QQ / 2;
+    const uint32_t r = quotient(neg ? QQ - v : v);
+    const uint32_t rm = r >= out ? r - out : r;  // r <= out / 2 + 1
+    return neg ? (rm ? out - rm : 0) : rm;
+}
+__device__ __forceinline__ uint32_t fix_quotient(uint64_t r, uint64_t num) {
+    uint64_t rem = num - r * QQ;  // below 3 q < 2^58, so 64-bit arithmetic is exact
+    if (rem >= QQ) rem -= QQ, r++;
+    if (rem >= QQ) r++;
+    return (uint32_t)r;
+}
+__device__ __forceinline__ uint32_t rescale_q0(uint64_t v) {
+    return rescale_centred(v, Q0, [](uint64_t u) {
+        const uint64_t x = u + (Q1 - 1) / 2;
+        uint64_t t = __umul64hi(x, BR1);  // floor(x / q1), at most one too small
+        if (x - t * Q1 >= Q1) t++;
+        return (uint32_t)t;
+    });
+}
+__device__ __forceinline__ uint32_t rescale_2p20(uint64_t v) {
+    return rescale_centred(v, 1u << 20, [](uint64_t u) {
+        return fix_quotient(__umul64hi(u, INVQ) >> 35, (u << 20) + QQ / 2);
+    });
+}
+__device__ __forceinline__ uint32_t rescale_pt(uint64_t v) {
+    return rescale_centred(v, PT, [](uint64_t u) {
+        return fix_quotient(((__umul64hi(u, INVQ) >> 8) * PT) >> 47, u * PT + QQ / 2);
+    });
+}
+
+// ---------------------------------------------------------------------------
 // Shared-memory negacyclic NTTs over u32 residues, executed cooperatively by
 // all threads of a CTA on `npoly` independent polynomials laid out at
 // smem + p * N.  Twiddles: w/wp for forward (bit-reversed psi powers) and the

@@ -170,6 +170,8 @@ int cuda_status(cudaError_t e) {
 }
 
 }  // namespace
+
+int ntt_tables(int device, const uint2** out) { return tables_for(device, out); }
 }  // namespace ipr
 
 extern "C" {
