@@ -29,7 +29,7 @@ namespace ipr {
 void set_last_error(const char* msg);
 cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar_all, int64_t cols,
                                     const uint32_t* wrows, const uint32_t* vmask, const uint32_t* tab, uint32_t* F,
-                                    uint32_t* r0, uint64_t* xb, uint32_t* itab, uint64_t* bt, uint64_t* btb,
+                                    uint32_t* r0, uint64_t* xb, uint32_t* itab, int* err_flag, uint64_t* bt, uint64_t* btb,
                                     uint64_t* bth, uint64_t* a_hat, cudaStream_t st);
 cudaError_t narrow_u64(const uint64_t* in, int64_t n, uint32_t* out, cudaStream_t st);
 cudaError_t offline_jntt(const uint32_t* act, int64_t inst, const uint32_t* fw, const uint32_t* fwp, uint32_t* E,
@@ -452,9 +452,10 @@ void run_collapse(CollapseSet& out, int num_cols, int nph, int t_exp, int bits_p
     }
     // the chains of at most 64 columns at a time share one F buffer
     const int chunk = num_cols < 64 ? num_cols : 64;
-    uint32_t *F = nullptr, *r0 = nullptr, *itab = nullptr;
+    uint32_t *F = nullptr, *r0 = nullptr, *itab = nullptr;  // itab: the tables, then the error flag
     uint64_t* xb = nullptr;
-    if (report(cudaMalloc(&itab, 8 * N * 4), "collapse scratch") ||
+    if (report(cudaMalloc(&itab, 8 * N * 4 + 16), "collapse scratch") ||
+        report(cudaMemset(itab + 8 * N, 0, sizeof(int)), "collapse scratch") ||
         report(cudaMalloc(&F, (size_t)chunk * 2 * HALF * CC * 4), "collapse scratch") ||
         report(cudaMalloc(&r0, (size_t)chunk * CC * 4), "collapse scratch") ||
         report(cudaMalloc(&xb, (size_t)chunk * N * 8), "collapse scratch")) {
@@ -468,12 +469,15 @@ void run_collapse(CollapseSet& out, int num_cols, int nph, int t_exp, int bits_p
         const int n = num_cols - c0 < chunk ? num_cols - c0 : chunk;
         const size_t ro = (size_t)c0 * HALF * CC;
         if (report(offline_collapse_arrays(C.r_all + ro, C.r_bar_all + ro, n, C.wrows, C.vmask, C.tab32, F, r0, xb, itab,
+                                           reinterpret_cast<int*>(itab + 8 * N),
                                            out.bt + (size_t)c0 * NINNER * N, out.btb + (size_t)c0 * NINNER * N,
                                            out.bth + (size_t)c0 * 3 * N, out.a_hat + (size_t)c0 * N, nullptr),
                    "collapse"))
             break;
     }
-    report(cudaDeviceSynchronize(), "collapse");
+    int flag = 0;
+    if (!report(cudaMemcpy(&flag, itab + 8 * N, sizeof(int), cudaMemcpyDeviceToHost), "collapse") && flag)
+        report_msg("gpu_collapse_run: a device-side wait ran out");
     dfree(itab);
     dfree(F);
     dfree(r0);

@@ -55,16 +55,17 @@ __device__ __forceinline__ uint64_t add_q(uint64_t a, uint64_t b) {  // a, b < q
     return v >= QQ ? v - QQ : v;
 }
 
-__device__ __forceinline__ uint64_t rescale_q(uint64_t v, uint64_t out_mod) {
-    // rescale (src/core/arith.rs:436-452) of a canonical v in [0, q)
-    const uint64_t half = QQ / 2;
-    const bool neg = v >= half;
-    const uint64_t u = neg ? QQ - v : v;
-    const unsigned __int128 num = (unsigned __int128)u * out_mod + half;
-    const uint64_t rr = (uint64_t)(num / QQ);
-    const uint64_t rm = rr % out_mod;
-    return neg ? (rm ? out_mod - rm : 0) : rm;
+// sum of three transformed digits (each below 10q) to below 8q: the fold's digit sums need no
+// tighter bound, since row 0 times two of them stays below 16 q^2 <= q 2^32
+__device__ __forceinline__ uint32_t sum3(uint32_t a, uint32_t b, uint32_t c, uint32_t q) {
+    const uint32_t s = csub(csub(a, 8 * q) + csub(b, 8 * q), 8 * q);
+    return csub(s + csub(c, 8 * q), 8 * q);
 }
+
+// out of line: inlined, the once-per-chain rescales cost the step loop registers (the four-CTA fold
+// ran 188 us instead of 167)
+__device__ __noinline__ uint32_t switch_row0(uint64_t v) { return rescale_q0(v); }
+__device__ __noinline__ uint32_t switch_row1(uint64_t v) { return rescale_2p20(v); }
 
 // switch_and_keep (src/pir/modulus_switch.rs:45-73) of thread t's coefficients e = t + 256 m of s:
 // row 0 -> 28-bit fields (2 per 7 bytes), row 1 -> 20-bit fields (2 per 5 bytes), LSB first;
@@ -73,7 +74,7 @@ template <typename SA>
 __device__ __forceinline__ void switch_keep(SA S_AT, int t, uint8_t* __restrict__ out) {
 #pragma unroll
     for (int m = 0; m < EPT; m++) {
-        const uint64_t a = rescale_q(S_AT(0, m), QP2), b = rescale_q(S_AT(1, m), QP1);
+        const uint64_t a = switch_row0(S_AT(0, m)), b = switch_row1(S_AT(1, m));
         const uint64_t an = __shfl_down_sync(0xffffffffu, a, 1), bn = __shfl_down_sync(0xffffffffu, b, 1);
         if (!(t & 1)) {
             const int tt = eA(t, m) >> 1;
@@ -365,8 +366,8 @@ __global__ void __launch_bounds__(F4_THREADS, STAGE ? 2 : 3)
 #pragma unroll
         for (int l = 0; l < 2; l++) {
             const uint32_t q = l ? Q1 : Q0;
-            // acc0: the six digit transforms' sum (< 12q); acc1: the packing output plus each
-            // batch's Montgomery-reduced MAC (< q + 2 x 2q = 5q), canonicalised after both batches
+            // acc0: the six digit transforms' sum (< 16q); acc1: the packing output plus each
+            // batch's Montgomery-reduced MAC (< q + 2 x 3q = 7q), canonicalised after both batches
             uint32_t acc0[EPT], acc1[EPT];
 #pragma unroll
             for (int m = 0; m < EPT; m++) acc0[m] = 0;
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(F4_THREADS, STAGE ? 2 : 3)
 #pragma unroll
                     for (int k = 0; k < 3; k++) v[k][m] = (uint32_t)((x >> (k * GADGET_BITS)) & mask);
                 }
-                forward_digits<3>(v, t, xbuf, bar, fwi + l * N, q);
+                forward_digits<3, false, true>(v, t, xbuf, bar, fwi + l * N, q);
                 if (l == 1 && r == 1) {
                     // s is consumed (the team barriers of the transforms ordered every read of
                     // it): the packed row j lands in its slots while the inverse transforms run
@@ -450,12 +451,14 @@ __global__ void __launch_bounds__(F4_THREADS, STAGE ? 2 : 3)
                     const uint32_t bv[EPT] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
                     for (int m = 0; m < EPT; m++) {
-                        acc0[m] += v[k][m];                    // 6 terms < 12q < 2^32
-                        part[m] += (uint64_t)bv[m] * v[k][m];  // 3 terms < 6 q^2 < q 2^32
+                        part[m] += (uint64_t)bv[m] * v[k][m];  // 3 terms < 30 q^2 < 2^61: redc < 3q
                     }
                 }
 #pragma unroll
-                for (int m = 0; m < EPT; m++) acc1[m] += redc(part[m], q);
+                for (int m = 0; m < EPT; m++) {
+                    acc0[m] += sum3(v[0][m], v[1][m], v[2][m], q);
+                    acc1[m] += redc(part[m], q);
+                }
             }
             uint32_t r0[EPT];
             if constexpr (STAGE) {
@@ -468,8 +471,8 @@ __global__ void __launch_bounds__(F4_THREADS, STAGE ? 2 : 3)
             }
 #pragma unroll
             for (int m = 0; m < EPT; m++) {
-                pr[2 * l][m] = csub(redc((uint64_t)r0[m] * acc0[m], q), q);  // < 12 q^2 < q 2^32
-                pr[2 * l + 1][m] = csub(csub(csub(acc1[m], 4 * q), 2 * q), q);  // < 5q -> [0, q)
+                pr[2 * l][m] = csub(redc((uint64_t)r0[m] * acc0[m], q), q);  // < 16 q^2 < q 2^32
+                pr[2 * l + 1][m] = csub(csub(csub(acc1[m], 4 * q), 2 * q), q);  // < 7q -> [0, q)
             }
         }
         inverse_limbs<2, 2>(pr, t, xbuf, bar, iwi);
@@ -494,24 +497,29 @@ __global__ void __launch_bounds__(F4_THREADS, STAGE ? 2 : 3)
 // 8 coefficients of layout A).  A step is a chain of dependent transforms, so with few chains
 // the time is its latency: here it holds one forward batch and one single inverse transform
 // where k_fold4 runs four and four, and each CTA has an SM's schedulers for itself.
-// 31 steps of up to 32 chains: 167 us (5.4 us a step), against 474 us for k_fold4; from about
+// 31 steps of up to 32 chains: 150 us (4.8 us a step), against 460 us for k_fold4; from about
 // 0.4 chains per SM on it is bound by issue like k_fold4, at a fifth more work per chain (both
 // limbs' CTAs compose s), so the server picks the form by the number of chains.
+// The exchanges are asynchronous stores that count on an mbarrier of the receiver (a cluster
+// barrier per exchange cost a memory barrier of about 1,000 of the step's 10,800 cycles).  Each
+// buffer has two halves used in turn: a CTA sends into a half again only after it has received
+// what its partner sent after reading that half.  A wait that runs out is remembered, later
+// waits are skipped, the chain runs on to the common last barrier and the error is reported.
 // Shared memory: exchange buffer 24 KB, bodies and row 0 / S staged by cp.async 32 KB, the two
-// exchange slots 16 KB.
-constexpr int FC_SMEM = (3 + 4 + 2) * N * 4;
+// exchanges' slots 32 KB, four mbarriers.
+constexpr int FC_SMEM = (3 + 4 + 4) * N * 4 + 64;
 
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
     k_fold_cluster(const uint32_t* __restrict__ row0s, const uint32_t* __restrict__ gsw,
                    const uint64_t* __restrict__ a_hat, const uint32_t* __restrict__ S, int64_t s_payload_stride,
                    const uint64_t* __restrict__ cvec, const uint2* __restrict__ fwi, const uint2* __restrict__ iwi,
                    int interp, int64_t db_cols, int qpp, uint8_t* __restrict__ resp, int64_t resp_payload_stride,
-                   int64_t resp_query_stride, FoldExtents ext) {
+                   int64_t resp_query_stride, FoldExtents ext, int* __restrict__ err_flag) {
     extern __shared__ uint4 fc_smem[];
     uint32_t* xbuf = reinterpret_cast<uint32_t*>(fc_smem);  // [3][N]
     uint32_t* stg = xbuf + 3 * N;                           // [4][N]: bodies of digits 0..2, row 0 or S
-    uint32_t* ex1 = stg + 4 * N;                            // [8][256] from CTA (l, 1 - r)
-    uint32_t* ex2 = ex1 + N;                                // [8][256] from CTA (1 - l, r)
+    uint4* ex = reinterpret_cast<uint4*>(stg + 4 * N);      // [2 exchanges][2 halves][2][256]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ex + 8 * 256);  // [2 exchanges][2 halves]
     const int t = threadIdx.x;
     const int rank = (int)umma::cluster_rank(), l = rank & 1, r = rank >> 1;
     const int wp = blockIdx.x >> 2, qg = blockIdx.y;
@@ -537,27 +545,43 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
 #pragma unroll
         for (int m = 0; m < EPT; m++) pk[m] = ok ? __ldg(pk_src + (int64_t)j * N + eA(t, m)) : 0;
     };
-    // pr -> x: inverse transform, residues of the other limb, CRT, + packed row
-    auto to_s = [&]() {
-        inverse_one<true>(pr, t, xbuf, 1, iw, q);
-#pragma unroll
-        for (int m = 0; m < EPT; m++) st_peer(ex2 + m * 256 + t, rank ^ 1, pr[m]);
-        umma::cluster_sync();
-#pragma unroll
-        for (int m = 0; m < EPT; m++) {
-            const uint32_t o = ex2[m * 256 + t];
-            x[m] = add_q(l ? crt2m(o, pr[m]) : crt2m(pr[m], o), pk[m]);
-        }
+    bool ok = true;
+    // exchange e, its n-th use: this thread's 8 words to the same thread of CTA `peer`, that thread's in return
+    auto exchange = [&](int e, uint32_t n, int peer, const uint32_t (&w)[EPT], uint32_t (&o)[EPT]) {
+        const int slot = e * 2 + (int)(n & 1);
+        uint64_t* bar = bars + slot;
+        uint4* buf = ex + slot * 512;
+        if (t == 0) umma::mbar_expect_tx(bar, 2 * 256 * 16);
+        const uint32_t pb = umma::map_to_rank(bar, (uint32_t)peer), pd = umma::map_to_rank(buf + t, (uint32_t)peer);
+        umma::st_async16(pd, w[0], w[1], w[2], w[3], pb);
+        umma::st_async16(pd + 256 * 16, w[4], w[5], w[6], w[7], pb);
+        if (ok) ok = umma::mbar_wait_cluster(bar, (n >> 1) & 1);
+        const uint4 a = buf[t], b = buf[256 + t];
+        o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+        o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
     };
-    umma::cluster_sync();  // every CTA of the cluster runs: its shared memory may be written
+    // pr -> x: inverse transform, residues of the other limb, CRT, + packed row
+    auto to_s = [&](uint32_t n) {
+        inverse_one<true>(pr, t, xbuf, 1, iw, q);
+        uint32_t o[EPT];
+        exchange(1, n, rank ^ 1, pr, o);
+#pragma unroll
+        for (int m = 0; m < EPT; m++) x[m] = add_q(l ? crt2m(o[m], pr[m]) : crt2m(pr[m], o[m]), pk[m]);
+    };
+    if (t == 0) {
+        for (int i = 0; i < 4; i++) umma::mbar_init(bars + i, 1);
+        umma::fence_mbar_init();
+    }
+    umma::cluster_sync();  // every CTA of the cluster runs and its mbarriers may be signalled
     {  // first step: G^-1(0) = 0, so s = (a_hat[j], INTT(S[j]) + c[j]) mod q
         const int j = wp * interp + interp - 1;
         load_pk(j);
 #pragma unroll
         for (int m = 0; m < EPT; m++) pr[m] = 0;
         if (r && s_ok((int64_t)j * 2 + l)) load_d8(pr, Sq + ((int64_t)j * 2 + l) * N + z8);
-        to_s();
+        to_s(0);
     }
+    uint32_t n = 0;  // steps done
     for (int step = interp - 2; step >= 0; step--) {
         const int j = wp * interp + step;
 #pragma unroll
@@ -579,44 +603,46 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
         for (int m = 0; m < EPT; m++)
 #pragma unroll
             for (int k = 0; k < 3; k++) v[k][m] = (uint32_t)((x[m] >> (k * GADGET_BITS)) & mask);
-        forward_digits<3, true>(v, t, xbuf, 1, fw, q);
+        forward_digits<3, true, true>(v, t, xbuf, 1, fw, q);
         load_pk(j);
         cp_wait<0>();
-        uint32_t acc0[EPT], acc1[EPT];  // digit sum (< 6q), Montgomery-reduced product (< 2q)
+        uint32_t acc0[EPT], acc1[EPT];  // digit sum (< 8q), Montgomery-reduced product (< 3q)
         {
             uint64_t part[EPT];
 #pragma unroll
-            for (int m = 0; m < EPT; m++) {
-                acc0[m] = 0;
-                part[m] = 0;
-            }
+            for (int m = 0; m < EPT; m++) part[m] = 0;
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 const uint4 b0 = *reinterpret_cast<const uint4*>(stg + k * N + z8);
                 const uint4 b1 = *reinterpret_cast<const uint4*>(stg + k * N + z8 + 4);
                 const uint32_t bv[EPT] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-                for (int m = 0; m < EPT; m++) {
-                    acc0[m] += v[k][m];
-                    part[m] += (uint64_t)bv[m] * v[k][m];  // 3 terms < 6 q^2 < q 2^32
-                }
+                for (int m = 0; m < EPT; m++) part[m] += (uint64_t)bv[m] * v[k][m];  // 3 terms < 30 q^2 < 2^61
             }
 #pragma unroll
-            for (int m = 0; m < EPT; m++) acc1[m] = redc(part[m], q);
+            for (int m = 0; m < EPT; m++) {
+                acc0[m] = sum3(v[0][m], v[1][m], v[2][m], q);
+                acc1[m] = redc(part[m], q);
+            }
         }
+        uint32_t snd[EPT], o[EPT];
 #pragma unroll
-        for (int m = 0; m < EPT; m++) st_peer(ex1 + m * 256 + t, rank ^ 2, r ? acc0[m] : acc1[m]);
-        umma::cluster_sync();
+        for (int m = 0; m < EPT; m++) snd[m] = r ? acc0[m] : acc1[m];
+        exchange(0, n, rank ^ 2, snd, o);
         const uint4 e0 = *reinterpret_cast<const uint4*>(stg + 3 * N + z8);
         const uint4 e1 = *reinterpret_cast<const uint4*>(stg + 3 * N + z8 + 4);
         const uint32_t ev[EPT] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
 #pragma unroll
         for (int m = 0; m < EPT; m++) {
-            const uint32_t o = ex1[m * 256 + t];
-            if (r) pr[m] = csub(csub(csub(acc1[m] + o + ev[m], 4 * q), 2 * q), q);  // < 5q
-            else pr[m] = csub(redc((uint64_t)ev[m] * (acc0[m] + o), q), q);         // < 12 q^2 < q 2^32
+            if (r) pr[m] = csub(csub(csub(acc1[m] + o[m] + ev[m], 4 * q), 2 * q), q);  // < 7q
+            else pr[m] = csub(redc((uint64_t)ev[m] * (acc0[m] + o[m]), q), q);      // < 16 q^2 < q 2^32
         }
-        to_s();
+        to_s(++n);
+    }
+    umma::cluster_sync();  // every store into this CTA has landed
+    if (!__syncthreads_and(ok)) {
+        if (t == 0) atomicExch(err_flag, 32);
+        return;
     }
     // switch_and_keep of row r, as switch_keep; the two limbs' CTAs take half of the fields each
     const int64_t ro = (int64_t)payload * resp_payload_stride + 8 + (int64_t)qin * resp_query_stride +
@@ -626,7 +652,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
 #pragma unroll
     for (int mm = 0; mm < EPT / 2; mm++) {
         const int m = l * (EPT / 2) + mm;
-        const uint64_t a = rescale_q(l ? x[EPT / 2 + mm] : x[mm], r ? QP1 : QP2);
+        const uint64_t xv = l ? x[EPT / 2 + mm] : x[mm];
+        const uint64_t a = r ? switch_row1(xv) : switch_row0(xv);
         const uint64_t an = __shfl_down_sync(0xffffffffu, a, 1);
         if (t & 1) continue;
         const int tt = eA(t, m) >> 1;
@@ -698,7 +725,7 @@ cudaError_t launch_fold4(const uint32_t* row0s, const uint32_t* gsw_scaled, cons
                          int64_t s_payload_stride, const uint64_t* cvec, const uint32_t* fwi, const uint32_t* iwi,
                          int interp, int c_groups, int num_queries, int64_t db_cols, int qpp, uint8_t* resp,
                          int64_t resp_payload_stride, int64_t resp_query_stride, const FoldExtents& ext,
-                         cudaStream_t st, FoldForm form) {
+                         cudaStream_t st, FoldForm form, int* err_flag) {
     if (interp < 1 || c_groups < 1 || num_queries < 1 || num_queries > 65535 || qpp < 1) return cudaErrorInvalidValue;
     cudaError_t e;
     if ((e = check_extent(row0s, 2ull * N * 4, "fold: row 0")) != cudaSuccess ||
@@ -715,7 +742,7 @@ cudaError_t launch_fold4(const uint32_t* row0s, const uint32_t* gsw_scaled, cons
     if (form == FoldForm::kCluster)
         k_fold_cluster<<<dim3(4 * c_groups, num_queries), 256, FC_SMEM, st>>>(
             row0s, gsw_scaled, a_hat, S, s_payload_stride, cvec, fw, iw, interp, db_cols, qpp, resp,
-            resp_payload_stride, resp_query_stride, ext);
+            resp_payload_stride, resp_query_stride, ext, err_flag);
     else if (form == FoldForm::kStaged)
         k_fold4<true><<<grid, F4_THREADS, F4_SMEM, st>>>(row0s, gsw_scaled, a_hat, S, s_payload_stride, cvec, fw, iw,
                                                          interp, c_groups, db_cols, qpp, resp, resp_payload_stride,

@@ -134,10 +134,10 @@ __device__ __forceinline__ void xchg_b2a(uint32_t (&v)[P][EPT], int t, uint32_t*
 }
 
 // forward NTT of P gadget-digit polynomials (< 2^19) of one limb: layout A in, layout D out
-// in [0, 2q); xbuf holds XP >= P polynomials of this team.  Bounds: after stage s <= 6 every
+// in [0, 2q), or below 10q with RAW; xbuf holds XP >= P polynomials of this team.  Bounds: after stage s <= 6 every
 // value is below 2^19 + 2q (s + 1) <= 2^19 + 14q; stage 7 reduces x first (outputs < 4q);
 // stages 8..10 add 2q each (< 10q < 2^32); one reduction at the end.
-template <int P, bool HOIST = false>
+template <int P, bool HOIST = false, bool RAW = false>
 __device__ __forceinline__ void forward_digits(uint32_t (&v)[P][EPT], int t, uint32_t* xbuf, int bar,
                                                const uint2* __restrict__ tw, uint32_t q) {
     const int l = t & 31, w = t >> 5;
@@ -157,10 +157,12 @@ __device__ __forceinline__ void forward_digits(uint32_t (&v)[P][EPT], int t, uin
     nttr::c_to_d<P>(v, l, wb);
     fstage<P, 0, 2, 1, HOIST>(v, 9, hd, tw, q);
     fstage<P, 0, 1, 1, HOIST>(v, 10, hd, tw, q);
+    if constexpr (!RAW) {
 #pragma unroll
-    for (int p = 0; p < P; p++)
+        for (int p = 0; p < P; p++)
 #pragma unroll
-        for (int k = 0; k < EPT; k++) v[p][k] = red16(v[p][k], q);
+            for (int k = 0; k < EPT; k++) v[p][k] = red16(v[p][k], q);
+    }
 }
 
 // Gentleman-Sande butterfly with a plain inverse twiddle: x + y, (x - y) * w.  Inputs below
@@ -277,13 +279,6 @@ __device__ __forceinline__ void load_d8(uint32_t (&r)[EPT], const uint32_t* __re
 
 __device__ __forceinline__ uint32_t mul_canon(uint32_t x, uint32_t w, uint32_t wp, uint32_t q) {
     return csub(shoup_lazy(x, w, wp, q), q);
-}
-
-// 32-bit store into the shared memory of CTA `rank` of the cluster, at this CTA's address p
-__device__ __forceinline__ void st_peer(const void* p, uint32_t rank, uint32_t v) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
 }  // namespace nttl

@@ -210,8 +210,8 @@ struct CollapseScale {
 struct ChainSmem {
     uint32_t xb[3][N];            // exchange buffer of the transforms
     uint32_t wm[3][N];            // this limb's W mask times N^-1 R
-    uint32_t pr[2][EPT][256];     // the other limb's residues of x, double buffered by step
-    uint32_t pv[2][3 * 4][256];   // the other limb's transformed digits, half of the slots
+    uint4 ex[2][5][256];          // from the other limb, halves used in turn: x's residues (2), digits (3)
+    uint64_t bars[2];
 };
 
 constexpr uint32_t INV5 = 3277;  // 5^-1 mod 2N
@@ -233,22 +233,25 @@ __device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8]) {
 // Bound by the latency of a step where chains are few and by instruction issue where they
 // fill the chip: 1023 dependent steps of three forward transforms, a product and one inverse
 // transform per limb.  A limb needs the other only for the CRT, so each has an SM's
-// schedulers to itself, and one exchange through distributed shared memory per step carries
-// the residues (both CTAs then compose x, which thread t keeps as its 8 coefficients of layout
-// A).  The same exchange carries half of the transformed digits, so that each CTA stores
-// whole 32-byte sectors of the interleaved bold_t rows.  The transforms are the fold's lazily
+// schedulers to itself, and one exchange per step through distributed shared memory
+// (asynchronous stores counted on an mbarrier of the receiver) carries the residues; both CTAs
+// then compose x, which thread t keeps as its 8 coefficients of layout A.  The same exchange
+// carries half of the transformed digits, so that each CTA stores whole 32-byte sectors of the
+// interleaved bold_t rows.  A CTA sends into a half of the exchange buffer again only after it
+// has received what its partner sent after reading that half.  A wait that runs out is
+// remembered, later waits are skipped, the chain runs on to the common last barrier and the
+// error is reported.  The transforms are the fold's lazily
 // reduced ones; their N^-1 sits in the W mask (with the Montgomery R) and in F.
-// 1 / 148 chain pairs of two at a time per SM: 5.0 / 8.0 us a step (37% and about 50% of the
-// issue slots; the rest is dependent latency, the exchange about a tenth of a step), against
+// One instance (2 chains) 4.6 us a step, 74 instances (two chains' CTAs per SM) 7.5 us, against
 // 14 us a step for one 512-thread CTA per chain, which also stored bold_t in 4-byte pieces.
-// One instance (2 chains) 14.4 -> 5.2 ms, 74 instances 21 -> 8.2 ms.  More registers (one CTA
-// per SM, 138 instead of 128) measured the same.
+// A cluster barrier per exchange in place of the counted stores: 5.0 us (its memory barrier);
+// more registers (one CTA per SM, 138 instead of 128) measured the same.
 template <bool WROWS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
     k_off_collapse(const uint32_t* __restrict__ F, int64_t inst0, const uint32_t* __restrict__ wmask,
                    const uint2* __restrict__ fwi, const uint2* __restrict__ iwi, CollapseScale sc,
                    uint64_t* __restrict__ bt, uint64_t* __restrict__ btb, uint32_t* __restrict__ r0,
-                   uint64_t* __restrict__ xbar0, const uint32_t* __restrict__ wrows) {
+                   uint64_t* __restrict__ xbar0, const uint32_t* __restrict__ wrows, int* __restrict__ err_flag) {
     extern __shared__ __align__(16) uint8_t csm_raw[];
     ChainSmem& sm = *reinterpret_cast<ChainSmem*>(csm_raw);
     const int t = threadIdx.x;
@@ -269,27 +272,42 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
     const uint32_t ez = exponent_of_slot((uint32_t)z8);
     uint64_t x[EPT];
     uint32_t y[EPT];
-    // y (N^-1 times the limb's values, layout D) -> x: inverse transform, exchange, CRT
-    auto to_raw2 = [&](int par) {
-        nttl::inverse_one(y, t, &sm.xb[0][0], 1, iw, q);
-#pragma unroll
-        for (int m = 0; m < EPT; m++) nttl::st_peer(&sm.pr[par][m][t], peer, y[m]);
-        umma::cluster_sync();
-#pragma unroll
-        for (int m = 0; m < EPT; m++) {
-            const uint32_t o = sm.pr[par][m][t];
-            x[m] = g ? crt2m(o, y[m]) : crt2m(y[m], o);
-        }
+    bool ok = true;
+    // 16 bytes of step use n to slot k of the same thread of the other CTA
+    auto send = [&](uint32_t n, int k, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+        umma::st_async16(umma::map_to_rank(&sm.ex[n & 1][k][t], (uint32_t)peer), w0, w1, w2, w3,
+                         umma::map_to_rank(&sm.bars[n & 1], (uint32_t)peer));
     };
+    auto receive = [&](uint32_t n, uint32_t bytes) {  // thread 0 says how many bytes this use counts
+        if (t == 0) umma::mbar_expect_tx(&sm.bars[n & 1], bytes);
+        if (ok) ok = umma::mbar_wait_cluster(&sm.bars[n & 1], (n >> 1) & 1);
+    };
+    // y (N^-1 times the limb's values, layout D) -> x: inverse transform, exchange, CRT
+    auto to_raw2 = [&](uint32_t n, uint32_t bytes) {
+        nttl::inverse_one(y, t, &sm.xb[0][0], 1, iw, q);
+        send(n, 0, y[0], y[1], y[2], y[3]);
+        send(n, 1, y[4], y[5], y[6], y[7]);
+        receive(n, bytes);
+        const uint4 a = sm.ex[n & 1][0][t], b = sm.ex[n & 1][1][t];
+        const uint32_t o[EPT] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int m = 0; m < EPT; m++) x[m] = g ? crt2m(o[m], y[m]) : crt2m(y[m], o[m]);
+    };
+    if (t == 0) {
+        umma::mbar_init(&sm.bars[0], 1);
+        umma::mbar_init(&sm.bars[1], 1);
+        umma::fence_mbar_init();
+    }
     // x = raw(r_all[1023]): r_all[1023] is never updated (packing.rs:2691)
     nttl::load_d8(y, Fc + (int64_t)(HALF - 1) * 2 * N + z8);
 #pragma unroll
     for (int m = 0; m < EPT; m++) y[m] = nttl::mul_canon(y[m], nv, nvp, q);
-    umma::cluster_sync();  // both CTAs run (their shared memory is addressable) and wm is loaded
-    to_raw2(1);
+    umma::cluster_sync();  // both CTAs run, their mbarriers may be signalled, and wm is loaded
+    to_raw2(0, 2 * 256 * 16);
+    uint32_t n = 0;  // exchanges done since
     uint32_t gi = gen_pow(HALF - 2);
     for (int i = HALF - 2; i >= 0; i--) {
-        const int par = i & 1;
+        n++;
         uint32_t f[EPT];
         nttl::load_d8(f, Fc + (int64_t)i * 2 * N + z8);
         uint32_t v[3][EPT];
@@ -304,10 +322,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
 #pragma unroll
             for (int m = 0; m < EPT; m++) v[k][m] = nttr::csub(v[k][m], q);
 #pragma unroll
-            for (int m = 0; m < 4; m++) {
-                own[k][m] = g ? v[k][4 + m] : v[k][m];
-                nttl::st_peer(&sm.pv[par][k * 4 + m][t], peer, g ? v[k][m] : v[k][4 + m]);
-            }
+            for (int m = 0; m < 4; m++) own[k][m] = g ? v[k][4 + m] : v[k][m];
+            send(n, 2 + k, g ? v[k][0] : v[k][4], g ? v[k][1] : v[k][5], g ? v[k][2] : v[k][6], g ? v[k][3] : v[k][7]);
         }
         const uint32_t ti = chain ? 2 * N - gi : gi;
         if (WROWS) {
@@ -345,20 +361,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
             for (int m = 0; m < EPT; m++) o[m] = mod64((uint64_t)y[m] * N, q, limb_br(g));
             d[0] = make_uint4(o[0], o[1], o[2], o[3]);
             d[1] = make_uint4(o[4], o[5], o[6], o[7]);
-            umma::cluster_sync();
+            receive(n, 3 * 256 * 16);
         } else {
-            to_raw2(par);
+            to_raw2(n, 5 * 256 * 16);
         }
         // bold_t[i][k] condensed: limb 0 in the low word, limb 1 in the high word
         // (condense_matrix); this CTA stores slots z8 + 4 g .. + 4
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             uint32_t w[8];
+            const uint4 e = sm.ex[n & 1][2 + k][t];
+            const uint32_t o[4] = {e.x, e.y, e.z, e.w};
 #pragma unroll
             for (int m = 0; m < 4; m++) {
-                const uint32_t o = sm.pv[par][k * 4 + m][t];
-                w[2 * m] = g ? o : own[k][m];
-                w[2 * m + 1] = g ? own[k][m] : o;
+                w[2 * m] = g ? o[m] : own[k][m];
+                w[2 * m + 1] = g ? own[k][m] : o[m];
             }
             st_sector(out + (((int64_t)i * 3 + k) * N + z8 + 4 * g) * 2, w);
         }
@@ -366,6 +383,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
     if (chain == 1 && g == 0)
 #pragma unroll
         for (int m = 0; m < EPT; m++) xbar0[I * N + eA(t, m)] = x[m];
+    umma::cluster_sync();  // every store into this CTA has landed
+    if (!ok) {  // device memory or mapped host memory
+        *static_cast<volatile int*>(err_flag) = 33;
+        __threadfence_system();
+    }
 }
 
 // per instance: bold_t_hat = NTT(digits(raw(r_bar_all[0]))), a_hat = raw(r_all[0] + V * bold_t_hat)
@@ -524,7 +546,7 @@ int cuda_fail(cudaError_t e, const char* what) {
 // tables with their companions interleaved, the inverse twiddles without the halving).
 cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar_all, int64_t cols,
                                     const uint32_t* wrows, const uint32_t* vmask, const uint32_t* tab /*fw fwp iw iwp*/,
-                                    uint32_t* F, uint32_t* r0, uint64_t* xb, uint32_t* itab, uint64_t* bt, uint64_t* btb,
+                                    uint32_t* F, uint32_t* r0, uint64_t* xb, uint32_t* itab, int* err_flag, uint64_t* bt, uint64_t* btb,
                                     uint64_t* bth, uint64_t* a_hat, cudaStream_t st) {
     const int coll_smem = (int)sizeof(CollapseSmem);
     cudaError_t e = collapse_attributes();
@@ -534,7 +556,7 @@ cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar
     uint2* it = reinterpret_cast<uint2*>(itab);
     k_interleave<<<2 * N / 256, 256, 0, st>>>(fw, fwp, iw, it, it + 2 * N);
     k_off_collapse<true><<<dim3((unsigned)(2 * cols), 2), 256, (int)sizeof(ChainSmem), st>>>(
-        F, 0, nullptr, it, it + 2 * N, collapse_scale(), bt, btb, r0, xb, wrows);
+        F, 0, nullptr, it, it + 2 * N, collapse_scale(), bt, btb, r0, xb, wrows, err_flag);
     k_off_finish<<<(unsigned)cols, 512, coll_smem, st>>>(r0, xb, 0, vmask, fw, fwp, iw, iwp, bth, a_hat);
     return cudaGetLastError();
 }
@@ -571,8 +593,10 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
     const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(instances, budget / kOfflineScratchPerInstance));
     uint32_t *d_tab = nullptr, *d_query = nullptr, *d_wv = nullptr, *d_act = nullptr, *d_E = nullptr, *d_r0 = nullptr;
     uint64_t* d_xb = nullptr;
+    int* d_err = nullptr;
     auto release = [&]() {
-        for (void* p : {(void*)d_tab, (void*)d_query, (void*)d_wv, (void*)d_act, (void*)d_E, (void*)d_r0, (void*)d_xb})
+        for (void* p : {(void*)d_tab, (void*)d_query, (void*)d_wv, (void*)d_act, (void*)d_E, (void*)d_r0, (void*)d_xb,
+                        (void*)d_err})
             if (p) cudaFree(p);
     };
     cudaError_t e;
@@ -582,7 +606,8 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
         (e = cudaMalloc(&d_act, chunk * 2ull * N * N * 4)) != cudaSuccess ||
         (e = cudaMalloc(&d_E, chunk * 2ull * N * N * 4)) != cudaSuccess ||
         (e = cudaMalloc(&d_r0, chunk * 2ull * N * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&d_xb, chunk * (uint64_t)N * 8)) != cudaSuccess) {
+        (e = cudaMalloc(&d_xb, chunk * (uint64_t)N * 8)) != cudaSuccess ||
+        (e = cudaMalloc(&d_err, sizeof(int))) != cudaSuccess) {
         release();
         return cuda_fail(e, "scratch allocation");
     }
@@ -591,7 +616,8 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
     uint32_t *d_wm = d_wv, *d_vm = d_wv + wmask.size();
     int status = IPR_OK;
     do {
-        if ((e = cudaMemcpyAsync(d_fw, hp.fw.data(), tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        if ((e = cudaMemsetAsync(d_err, 0, sizeof(int), st)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(d_fw, hp.fw.data(), tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_fwp, hp.fwp.data(), tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_iw, hp.iw.data(), tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_iwp, hp.iwp.data(), tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
@@ -619,12 +645,20 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
             k_off_gather<<<dim3(N / GZ, (unsigned)c, 2), 256, gather_smem, st>>>(d_E, c, d_act);  // F reuses act
             k_off_collapse<false><<<dim3((unsigned)(2 * c), 2), 256, (int)sizeof(ChainSmem), st>>>(
                 d_act, (int64_t)i0, d_wm, reinterpret_cast<uint2*>(d_fwi), reinterpret_cast<uint2*>(d_iwi),
-                collapse_scale(), d_bt, d_btb, d_r0, d_xb, nullptr);
+                collapse_scale(), d_bt, d_btb, d_r0, d_xb, nullptr, d_err);
             k_off_finish<<<(unsigned)c, 512, coll_smem, st>>>(d_r0, d_xb, (int64_t)i0, d_vm, d_fw, d_fwp, d_iw, d_iwp,
                                                               d_bth, d_a_hat);
             if ((e = cudaGetLastError()) != cudaSuccess) status = cuda_fail(e, "launch");
         }
-        if (status == IPR_OK && (e = cudaStreamSynchronize(st)) != cudaSuccess) status = cuda_fail(e, "run");
+        int flag = 0;
+        if (status == IPR_OK &&
+            ((e = cudaMemcpyAsync(&flag, d_err, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+             (e = cudaStreamSynchronize(st)) != cudaSuccess))
+            status = cuda_fail(e, "run");
+        if (status == IPR_OK && flag) {
+            set_last_error("offline precomputation: a device-side wait ran out");
+            status = IPR_E_TIMEOUT;
+        }
     } while (false);
     cudaStreamSynchronize(st);
     release();
@@ -658,6 +692,7 @@ struct ipr_inspiring {
     uint32_t *fw = nullptr, *fwp = nullptr, *iw = nullptr, *iwp = nullptr, *wm = nullptr, *vm = nullptr;
     uint32_t *fwi = nullptr, *iwi = nullptr;  // the twiddles interleaved with their companions
     uint32_t *act = nullptr, *E = nullptr, *r0 = nullptr, *S = nullptr;
+    int *h_err = nullptr, *d_err = nullptr;  // mapped host memory: a device-side wait ran out
     uint64_t *xb = nullptr, *a_hat = nullptr, *bt = nullptr, *btb = nullptr, *bth = nullptr, *R = nullptr;
     template <typename T>
     cudaError_t alloc(T** p, size_t bytes) {
@@ -674,6 +709,7 @@ void ipr_inspiring_destroy(ipr_inspiring* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     for (void* p : ctx->allocs) cudaFree(p);
+    if (ctx->h_err) cudaFreeHost(ctx->h_err);
     delete ctx;
 }
 
@@ -702,6 +738,8 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
         (e = c->alloc(&c->bt, ms * ipr::NINNER * ipr::N * 8)) || (e = c->alloc(&c->btb, ms * ipr::NINNER * ipr::N * 8)) ||
         (e = c->alloc(&c->bth, ms * 3 * ipr::N * 8)) || (e = c->alloc(&c->S, ms * 2 * ipr::N * 4)) ||
         (e = c->alloc(&c->R, ms * ipr::N * 8)) ||
+        (e = cudaHostAlloc(&c->h_err, sizeof(int), cudaHostAllocMapped)) ||
+        (e = cudaHostGetDevicePointer(&c->d_err, c->h_err, 0)) ||
         (e = cudaMemcpy(c->fw, hp.fw.data(), tb, cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(c->fwp, hp.fwp.data(), tb, cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(c->iw, hp.iw.data(), tb, cudaMemcpyHostToDevice)) ||
@@ -717,6 +755,7 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
         ipr_inspiring_destroy(c);
         return ipr::cuda_fail(e, "ipr_inspiring_create");
     }
+    *c->h_err = 0;
     *out = c;
     return IPR_OK;
 }
@@ -729,6 +768,10 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     }
     cudaError_t e = cudaSetDevice(c->device);
     if (e != cudaSuccess) return ipr::cuda_fail(e, "set device");
+    if (*static_cast<volatile int*>(c->h_err)) {
+        ipr::set_last_error("ipr_inspiring_pack: a device-side wait of an earlier call ran out");
+        return IPR_E_TIMEOUT;
+    }
     using namespace ipr;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int coll_smem = (int)sizeof(CollapseSmem);
@@ -737,7 +780,7 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     k_off_gather<<<dim3(N / GZ, (unsigned)sets, 2), 256, N * GZ * 4, st>>>(c->E, sets, c->act);
     k_off_collapse<false><<<dim3((unsigned)(2 * sets), 2), 256, (int)sizeof(ChainSmem), st>>>(
         c->act, 0, c->wm, reinterpret_cast<uint2*>(c->fwi), reinterpret_cast<uint2*>(c->iwi), collapse_scale(), c->bt,
-        c->btb, c->r0, c->xb, nullptr);
+        c->btb, c->r0, c->xb, nullptr, c->d_err);
     k_off_finish<<<(unsigned)sets, 512, coll_smem, st>>>(c->r0, c->xb, 0, c->vm, c->fw, c->fwp, c->iw, c->iwp, c->bth,
                                                          c->a_hat);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "offline kernels");

@@ -132,21 +132,21 @@ int ensure_scratch(ipr_server* s, unsigned nq) {
 
 // The one-chain fold's form for `chains` chains, by predicted time.  Chains run in rounds of
 // (chains per SM x SMs).  In hundredths of a round of two chains per SM staging the RGSW bodies
-// in shared memory (830 us for 31 steps):
-//   two per SM, staged       100 a round, 57 for a last round of at most one chain per SM (474 us)
-//   three per SM, bodies from L2 (more warps to hide latency, 80 registers)  122 a round
-//   four CTAs per chain      20 (167 us) while the chip is not full, then 72 per chain and SM
-// Measured at 148 SMs (us, staged form / four CTAs per chain): 32 chains 474 / 167, 64 474 / 274,
-// 96 474 / 384, 120 474 / 477, 162 830 / 615, 240 833 / 940, 384 1300 / 1442; 1,408 chains (64 payloads at
-// 1M) take 4 rounds of three per SM against 5 of two.  Forms 4 / 5 force one occupancy.
+// in shared memory (806 us for 31 steps):
+//   two per SM, staged       100 a round, 57 for a last round of at most one chain per SM (460 us)
+//   three per SM, bodies from L2 (more warps to hide latency, 80 registers)  157 a round
+//   four CTAs per chain      19 (150 us) while the chip is not full, then 66 per chain and SM
+// Measured at 148 SMs (us, staged form / four CTAs per chain): 32 chains 460 / 151, 64 460 / 259,
+// 96 460 / 351, 162 806 / 571, 240 806 / 904, 384 1254 / 1374, 768 2506 / 2614.  Forms 4 / 5 force one
+// occupancy.
 ipr::FoldForm fold_form(const ipr_server* s, int chains) {
     if (s->fold_mode == 4) return ipr::FoldForm::kThreePerSm;
     if (s->fold_mode == 5) return ipr::FoldForm::kStaged;
     const int64_t sm = s->sm_count > 0 ? s->sm_count : 1;
     const int64_t rest = chains % (2 * sm);
     const int64_t staged = chains / (2 * sm) * 100 + (rest == 0 ? 0 : (rest <= sm ? 57 : 100));
-    const int64_t three = (chains + 3 * sm - 1) / (3 * sm) * 122;
-    const int64_t cluster = chains * 72 / sm > 20 ? chains * 72 / sm : 20;
+    const int64_t three = (chains + 3 * sm - 1) / (3 * sm) * 157;
+    const int64_t cluster = chains * 66 / sm > 19 ? chains * 66 / sm : 19;
     if (cluster < staged && cluster < three) return ipr::FoldForm::kCluster;
     return three >= staged ? ipr::FoldForm::kStaged : ipr::FoldForm::kThreePerSm;
 }
@@ -198,7 +198,7 @@ int enqueue(ipr_server* s, unsigned nq, const uint8_t* d_query, uint8_t* d_resp,
                 CU(ipr::launch_fold4(s->d_row0m, s->d_gsw, s->d_ahat, s->d_S, 0, s->d_c, s->d_fwi, s->d_iwi,
                                      (int)p.interp, (int)p.c, (int)nq, (int64_t)p.db_cols, (int)nq, d_resp, 0,
                                      (int64_t)(4 + s->per_query_bytes()), ext, st,
-                                     fold_form(s, (int)(nq * p.c))));
+                                     fold_form(s, (int)(nq * p.c)), s->d_err));
             }
             else
                 CU(ipr::launch_fold3(s->d_row0s, s->d_gsw, s->d_ahat, s->d_S, 0, s->d_c, s->d_fwi, s->d_iwi,
@@ -350,7 +350,7 @@ int enqueue_batch(ipr_server* s, int B, const uint8_t* d_queries, uint8_t* d_res
             if (ipr::kBoundsChecked) ext.s_words -= ipr::g_fold_extent_cut.load();
             CU(ipr::launch_fold4(s->d_row0m, s->d_gsw, s->d_ahat, s->d_bS, (int64_t)(p.instances * 2 * kN), s->d_c,
                                  s->d_fwi, s->d_iwi, (int)p.interp, (int)p.c, nqt, (int64_t)p.db_cols, 2, d_resps, rb,
-                                 (int64_t)(4 + s->per_query_bytes()), ext, st, fold_form(s, (int)(nqt * p.c))));
+                                 (int64_t)(4 + s->per_query_bytes()), ext, st, fold_form(s, (int)(nqt * p.c)), s->d_err));
         }
         else
             CU(ipr::launch_fold3(s->d_row0s, s->d_gsw, s->d_ahat, s->d_bS, (int64_t)(p.instances * 2 * kN), s->d_c,

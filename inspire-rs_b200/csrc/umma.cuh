@@ -124,6 +124,38 @@ __device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
     return r;
 }
+// 16 bytes into the shared memory of another CTA of the cluster (`dst`, `mbar`: shared::cluster
+// addresses there), counted on its mbarrier: data and signal in one, without the memory barrier
+// that a release costs the sender
+__device__ __forceinline__ void st_async16(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t mbar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+                 "r"(a), "r"(b), "r"(c), "r"(d), "r"(mbar)
+                 : "memory");
+}
+// mbar_wait for data that another CTA of the cluster sends
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* mbar, uint32_t parity, uint64_t limit_ns = kWaitLimitNs) {
+    const uint32_t a = smem_addr(mbar);
+    auto poll = [&]() {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(a), "r"(parity)
+            : "memory");
+        return ok != 0;
+    };
+    if (poll()) return true;
+    const uint64_t t0 = global_ns();
+    for (uint32_t it = 0; it < (1u << 26); it++) {
+#pragma unroll 1
+        for (int k = 0; k < 8; k++)
+            if (poll()) return true;
+        if (global_ns() - t0 >= limit_ns) return false;
+    }
+    return false;
+}
+
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 

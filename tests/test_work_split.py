@@ -74,9 +74,9 @@ def test_raw_db_forms(pkg, orc, rows, per, entry, shift):
     assert (np.delete(got, np.s_[shift // 2:shift // 2 + want.size]) == 7).all()
 
 
-@pytest.mark.parametrize("groups,queries", [(1, 1), (28, 4), (30, 4), (25, 6), (25, 8)])
+@pytest.mark.parametrize("groups,queries", [(1, 1), (31, 4), (33, 4), (25, 6), (25, 9)])
 def test_fold_form_by_chains(pkg, orc, groups, queries):
-    """1 and 112 chains on clusters, 120 on two chains per SM, 150 on clusters, 200 on two per SM"""
+    """1 and 124 chains on clusters, 132 on two chains per SM, 150 on clusters, 225 on two per SM"""
     plan = _plan(pkg, 2 * groups, interp=2)
     with pkg.KeywordServer.synthetic(plan, seed=500 + groups) as srv:
         q = orc.synth_query(29 + queries, plan.db_rows, queries)
