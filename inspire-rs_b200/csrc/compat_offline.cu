@@ -32,8 +32,7 @@ cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar
                                     uint32_t* r0, uint64_t* xb, uint32_t* itab, int* err_flag, uint64_t* bt, uint64_t* btb,
                                     uint64_t* bth, uint64_t* a_hat, cudaStream_t st);
 cudaError_t narrow_u64(const uint64_t* in, int64_t n, uint32_t* out, cudaStream_t st);
-cudaError_t offline_jntt(const uint32_t* act, int64_t inst, const uint32_t* fw, const uint32_t* fwp, uint32_t* E,
-                         cudaStream_t st);
+cudaError_t offline_jntt(const uint32_t* act, int64_t inst, const uint2* fwi, uint32_t* E, cudaStream_t st);
 
 namespace {
 
@@ -279,7 +278,8 @@ struct PackState {
     uint64_t q0 = 0, q1 = 0;
     uint64_t *mono = nullptr, *mod_inv = nullptr, *a_ct = nullptr, *r_out = nullptr, *rb_out = nullptr;
     int *idx = nullptr, *idx_bar = nullptr;
-    uint32_t *tab32 = nullptr, *act = nullptr, *E = nullptr;
+    uint32_t *tab32 = nullptr;  // forward twiddles interleaved with their companions
+    uint32_t *act = nullptr, *E = nullptr;
 } g_pack;
 
 struct CollapseSet {  // one set of outputs (primary, or the "_new" set of the fold variants)
@@ -387,7 +387,7 @@ bool pack_sums(const uint64_t* d_a_ct) {
     PackState& P = g_pack;
     if (P.canonical) {
         k_act_from_u64<<<148 * 4, 256>>>(d_a_ct, P.act);
-        if (report(offline_jntt(P.act, 1, P.tab32, P.tab32 + 2 * N, P.E, nullptr), "packing transform")) return false;
+        if (report(offline_jntt(P.act, 1, reinterpret_cast<const uint2*>(P.tab32), P.E, nullptr), "packing transform")) return false;
         if (report(cudaFuncSetAttribute(k_pre_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * N * 4),
                    "packing gather"))
             return false;
@@ -632,13 +632,8 @@ void gpu_packing_setup(const uint64_t* h_mono_table, const int* h_idx, const int
     if (ok && P.canonical) {
         HostParams hp;
         host_params_init(hp);
-        std::vector<uint32_t> tab(8 * N);
-        std::memcpy(tab.data(), hp.fw.data(), 2 * N * 4);
-        std::memcpy(tab.data() + 2 * N, hp.fwp.data(), 2 * N * 4);
-        std::memcpy(tab.data() + 4 * N, hp.iw.data(), 2 * N * 4);
-        std::memcpy(tab.data() + 6 * N, hp.iwp.data(), 2 * N * 4);
-        ok = !report(cudaMalloc(&P.tab32, tab.size() * 4), "packing buffers") &&
-             !report(cudaMemcpy(P.tab32, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice), "packing tables") &&
+        ok = !report(cudaMalloc(&P.tab32, hp.fwi.size() * 4), "packing buffers") &&
+             !report(cudaMemcpy(P.tab32, hp.fwi.data(), hp.fwi.size() * 4, cudaMemcpyHostToDevice), "packing tables") &&
              !report(cudaMalloc(&P.act, 2ull * N * N * 4), "packing buffers") &&
              !report(cudaMalloc(&P.E, 2ull * N * N * 4), "packing buffers");
     } else if (ok) {

@@ -48,7 +48,8 @@ using nttr::eA;
 using nttr::eD;
 using nttr::EPT;
 constexpr int HALF = N / 2;   // packing outputs per instance (num_to_pack_half)
-constexpr int HCOLS = 4;      // DB columns per CTA in k_off_hint
+constexpr int HCOLS = 4;      // LWE columns per CTA in k_lwe_prep
+constexpr int HP = 2;         // DB columns per CTA in k_off_hint
 constexpr int JS = 8;         // slots per CTA in k_off_jntt
 constexpr int GZ = 8;         // z columns per CTA in k_off_gather
 constexpr uint64_t MASK19 = (1ull << GADGET_BITS) - 1;
@@ -65,66 +66,65 @@ __device__ __forceinline__ uint32_t gen_pow(uint32_t i) {
 }
 
 // act[l][c][s] = tau_{-1}-permuted NTT_l(DB column c) * query, for chunk-local columns c.
-// 512 threads: group g = threadIdx.x / 256 transforms limb g; HCOLS columns per CTA.
-__global__ void __launch_bounds__(512, 1)
+// Bound by instruction issue: one limb and HP columns per CTA of 256 threads (four CTAs per SM),
+// the lazily reduced digit transform (DB entries are below 2^16).  129,024 columns 1.36 ms,
+// against 2.76 ms for both limbs of four columns in one CTA on canonical butterflies.
+// grid (ncols / HP, 2 limbs)
+__global__ void __launch_bounds__(256, 4)
     k_off_hint(const uint16_t* __restrict__ db, int64_t db_rows, int64_t col0, int64_t ncols,
-               const uint32_t* __restrict__ query, const uint32_t* __restrict__ fw, const uint32_t* __restrict__ fwp,
-               uint32_t* __restrict__ act) {
-    extern __shared__ uint32_t hsm[];  // [2 groups][HCOLS][N]
-    const int g = threadIdx.x >> 8, t = threadIdx.x & 255;
+               const uint32_t* __restrict__ query, const uint2* __restrict__ fwi, uint32_t* __restrict__ act) {
+    __shared__ __align__(16) uint32_t xbuf[HP * N];
+    const int g = blockIdx.y, t = threadIdx.x;
     const uint32_t q = limb_q(g);
     const uint64_t br = limb_br(g);
-    uint32_t* xbuf = hsm + g * HCOLS * N;
-    const int64_t c0 = (int64_t)blockIdx.x * HCOLS;
+    const int64_t c0 = (int64_t)blockIdx.x * HP;
     const int polys = (int)(db_rows / N);
-    uint32_t acc[HCOLS][EPT];  // canonical running sum over the column's row polynomials
+    uint32_t acc[HP][EPT];  // canonical running sum over the column's row polynomials
 #pragma unroll
-    for (int p = 0; p < HCOLS; p++)
+    for (int p = 0; p < HP; p++)
 #pragma unroll
         for (int m = 0; m < EPT; m++) acc[p][m] = 0;
     for (int row = 0; row < polys; row++) {
-        uint32_t v[HCOLS][EPT];
+        uint32_t v[HP][EPT];
 #pragma unroll
-        for (int p = 0; p < HCOLS; p++) {
-            const bool live = c0 + p < ncols;
-            const uint16_t* col = db + (col0 + (live ? c0 + p : 0)) * db_rows + (int64_t)row * N;
+        for (int p = 0; p < HP; p++) {
+            const uint16_t* col = db + (col0 + c0 + p) * db_rows + (int64_t)row * N;
 #pragma unroll
-            for (int m = 0; m < EPT; m++) v[p][m] = live ? (uint32_t)__ldg(col + eA(t, m)) : 0u;
+            for (int m = 0; m < EPT; m++) v[p][m] = (uint32_t)__ldg(col + eA(t, m));
         }
-        nttr::forward<HCOLS>(v, t, xbuf, 1 + g, fw + g * N, fwp + g * N, q);  // layout D, canonical
-        const uint32_t* qr = query + ((int64_t)row * 2 + g) * N;
+        nttl::forward_digits<HP, true, true>(v, t, xbuf, 1, fwi + g * N, q);  // layout D, below 10 q
+        uint32_t qr[EPT];
+        nttl::load_d8(qr, query + ((int64_t)row * 2 + g) * N + eD(t, 0));
 #pragma unroll
-        for (int p = 0; p < HCOLS; p++)
+        for (int p = 0; p < HP; p++)
 #pragma unroll
-            for (int m = 0; m < EPT; m++) acc[p][m] = mod64((uint64_t)v[p][m] * __ldg(qr + eD(t, m)) + acc[p][m], q, br);
+            for (int m = 0; m < EPT; m++) acc[p][m] = mod64((uint64_t)v[p][m] * qr[m] + acc[p][m], q, br);
     }
     // slot w = eD(t, m) holds V[w]; the permuted polynomial has V[w] at tau_{-1}(w) (an involution)
-    nttr::group_bar(1 + g);
+    nttr::group_bar(1);
 #pragma unroll
-    for (int p = 0; p < HCOLS; p++)
+    for (int p = 0; p < HP; p++)
 #pragma unroll
         for (int m = 0; m < EPT; m++) xbuf[p * N + auto_src(2 * N - 1, eD(t, m))] = acc[p][m];
-    nttr::group_bar(1 + g);
+    nttr::group_bar(1);
 #pragma unroll
-    for (int p = 0; p < HCOLS; p++) {
-        if (c0 + p >= ncols) break;
+    for (int p = 0; p < HP; p++) {
         uint32_t* dst = act + ((int64_t)g * ncols + c0 + p) * N;
 #pragma unroll
         for (int m = 0; m < EPT; m++) dst[eA(t, m)] = xbuf[p * N + eA(t, m)];
     }
 }
 
-// E[l][I][s][z] = N^-1 * NTT over j of act[l][I][j][s], JS consecutive slots per CTA.
-// grid (N / JS, instances, 2 limbs), 256 threads
-__global__ void __launch_bounds__(256)
-    k_off_jntt(const uint32_t* __restrict__ act, int64_t inst, const uint32_t* __restrict__ fw,
-               const uint32_t* __restrict__ fwp, uint32_t* __restrict__ E) {
-    __shared__ __align__(16) uint32_t xbuf[4 * N];
+// E[l][I][s][z] = N^-1 * NTT over j of act[l][I][j][s], JS consecutive slots per CTA (the 32 bytes
+// of a row that they take are one sector).  grid (N / JS, instances, 2 limbs), 256 threads, 64 KB
+// of dynamic shared memory
+__global__ void __launch_bounds__(256, 2)
+    k_off_jntt(const uint32_t* __restrict__ act, int64_t inst, const uint2* __restrict__ fwi, uint32_t* __restrict__ E) {
+    extern __shared__ __align__(16) uint32_t jbuf[];  // [JS][N]
     const int t = threadIdx.x;
     const int s0 = blockIdx.x * JS, l = blockIdx.z;
     const int64_t base = ((int64_t)l * inst + blockIdx.y) * N * N;
     const uint32_t q = limb_q(l);
-    const uint64_t br = limb_br(l);
     uint32_t v[JS][EPT];
 #pragma unroll
     for (int m = 0; m < EPT; m++) {
@@ -133,18 +133,19 @@ __global__ void __launch_bounds__(256)
         v[0][m] = a.x; v[1][m] = a.y; v[2][m] = a.z; v[3][m] = a.w;
         v[4][m] = b.x; v[5][m] = b.y; v[6][m] = b.z; v[7][m] = b.w;
     }
-    nttr::forward<JS, 4>(v, t, xbuf, 1, fw + l * N, fwp + l * N, q);
-    const uint32_t ninv = l ? (uint32_t)(Q1 - (Q1 - 1) / N) : (uint32_t)(Q0 - (Q0 - 1) / N);  // N^-1 mod q_l
+    nttl::forward_digits<JS, false, true>(v, t, jbuf, 1, fwi + l * N, q);  // canonical in: below 15 q through stage 6
+    const uint32_t ninv = q - (q - 1) / N, ninvp = (uint32_t)(((uint64_t)ninv << 32) / q);  // N^-1 mod q_l
 #pragma unroll
     for (int p = 0; p < JS; p++) {
         uint32_t o[EPT];
 #pragma unroll
-        for (int k = 0; k < EPT; k++) o[k] = mod64((uint64_t)v[p][k] * ninv, q, br);
+        for (int k = 0; k < EPT; k++) o[k] = nttl::mul_canon(v[p][k], ninv, ninvp, q);
         uint4* dst = reinterpret_cast<uint4*>(E + base + (int64_t)(s0 + p) * N + eD(t, 0));
         dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
         dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
 }
+constexpr int JNTT_SMEM = JS * N * 4;
 
 // F[I][chain][i][l][z] = E[l][I][tau(z)][z], tau = tau_{5^i} (chain 0) or tau_{-5^i} (chain 1),
 // for a tile of GZ columns z.  grid (N / GZ, instances, 2 limbs), 256 threads, 64 KB dynamic smem
@@ -162,9 +163,11 @@ __global__ void __launch_bounds__(256)
         *reinterpret_cast<uint4*>(&tile[s * GZ + 4]) = b;
     }
     __syncthreads();
-    for (int idx = t; idx < HALF * GZ; idx += 256) {
+    uint32_t gi = gen_pow((uint32_t)t / GZ);  // 5^i of this thread's i = t / GZ + 256 / GZ * round
+    const uint32_t g_step = gen_pow(256 / GZ);
+    for (int idx = t; idx < HALF * GZ; idx += 256, gi = (gi * g_step) & (2 * N - 1)) {
         const int i = idx / GZ, zz = idx % GZ;
-        const uint32_t z = (uint32_t)(z0 + zz), gi = gen_pow((uint32_t)i);
+        const uint32_t z = (uint32_t)(z0 + zz);
         F[(((I * 2 + 0) * HALF + i) * 2 + l) * N + z] = tile[auto_src(gi, z) * GZ + zz];
         F[(((I * 2 + 1) * HALF + i) * 2 + l) * N + z] = tile[auto_src(2 * N - gi, z) * GZ + zz];
     }
@@ -562,9 +565,10 @@ cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar
 }
 
 // E[l][I][s][z] = N^-1 * NTT over j of act[l][I][j][s] for `inst` instances
-cudaError_t offline_jntt(const uint32_t* act, int64_t inst, const uint32_t* fw, const uint32_t* fwp, uint32_t* E,
-                         cudaStream_t st) {
-    k_off_jntt<<<dim3(N / JS, (unsigned)inst, 2), 256, 0, st>>>(act, inst, fw, fwp, E);
+cudaError_t offline_jntt(const uint32_t* act, int64_t inst, const uint2* fwi, uint32_t* E, cudaStream_t st) {
+    cudaError_t e = cudaFuncSetAttribute(k_off_jntt, cudaFuncAttributeMaxDynamicSharedMemorySize, JNTT_SMEM);
+    if (e != cudaSuccess) return e;
+    k_off_jntt<<<dim3(N / JS, (unsigned)inst, 2), 256, JNTT_SMEM, st>>>(act, inst, fwi, E);
     return cudaGetLastError();
 }
 
@@ -591,26 +595,26 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
     // chunk of instances per pass, bounded by the scratch budget (0 = 4 GiB)
     const uint64_t budget = scratch_budget ? scratch_budget : (4ull << 30);
     const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(instances, budget / kOfflineScratchPerInstance));
-    uint32_t *d_tab = nullptr, *d_query = nullptr, *d_wv = nullptr, *d_act = nullptr, *d_E = nullptr, *d_r0 = nullptr;
-    uint64_t* d_xb = nullptr;
-    int* d_err = nullptr;
-    auto release = [&]() {
-        for (void* p : {(void*)d_tab, (void*)d_query, (void*)d_wv, (void*)d_act, (void*)d_E, (void*)d_r0, (void*)d_xb,
-                        (void*)d_err})
-            if (p) cudaFree(p);
-    };
-    cudaError_t e;
+    // one allocation for everything (each costs about 0.8 ms with its release): the parts, each a
+    // multiple of 256 bytes
     const size_t tb = 2 * N * sizeof(uint32_t);
-    if ((e = cudaMalloc(&d_tab, 8 * tb)) != cudaSuccess || (e = cudaMalloc(&d_query, query.size() * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&d_wv, 2 * wmask.size() * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&d_act, chunk * 2ull * N * N * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&d_E, chunk * 2ull * N * N * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&d_r0, chunk * 2ull * N * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&d_xb, chunk * (uint64_t)N * 8)) != cudaSuccess ||
-        (e = cudaMalloc(&d_err, sizeof(int))) != cudaSuccess) {
-        release();
-        return cuda_fail(e, "scratch allocation");
-    }
+    uint8_t* d_scratch = nullptr;
+    size_t used = 0;
+    auto part = [&](size_t bytes) {
+        const size_t at = used;
+        used += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t o_act = part(chunk * 2ull * N * N * 4), o_E = part(chunk * 2ull * N * N * 4),
+                 o_r0 = part(chunk * 2ull * N * 4), o_xb = part(chunk * (uint64_t)N * 8), o_tab = part(8 * tb),
+                 o_query = part(query.size() * 4), o_wv = part(2 * wmask.size() * 4), o_err = part(sizeof(int));
+    cudaError_t e = cudaMalloc(&d_scratch, used);
+    if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");
+    auto u32 = [&](size_t at) { return reinterpret_cast<uint32_t*>(d_scratch + at); };
+    uint32_t *d_tab = u32(o_tab), *d_query = u32(o_query), *d_wv = u32(o_wv), *d_act = u32(o_act), *d_E = u32(o_E),
+             *d_r0 = u32(o_r0);
+    uint64_t* d_xb = reinterpret_cast<uint64_t*>(d_scratch + o_xb);
+    int* d_err = reinterpret_cast<int*>(d_scratch + o_err);
     uint32_t *d_fw = d_tab, *d_fwp = d_tab + 2 * N, *d_iw = d_tab + 4 * N, *d_iwp = d_tab + 6 * N;
     uint32_t *d_fwi = d_tab + 8 * N, *d_iwi = d_tab + 12 * N;  // interleaved with their companions
     uint32_t *d_wm = d_wv, *d_vm = d_wv + wmask.size();
@@ -629,8 +633,8 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
             status = cuda_fail(e, "table upload");
             break;
         }
-        const int hint_smem = 2 * HCOLS * N * 4, gather_smem = N * GZ * 4, coll_smem = (int)sizeof(CollapseSmem);
-        if ((e = cudaFuncSetAttribute(k_off_hint, cudaFuncAttributeMaxDynamicSharedMemorySize, hint_smem)) ||
+        const int gather_smem = N * GZ * 4, coll_smem = (int)sizeof(CollapseSmem);
+        if ((e = cudaFuncSetAttribute(k_off_jntt, cudaFuncAttributeMaxDynamicSharedMemorySize, JNTT_SMEM)) ||
             (e = cudaFuncSetAttribute(k_off_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, gather_smem)) ||
             (e = collapse_attributes())) {
             status = cuda_fail(e, "kernel attributes");
@@ -639,9 +643,10 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
         for (uint64_t i0 = 0; i0 < instances && status == IPR_OK; i0 += chunk) {
             const int64_t c = (int64_t)std::min<uint64_t>(chunk, instances - i0);
             const int64_t ncols = c * N;
-            k_off_hint<<<(unsigned)((ncols + HCOLS - 1) / HCOLS), 512, hint_smem, st>>>(
-                d_db, (int64_t)db_rows, (int64_t)i0 * N, ncols, d_query, d_fw, d_fwp, d_act);
-            k_off_jntt<<<dim3(N / JS, (unsigned)c, 2), 256, 0, st>>>(d_act, c, d_fw, d_fwp, d_E);
+            const uint2* fwi = reinterpret_cast<uint2*>(d_fwi);
+            k_off_hint<<<dim3((unsigned)(ncols / HP), 2), 256, 0, st>>>(d_db, (int64_t)db_rows, (int64_t)i0 * N, ncols,
+                                                                        d_query, fwi, d_act);
+            k_off_jntt<<<dim3(N / JS, (unsigned)c, 2), 256, JNTT_SMEM, st>>>(d_act, c, fwi, d_E);
             k_off_gather<<<dim3(N / GZ, (unsigned)c, 2), 256, gather_smem, st>>>(d_E, c, d_act);  // F reuses act
             k_off_collapse<false><<<dim3((unsigned)(2 * c), 2), 256, (int)sizeof(ChainSmem), st>>>(
                 d_act, (int64_t)i0, d_wm, reinterpret_cast<uint2*>(d_fwi), reinterpret_cast<uint2*>(d_iwi),
@@ -661,7 +666,7 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
         }
     } while (false);
     cudaStreamSynchronize(st);
-    release();
+    cudaFree(d_scratch);
     return status;
 }
 
@@ -751,6 +756,7 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
         (e = ipr::init_device_kernels()) || (e = ipr::set_constants(hp.barrett, hp.q0_inv_mod_q1)) ||
         (e = cudaFuncSetAttribute(ipr::k_lwe_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * ipr::HCOLS * ipr::N * 4)) ||
         (e = cudaFuncSetAttribute(ipr::k_off_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, ipr::N * ipr::GZ * 4)) ||
+        (e = cudaFuncSetAttribute(ipr::k_off_jntt, cudaFuncAttributeMaxDynamicSharedMemorySize, ipr::JNTT_SMEM)) ||
         (e = ipr::collapse_attributes())) {
         ipr_inspiring_destroy(c);
         return ipr::cuda_fail(e, "ipr_inspiring_create");
@@ -776,7 +782,8 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int coll_smem = (int)sizeof(CollapseSmem);
     k_lwe_prep<<<dim3(N / HCOLS, (unsigned)sets), 512, 2 * HCOLS * N * 4, st>>>(d_lwe, sets, c->fw, c->fwp, c->act);
-    k_off_jntt<<<dim3(N / JS, (unsigned)sets, 2), 256, 0, st>>>(c->act, sets, c->fw, c->fwp, c->E);
+    k_off_jntt<<<dim3(N / JS, (unsigned)sets, 2), 256, JNTT_SMEM, st>>>(c->act, sets, reinterpret_cast<uint2*>(c->fwi),
+                                                                        c->E);
     k_off_gather<<<dim3(N / GZ, (unsigned)sets, 2), 256, N * GZ * 4, st>>>(c->E, sets, c->act);
     k_off_collapse<false><<<dim3((unsigned)(2 * sets), 2), 256, (int)sizeof(ChainSmem), st>>>(
         c->act, 0, c->wm, reinterpret_cast<uint2*>(c->fwi), reinterpret_cast<uint2*>(c->iwi), collapse_scale(), c->bt,
