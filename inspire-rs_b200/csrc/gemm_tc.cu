@@ -327,6 +327,27 @@ cudaError_t make_u16_col_map(CUtensorMap* map, const uint16_t* db, int db_rows, 
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+cudaError_t make_u64_row_map(CUtensorMap* map, const uint64_t* base, uint64_t row_words, uint64_t rows,
+                             uint32_t box_words, uint32_t box_rows) {
+    if (!g_encode) {
+        cudaDriverEntryPointQueryResult q;
+        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", (void**)&g_encode, cudaEnableDefault, &q);
+        if (e != cudaSuccess) return e;
+        if (!g_encode || q != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
+    }
+    if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_words & 1) || (box_words & 1) || box_words > 256 || !box_rows ||
+        box_rows > 256)
+        return cudaErrorInvalidValue;
+    cuuint64_t dims[2] = {row_words, rows};
+    cuuint64_t strides[1] = {row_words * 8};
+    cuuint32_t box[2] = {box_words, box_rows};
+    cuuint32_t elem[2] = {1, 1};
+    CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<uint64_t*>(base), dims, strides, box, elem,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 int gemm1_stages(int nt) {
     const int per = 2 * A_STAGE_BYTES + nt * TILE_K;
     int s = (210 * 1024) / per;

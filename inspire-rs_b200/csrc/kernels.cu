@@ -13,6 +13,7 @@
 //   k_response_frame serialize_keyword_response framing (wire.rs:708-726)
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "bounds.cuh"
@@ -607,135 +608,176 @@ __global__ void __launch_bounds__(GT_WARPS * 32, 1)
 //              + y_l[k][rotbar_i(z)] Tbar_l[j][i,k][z] + sum_k z_l[k][z] That_l[j][k][z]
 // with rot_i = auto_src(5^i mod 2N, .), rotbar_i = auto_src(2N - 5^i, .).
 // The client key y_body stays in shared memory; the precomputed bold_t stream
-// (the dominant HBM traffic) is read once per payload with 16-byte
-// non-allocating loads, two adjacent slots per thread.  Slots z and z+1 (z even)
-// rotate to the slot pair {s, s^1}, so each gather is one 16-byte smem load.
+// (the dominant HBM traffic) is read once per payload, two adjacent slots per thread.
+// Slots z and z+1 (z even) rotate to the slot pair {s, s^1}, so each gather is one
+// 16-byte smem load.
 //
-// Bound by the HBM stream.  A thread keeps the loads of two rotations in flight
-// while it multiplies a third, and the rotations of one (256 slots, output) task are
-// split between the CTAs of a cluster, which add their residues through
-// distributed shared memory: a task is 1023 dependent memory latencies long, so
-// without the split a small database leaves the chip idle (8 outputs are 64 tasks).
-// Whole call at 1 / 8 / 96 / 192 outputs: 71 / 161 / 1667 / 3266 us (0.10 / 0.81 / 9.7 / 19.3 GB;
-// 5.9 TB/s at 192) against 898 / 941 / 2113 / 3332 us unsplit with two rotations loaded and
-// then multiplied.  Three rotations in flight (114 registers instead of 80) measured the same.
+// Bound by the HBM stream.  TMA boxes of PT_ROT rotations (their T rows, then their Tbar rows, of
+// one block of 256 slots) pass through a ring in shared memory; two groups of four warps take
+// every other rotation of a box.  The rotations of all (output, slot block) tasks form one
+// sequence that the CTAs, one per SM, share out evenly in units of PACK_UNIT rotations, so the
+// chip is full and the last wave short at every database size; a CTA that ends or begins inside a
+// task adds its residues to S with atomic additions (at most PACK_PARTS of them per task,
+// below 2^32; S is zero before).  S is left as a sum of residues, not reduced.
+// Packing stage at 1 / 8 / 32 / 96 / 192 outputs (0.10 / 0.81 / 3.2 / 9.7 / 19.3 GB): 28 / 136 / 490 / 1381 /
+// 2768 us (7.0 TB/s at 192).  Loads into registers, two rotations ahead, with the rotations of a
+// task split over a cluster: 71 / 161 / 592 / 1667 / 3266 us (5.9 TB/s); one CTA per task:
+// 898 / 941 / 1000 / 2113 / 3332 us.
 // ---------------------------------------------------------------------------
-constexpr int PACK_THREADS = 128;
-constexpr int PACK_ZB = 2 * PACK_THREADS;  // slots per CTA
-constexpr int PACK_CHUNK = 32;             // rotations between reductions
-constexpr int PACK_MAX_SPLITS = 8;         // CTAs of a cluster (the portable limit)
+constexpr int PACK_ZB = 256;            // slots per task
+constexpr int PACK_UNIT = 16;           // rotations a CTA's share is a multiple of
+constexpr int PACK_UNITS = (NROT + PACK_UNIT - 1) / PACK_UNIT;
+constexpr int PACK_PARTS = 15;          // 15 q < 2^32
+constexpr int PT_ROT = 2, PT_STAGES = 6;
+constexpr int PT_GROUPS = 2, PT_THREADS = (PT_GROUPS * 4 + 1) * 32;
+constexpr int PT_BOX = PT_ROT * T_EXP * PACK_ZB * 8;  // bytes of one box
+constexpr int PT_SMEM = 128 + T_EXP * N * 8 + PT_STAGES * 2 * PT_BOX + 4 * 128 * 4 + 2 * PT_STAGES * 8;
+static_assert(PACK_UNIT % PT_ROT == 0, "a CTA's share is whole boxes");
 
-__device__ __forceinline__ void ldg_nc_v2(const uint64_t* p, uint64_t& a, uint64_t& b) {
-    asm volatile("ld.global.nc.L1::no_allocate.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p));
-}
-
-// the six word pairs of one rotation's precomputation
-struct PackRow {
-    uint64_t t[T_EXP][2], tb[T_EXP][2];
-};
-
-__device__ __forceinline__ void pack_load(PackRow& r, const uint64_t* __restrict__ T, const uint64_t* __restrict__ Tb,
-                                          int i) {
-#pragma unroll
-    for (int k = 0; k < T_EXP; k++) {
-        ldg_nc_v2(T + (int64_t)(i * T_EXP + k) * N, r.t[k][0], r.t[k][1]);
-        ldg_nc_v2(Tb + (int64_t)(i * T_EXP + k) * N, r.tb[k][0], r.tb[k][1]);
+__global__ void __launch_bounds__(PT_THREADS, 1)
+    k_pack(const __grid_constant__ CUtensorMap tm_t, const __grid_constant__ CUtensorMap tm_tb,
+           const uint64_t* __restrict__ bth, const uint64_t* __restrict__ y_body, const uint64_t* __restrict__ z_body,
+           int num_outputs, uint32_t* __restrict__ S, int* __restrict__ err_flag) {
+    extern __shared__ uint8_t pt_raw[];
+    uint8_t* base = pt_raw + ((128 - (umma::smem_addr(pt_raw) & 127)) & 127);
+    uint64_t* ys = reinterpret_cast<uint64_t*>(base);                         // [3][N] condensed
+    uint8_t* ring = base + T_EXP * N * 8;                                     // [stage][T, Tbar][row][256 u64]
+    uint32_t* part = reinterpret_cast<uint32_t*>(ring + PT_STAGES * 2 * PT_BOX);  // [4][128] residues of group 1
+    uint64_t* full = reinterpret_cast<uint64_t*>(part + 4 * 128);
+    uint64_t* empty = full + PT_STAGES;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < PT_STAGES; s++) {
+            umma::mbar_init(&full[s], 1);
+            umma::mbar_init(&empty[s], PT_GROUPS * 4);
+        }
+        umma::fence_mbar_init();
     }
-}
-
-// grid (N / PACK_ZB, outputs, splits), clusters of (1, 1, splits)
-__global__ void __launch_bounds__(PACK_THREADS) k_pack(const uint64_t* __restrict__ bt,
-                                                       const uint64_t* __restrict__ btb,
-                                                       const uint64_t* __restrict__ bth,
-                                                       const uint64_t* __restrict__ y_body,
-                                                       const uint64_t* __restrict__ z_body,
-                                                       uint32_t* __restrict__ S) {
-    extern __shared__ uint64_t ys[];  // [3][N] condensed
-    __shared__ uint32_t part[4][PACK_THREADS];  // this CTA's residues: [limb * 2 + slot][thread]
-    const int splits = gridDim.z, rank = blockIdx.z;
-    const int j = blockIdx.y;
-    const int z = blockIdx.x * PACK_ZB + 2 * threadIdx.x;
-    const uint32_t ez = exponent_of_slot(z);
-    const uint64_t* T = bt + (int64_t)j * NINNER * N + z;
-    const uint64_t* Tb = btb + (int64_t)j * NINNER * N + z;
-    // chunks of PACK_CHUNK rotations, shared out evenly (splits <= number of chunks)
-    constexpr int CHUNKS = (NROT + PACK_CHUNK - 1) / PACK_CHUNK;
-    const int ibeg = CHUNKS * rank / splits * PACK_CHUNK;
-    int iend_all = CHUNKS * (rank + 1) / splits * PACK_CHUNK;
-    if (iend_all > NROT) iend_all = NROT;
-    PackRow ra, rb;
-    pack_load(ra, T, Tb, ibeg);
-    pack_load(rb, T, Tb, ibeg + 1 < iend_all ? ibeg + 1 : ibeg);
+    // this CTA's units of the sequence [output][slot block][unit of rotations]
+    const int64_t total = (int64_t)num_outputs * (N / PACK_ZB) * PACK_UNITS;
+    const int64_t u_beg = total * blockIdx.x / gridDim.x, u_end = total * (blockIdx.x + 1) / gridDim.x;
     for (int i = threadIdx.x; i < T_EXP * N; i += blockDim.x) ys[i] = y_body[i];
     __syncthreads();
-    uint64_t a00 = 0, a01 = 0, a10 = 0, a11 = 0;  // a{limb}{slot}
-    uint32_t g = 1;                               // 5^i mod 2N
-    for (int e = ibeg, b = 5; e; e >>= 1, b = (b * b) & (2 * N - 1))
-        if (e & 1) g = (g * b) & (2 * N - 1);
-    auto mac = [&](const PackRow& r) {
-        const uint32_t s1 = slot_of_exponent((g * ez) & (2 * N - 1));
-        const uint32_t s2 = slot_of_exponent(((2 * N - g) * ez) & (2 * N - 1));
+    bool ok = true;
+    if (warp == PT_GROUPS * 4) {
+        if (lane == 0) {  // TMA producer: every box of the CTA's units in order
+            int stage = 0;
+            uint32_t phase = 0;
+            int issued = 0;
+            for (int64_t u = u_beg; u < u_end && ok; u++) {
+                const int64_t task = u / PACK_UNITS;
+                const int i0 = (int)(u % PACK_UNITS) * PACK_UNIT, i1 = min(i0 + PACK_UNIT, NROT);
+                const int row0 = (int)(task / (N / PACK_ZB)) * NINNER, z0 = (int)(task % (N / PACK_ZB)) * PACK_ZB;
+                for (int i = i0; i < i1; i += PT_ROT) {  // the box of the last rotation reads past it, unused
+                    if (!umma::mbar_wait(&empty[stage], phase ^ 1)) {
+                        ok = false;
+                        break;
+                    }
+                    umma::mbar_expect_tx(&full[stage], 2 * PT_BOX);
+                    uint8_t* dst = ring + stage * 2 * PT_BOX;
+                    umma::tma_load_2d(dst, &tm_t, z0, row0 + i * T_EXP, &full[stage]);
+                    umma::tma_load_2d(dst + PT_BOX, &tm_tb, z0, row0 + i * T_EXP, &full[stage]);
+                    issued++;
+                    if (++stage == PT_STAGES) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                }
+            }
+            if (!ok) atomicExch(err_flag, 34);
+            // every box issued has landed before the CTA may exit
+            for (int b = issued > PT_STAGES ? issued - PT_STAGES : 0; b < issued; b++)
+                umma::mbar_wait(&full[b % PT_STAGES], (uint32_t)((b / PT_STAGES) & 1), umma::kDrainLimitNs);
+        }
+    } else {
+        const int grp = warp >> 2, t = threadIdx.x & 127;
+        int stage = 0;
+        uint32_t phase = 0;
+        int64_t u = u_beg;
+        while (u < u_end) {  // one task, or the part of it that is this CTA's
+            const int64_t task = u / PACK_UNITS;
+            const int64_t t_end = min(u_end, (task + 1) * PACK_UNITS);
+            const int j = (int)(task / (N / PACK_ZB));
+            const int z = (int)(task % (N / PACK_ZB)) * PACK_ZB + 2 * t;
+            const uint32_t ez = exponent_of_slot(z);
+            const int ibeg = (int)(u % PACK_UNITS) * PACK_UNIT;
+            const int iend = min(ibeg + (int)(t_end - u) * PACK_UNIT, NROT);
+            uint64_t a00 = 0, a01 = 0, a10 = 0, a11 = 0;  // a{limb}{slot}
+            uint32_t g = 1;                               // 5^(i + grp) mod 2N
+            for (int e = ibeg + grp, b = 5; e; e >>= 1, b = (b * b) & (2 * N - 1))
+                if (e & 1) g = (g * b) & (2 * N - 1);
+            int since = 0;
+            for (int i = ibeg; i < iend; i += PT_ROT) {
+                if (ok) {
+                    const bool got = umma::mbar_wait(&full[stage], phase);
+                    if (!__all_sync(0xffffffffu, got)) {  // the warp gives up together and runs on without data
+                        ok = false;
+                        if (lane == 0) atomicExch(err_flag, 34);
+                    }
+                }
+                if (ok && i + grp < iend) {
+                    const uint8_t* row = ring + stage * 2 * PT_BOX + grp * T_EXP * PACK_ZB * 8 + t * 16;
+                    const uint32_t s1 = slot_of_exponent((g * ez) & (2 * N - 1));
+                    const uint32_t s2 = slot_of_exponent(((2 * N - g) * ez) & (2 * N - 1));
 #pragma unroll
-        for (int k = 0; k < T_EXP; k++) {
-            const ulonglong2 yp = *reinterpret_cast<const ulonglong2*>(ys + k * N + (s1 & ~1u));
-            const ulonglong2 bp = *reinterpret_cast<const ulonglong2*>(ys + k * N + (s2 & ~1u));
-            const uint64_t y0 = (s1 & 1) ? yp.y : yp.x, y1 = (s1 & 1) ? yp.x : yp.y;
-            const uint64_t b0 = (s2 & 1) ? bp.y : bp.x, b1 = (s2 & 1) ? bp.x : bp.y;
-            a00 += (uint64_t)(uint32_t)y0 * (uint32_t)r.t[k][0] + (uint64_t)(uint32_t)b0 * (uint32_t)r.tb[k][0];
-            a01 += (uint64_t)(uint32_t)y1 * (uint32_t)r.t[k][1] + (uint64_t)(uint32_t)b1 * (uint32_t)r.tb[k][1];
-            a10 += (y0 >> 32) * (r.t[k][0] >> 32) + (b0 >> 32) * (r.tb[k][0] >> 32);
-            a11 += (y1 >> 32) * (r.t[k][1] >> 32) + (b1 >> 32) * (r.tb[k][1] >> 32);
-        }
-        g = (g * 5) & (2 * N - 1);
-    };
-    for (int i0 = ibeg; i0 < iend_all; i0 += PACK_CHUNK) {
-        const int iend = i0 + PACK_CHUNK < iend_all ? i0 + PACK_CHUNK : iend_all;
-        int i = i0;
-#pragma unroll 1
-        for (; i + 1 < iend; i += 2) {  // ra holds row i, rb row i + 1
-            mac(ra);
-            pack_load(ra, T, Tb, i + 2 < iend_all ? i + 2 : i);
-            mac(rb);
-            pack_load(rb, T, Tb, i + 3 < iend_all ? i + 3 : i);
-        }
-        if (i < iend) mac(ra);  // only the last chunk is odd
-        // <= 192 products of two 28-bit values plus a residue: no overflow
-        a00 = modq(a00, 0); a01 = modq(a01, 0);
-        a10 = modq(a10, 1); a11 = modq(a11, 1);
-    }
-    if (rank == 0) {
-        const uint64_t* Th = bth + (int64_t)j * T_EXP * N + z;
+                    for (int k = 0; k < T_EXP; k++) {
+                        const ulonglong2 tv = *reinterpret_cast<const ulonglong2*>(row + k * PACK_ZB * 8);
+                        const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(row + PT_BOX + k * PACK_ZB * 8);
+                        const ulonglong2 yp = *reinterpret_cast<const ulonglong2*>(ys + k * N + (s1 & ~1u));
+                        const ulonglong2 bp = *reinterpret_cast<const ulonglong2*>(ys + k * N + (s2 & ~1u));
+                        const uint64_t y0 = (s1 & 1) ? yp.y : yp.x, y1 = (s1 & 1) ? yp.x : yp.y;
+                        const uint64_t b0 = (s2 & 1) ? bp.y : bp.x, b1 = (s2 & 1) ? bp.x : bp.y;
+                        a00 += (uint64_t)(uint32_t)y0 * (uint32_t)tv.x + (uint64_t)(uint32_t)b0 * (uint32_t)bv.x;
+                        a01 += (uint64_t)(uint32_t)y1 * (uint32_t)tv.y + (uint64_t)(uint32_t)b1 * (uint32_t)bv.y;
+                        a10 += (y0 >> 32) * (tv.x >> 32) + (b0 >> 32) * (bv.x >> 32);
+                        a11 += (y1 >> 32) * (tv.y >> 32) + (b1 >> 32) * (bv.y >> 32);
+                    }
+                }
+                g = (g * 25) & (2 * N - 1);
+                __syncwarp();
+                if (lane == 0) umma::mbar_arrive(&empty[stage]);
+                if (++stage == PT_STAGES) {
+                    stage = 0;
+                    phase ^= 1;
+                }
+                if (++since == 32) {  // 192 products of two 28-bit values plus a residue: no overflow
+                    a00 = modq(a00, 0); a01 = modq(a01, 0);
+                    a10 = modq(a10, 1); a11 = modq(a11, 1);
+                    since = 0;
+                }
+            }
+            if (grp == 0 && ibeg == 0) {  // the task's first part adds the z_body x That term
+                a00 = modq(a00, 0); a01 = modq(a01, 0);
+                a10 = modq(a10, 1); a11 = modq(a11, 1);
+                const uint64_t* Th = bth + (int64_t)j * T_EXP * N + z;
 #pragma unroll
-        for (int k = 0; k < T_EXP; k++) {
-            const uint64_t t0 = Th[k * N], t1 = Th[k * N + 1];
-            const uint64_t z0 = z_body[k * N + z], z1 = z_body[k * N + z + 1];
-            a00 += (uint64_t)(uint32_t)z0 * (uint32_t)t0;
-            a01 += (uint64_t)(uint32_t)z1 * (uint32_t)t1;
-            a10 += (z0 >> 32) * (t0 >> 32);
-            a11 += (z1 >> 32) * (t1 >> 32);
+                for (int k = 0; k < T_EXP; k++) {
+                    const uint64_t t0 = Th[k * N], t1 = Th[k * N + 1];
+                    const uint64_t z0 = z_body[k * N + z], z1 = z_body[k * N + z + 1];
+                    a00 += (uint64_t)(uint32_t)z0 * (uint32_t)t0;
+                    a01 += (uint64_t)(uint32_t)z1 * (uint32_t)t1;
+                    a10 += (z0 >> 32) * (t0 >> 32);
+                    a11 += (z1 >> 32) * (t1 >> 32);
+                }
+            }
+            uint32_t r[4] = {modq(a00, 0), modq(a01, 0), modq(a10, 1), modq(a11, 1)};  // limb * 2 + slot
+            if (grp == 1) {
+#pragma unroll
+                for (int v = 0; v < 4; v++) part[v * 128 + t] = r[v];
+            }
+            umma::named_bar(1, PT_GROUPS * 128);
+            if (grp == 0) {
+                uint32_t* Sj = S + (int64_t)j * 2 * N + z;
+#pragma unroll
+                for (int v = 0; v < 4; v++) {
+                    const uint32_t q = v >> 1 ? Q1 : Q0, sum = r[v] + part[v * 128 + t];
+                    atomicAdd(Sj + (v >> 1) * N + (v & 1), min(sum, sum - q));
+                }
+            }
+            umma::named_bar(1, PT_GROUPS * 128);  // part may be written again
+            u = t_end;
         }
-        a00 = modq(a00, 0); a01 = modq(a01, 0);
-        a10 = modq(a10, 1); a11 = modq(a11, 1);
     }
-    uint32_t* Sj = S + (int64_t)j * 2 * N;
-    part[0][threadIdx.x] = (uint32_t)a00;
-    part[1][threadIdx.x] = (uint32_t)a01;
-    part[2][threadIdx.x] = (uint32_t)a10;
-    part[3][threadIdx.x] = (uint32_t)a11;
-    umma::cluster_sync();
-    for (int v = rank; v < 4; v += splits) {  // CTA `rank` adds up residue kinds rank, rank + splits, ...
-        uint64_t sum = 0;
-        for (int r = 0; r < splits; r++) {
-            uint32_t x;
-            asm volatile("ld.shared::cluster.u32 %0, [%1];"
-                         : "=r"(x)
-                         : "r"(umma::map_to_rank(&part[v][threadIdx.x], (uint32_t)r))
-                         : "memory");
-            sum += x;
-        }
-        Sj[(v >> 1) * N + z + (v & 1)] = modq(sum, v >> 1);
-    }
-    umma::cluster_sync();  // no CTA leaves while its residues are being read
 }
 
 // ---------------------------------------------------------------------------
@@ -788,7 +830,7 @@ __global__ void __launch_bounds__(512) k_intt_crt(const uint32_t* __restrict__ S
             for (int m = 0; m < 8; m++) v[p][m] = mod64(acc[m], q, g ? BR1 : BR0);
         } else {
 #pragma unroll
-            for (int m = 0; m < 8; m++) v[p][m] = sv[m];
+            for (int m = 0; m < 8; m++) v[p][m] = mod64(sv[m], q, g ? BR1 : BR0);  // k_pack leaves sums of residues
         }
     }
     nttr::inverse<INTT_P>(v, t, &sm[g][0][0], 1 + g, iw + g * N, iwp + g * N, q);
@@ -1053,7 +1095,7 @@ __global__ void k_synth_modq(uint64_t* out, int64_t n, uint64_t seed, uint64_t s
 // per-device kernel attributes (dynamic shared memory above 48 KB); call once
 // with the target device current
 cudaError_t init_device_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(k_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, T_EXP * N * 8);
+    cudaError_t e = cudaFuncSetAttribute(k_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_gemv_staged_f64<GSF_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              gsf_smem(GF_MAX_ROWS));
@@ -1138,34 +1180,20 @@ cudaError_t launch_gemv(const uint16_t* db, int db_rows, int64_t db_cols, int nq
     return cudaGetLastError();
 }
 
-// CTAs per (256 slots, output) task: doubled until the grid is about 6 CTAs per SM (4 fit),
-// where the stream is bandwidth-bound and the last wave short.  Measured packing times with
-// 1 / 2 / 4 / 8 CTAs per task: 8 outputs 485 / 261 / 169 / 161 us, 32 outputs 631 / 608 / 608 /
-// 592 us, 64 outputs 1194 / 1091 / 1137 / 1150 us, 96 outputs 1788 / 1667 / 1678 / 1697 us,
-// 192 outputs 3300 / 3266 / 3322 / 3354 us.
-int pack_splits(int num_outputs, int sm_count) {
-    const int tasks = N / PACK_ZB * num_outputs;
-    int s = 2;
-    while (s < PACK_MAX_SPLITS && tasks * s < 6 * sm_count) s *= 2;
-    return s;
+cudaError_t launch_pack(const CUtensorMap* tm_t, const CUtensorMap* tm_tb, const uint64_t* bth, const uint64_t* y,
+                        const uint64_t* z, uint32_t* S, int num_outputs, int sm_count, int* err_flag, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(S, 0, (size_t)num_outputs * 2 * N * 4, st);
+    if (e != cudaSuccess) return e;
+    // at most PACK_PARTS shares touch a task: a share is at least 1 / (PACK_PARTS - 1) of one
+    const int64_t tasks = (int64_t)num_outputs * (N / PACK_ZB);
+    const int grid = (int)std::min<int64_t>(sm_count, tasks * (PACK_PARTS - 2));
+    k_pack<<<grid, PT_THREADS, PT_SMEM, st>>>(*tm_t, *tm_tb, bth, y, z, num_outputs, S, err_flag);
+    return cudaGetLastError();
 }
 
-cudaError_t launch_pack(const uint64_t* bt, const uint64_t* btb, const uint64_t* bth, const uint64_t* y,
-                        const uint64_t* z, uint32_t* S, int num_outputs, int sm_count, cudaStream_t st) {
-    const int splits = pack_splits(num_outputs, sm_count);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(N / PACK_ZB, num_outputs, splits);
-    cfg.blockDim = dim3(PACK_THREADS);
-    cfg.dynamicSmemBytes = T_EXP * N * 8;
-    cfg.stream = st;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 1;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = splits;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_pack, bt, btb, bth, y, z, S);
+// box of PT_ROT rotations' rows of one of the precomputation arrays ([outputs][3069][N] u64), 256 slots wide
+cudaError_t make_pack_map(CUtensorMap* map, const uint64_t* rows, int num_outputs) {
+    return make_u64_row_map(map, rows, N, (uint64_t)num_outputs * NINNER, PACK_ZB, PT_ROT * T_EXP);
 }
 
 cudaError_t launch_intt_crt(const uint32_t* S, const uint32_t* iw, const uint32_t* iwp, uint64_t* R,

@@ -24,10 +24,15 @@ cudaError_t launch_gemv(const uint16_t* db, int db_rows, int64_t db_cols, int nq
                         uint64_t* c, int sm_count, cudaStream_t st, int form = 0, int* err_flag = nullptr);
 // 2D tensor map over the column-major u16 DB ([db_cols][db_rows]), boxes of box_rows x box_cols
 // with the 32-byte swizzle (box_rows = 16)
+// 2D map over [rows][row_words] u64, boxes of box_words x box_rows, not swizzled
+cudaError_t make_u64_row_map(CUtensorMap* map, const uint64_t* base, uint64_t row_words, uint64_t rows,
+                             uint32_t box_words, uint32_t box_rows);
 cudaError_t make_u16_col_map(CUtensorMap* map, const uint16_t* db, int db_rows, int64_t db_cols, uint32_t box_rows,
                              uint32_t box_cols);
-cudaError_t launch_pack(const uint64_t* bt, const uint64_t* btb, const uint64_t* bth, const uint64_t* y,
-                        const uint64_t* z, uint32_t* S, int num_outputs, int sm_count, cudaStream_t st);
+// S: sums of at most 15 residues per entry (not reduced), from the arrays behind the two maps
+cudaError_t launch_pack(const CUtensorMap* tm_t, const CUtensorMap* tm_tb, const uint64_t* bth, const uint64_t* y,
+                        const uint64_t* z, uint32_t* S, int num_outputs, int sm_count, int* err_flag, cudaStream_t st);
+cudaError_t make_pack_map(CUtensorMap* map, const uint64_t* rows, int num_outputs);
 // R = from_ntt(S) per (client, output) polynomial pair; with z_bodies non-null the
 // z_body x That term of client f / instances is added to S first
 cudaError_t launch_intt_crt(const uint32_t* S, const uint32_t* iw, const uint32_t* iwp, uint64_t* R,

@@ -693,6 +693,7 @@ struct ipr_inspiring {
     int device = 0;
     int max_sets = 0;
     int sm_count = 148;
+    CUtensorMap tm_bt, tm_btb;
     std::vector<void*> allocs;
     uint32_t *fw = nullptr, *fwp = nullptr, *iw = nullptr, *iwp = nullptr, *wm = nullptr, *vm = nullptr;
     uint32_t *fwi = nullptr, *iwi = nullptr;  // the twiddles interleaved with their companions
@@ -753,6 +754,7 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
         (e = cudaMemcpy(c->iwi, hp.iwi.data(), 2 * tb, cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(c->wm, wmask.data(), wmask.size() * 4, cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(c->vm, vmask.data(), vmask.size() * 4, cudaMemcpyHostToDevice)) ||
+        (e = ipr::make_pack_map(&c->tm_bt, c->bt, max_sets)) || (e = ipr::make_pack_map(&c->tm_btb, c->btb, max_sets)) ||
         (e = ipr::init_device_kernels()) || (e = ipr::set_constants(hp.barrett, hp.q0_inv_mod_q1)) ||
         (e = cudaFuncSetAttribute(ipr::k_lwe_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * ipr::HCOLS * ipr::N * 4)) ||
         (e = cudaFuncSetAttribute(ipr::k_off_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, ipr::N * ipr::GZ * 4)) ||
@@ -791,7 +793,7 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     k_off_finish<<<(unsigned)sets, 512, coll_smem, st>>>(c->r0, c->xb, 0, c->vm, c->fw, c->fwp, c->iw, c->iwp, c->bth,
                                                          c->a_hat);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "offline kernels");
-    if ((e = launch_pack(c->bt, c->btb, c->bth, d_y_body, d_z_body, c->S, sets, c->sm_count, st)) != cudaSuccess ||
+    if ((e = launch_pack(&c->tm_bt, &c->tm_btb, c->bth, d_y_body, d_z_body, c->S, sets, c->sm_count, c->d_err, st)) != cudaSuccess ||
         (e = launch_intt_crt(c->S, c->iw, c->iwp, c->R, sets, st)) != cudaSuccess)
         return cuda_fail(e, "online kernels");
     k_inspiring_out<<<148, 256, 0, st>>>(c->a_hat, c->R, d_lwe, sets, d_out);

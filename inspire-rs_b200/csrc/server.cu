@@ -182,8 +182,8 @@ int enqueue(ipr_server* s, unsigned nq, const uint8_t* d_query, uint8_t* d_resp,
             }
         }
         rec(2);
-        CU(ipr::launch_pack(s->d_bt, s->d_btb, s->d_bth, s->d_y, s->d_z, s->d_S, (int)p.instances, s->sm_count,
-                            st));
+        CU(ipr::launch_pack(&s->tm_bt, &s->tm_btb, s->d_bth, s->d_y, s->d_z, s->d_S, (int)p.instances, s->sm_count,
+                            s->d_err, st));
         rec(3);
         if (s->fold_mode >= 2) {
             const bool chain = s->fold_mode >= 3;
@@ -465,6 +465,8 @@ int init_common(ipr_server* s, int device, const ipr_plan* plan) {
     CU(cudaMallocHost(&s->h_err, sizeof(int)));
     *s->h_err = 0;
     CU(ipr::make_u8_tile_map(&s->tm_db, s->d_db8, plan->db_rows, 2 * plan->db_cols, 128));
+    CU(ipr::make_pack_map(&s->tm_bt, s->d_bt, (int)plan->instances));
+    CU(ipr::make_pack_map(&s->tm_btb, s->d_btb, (int)plan->instances));
     s->events.resize((size_t)kMaxProfileSlots * (IPR_NSTAGES + 1), nullptr);
     return ensure_scratch(s, 2);
 }

@@ -72,6 +72,7 @@ struct ipr_server {
     std::mutex mu;
     // batched path: precomputation re-indexed by slot (Tpp), batch scratch
     uint8_t* d_tpp = nullptr;
+    CUtensorMap tm_bt, tm_btb;  // the single-payload packing's view of d_bt, d_btb
     CUtensorMap tm_tpp;
     int bcap = 0, y8_np = 0;
     uint8_t* d_bq = nullptr;

@@ -20,9 +20,9 @@ def _group(resp, c, query, g):
     return resp[off:off + RESULT]
 
 
-@pytest.mark.parametrize("instances", [1, 13, 14, 27, 28, 55, 56])
+@pytest.mark.parametrize("instances", [1, 2, 3, 13, 28, 56])
 def test_single_payload_packing_split(pkg, orc, instances):
-    """8, 4 or 2 CTAs per packing task (the count doubles until the grid is 6 CTAs per SM)"""
+    """thirteen CTAs per packing task (one output), shares that begin and end inside tasks"""
     plan = _plan(pkg, instances)
     with pkg.KeywordServer.synthetic(plan, seed=300 + instances) as srv:
         q = orc.synth_query(17 + instances, plan.db_rows, 2)
