@@ -365,6 +365,22 @@ def deserialize_keyword_response(data: bytes) -> KeywordResponsePayload:
     return KeywordResponsePayload(responses, stash)
 
 
+def _input(data):
+    """(keeper, pointer) to the bytes of a payload: a bytes object is read in place (the library copies
+    it before the call returns), anything else with the buffer protocol through a copy"""
+    if type(data) is bytes:
+        return data, ctypes.cast(ctypes.c_char_p(data), _u8p)
+    buf = (ctypes.c_uint8 * len(data)).from_buffer_copy(data)
+    return buf, ctypes.cast(buf, _u8p)
+
+
+def _output(cap: int):
+    """(keeper, pointer) to cap bytes that the library will write: not zeroed"""
+    import numpy as np
+    buf = np.empty(max(cap, 1), dtype=np.uint8)
+    return buf, ctypes.cast(buf.ctypes.data, _u8p)
+
+
 # ---------------------------------------------------------------------------
 # server
 # ---------------------------------------------------------------------------
@@ -511,13 +527,13 @@ class KeywordServer:
 
     def respond_to_serialized_query(self, query: bytes) -> bytes:
         """keyword.rs:636-640: serialized query payload -> serialized response."""
-        q = (ctypes.c_uint8 * len(query)).from_buffer_copy(query)
+        keep, q = _input(query)
         nq = query[0] if query else 0
         cap = int(_srv_rbytes(self._h, nq))
-        out = (ctypes.c_uint8 * cap)()
+        out, outp = _output(cap)
         n = _sz()
-        _check(_respond(self._h, q, len(query), out, cap, ctypes.byref(n)), "respond")
-        return bytes(out)[:n.value]
+        _check(_respond(self._h, q, len(query), outp, cap, ctypes.byref(n)), "respond")
+        return out[:n.value].tobytes()
 
     def respond(self, payload: KeywordQueryPayload) -> KeywordResponsePayload:
         """KeywordServer::respond (keyword.rs:534-628)."""
@@ -530,11 +546,15 @@ class KeywordServer:
         n = len(queries)
         if n == 0:
             return []
-        qbufs = [(ctypes.c_uint8 * len(q)).from_buffer_copy(q) for q in queries]
+        ins = [_input(q) for q in queries]
         caps = [int(_srv_rbytes(self._h, q[0] if q else 0)) for q in queries]
-        obufs = [(ctypes.c_uint8 * c)() for c in caps]
-        qp = (_u8p * n)(*[ctypes.cast(b, _u8p) for b in qbufs])
-        op = (_u8p * n)(*[ctypes.cast(b, _u8p) for b in obufs])
+        offs = [0]
+        for c in caps:
+            offs.append(offs[-1] + c)
+        out, _ = _output(offs[-1])
+        base = out.ctypes.data
+        qp = (_u8p * n)(*[p for _, p in ins])
+        op = (_u8p * n)(*[ctypes.cast(base + o, _u8p) for o in offs[:n]])
         lens = (_sz * n)(*[len(q) for q in queries])
         capa = (_sz * n)(*caps)
         olen = (_sz * n)()
@@ -544,7 +564,7 @@ class KeywordServer:
             if sts[i]:
                 raise IprError(sts[i], f"respond_batch[{i}]")
         _check(st, "respond_batch")
-        return [bytes(obufs[i])[:olen[i]] for i in range(n)]
+        return [out[offs[i]:offs[i] + olen[i]].tobytes() for i in range(n)]
 
     def prepare_batch(self, max_payloads: int = 64):
         _check(_prepare_batch(self._h, max_payloads), "prepare_batch")
@@ -800,20 +820,20 @@ class KeywordClient:
             nonce, self._nonce = self._nonce, self._nonce + 1
         b = (_u64 * max(len(buckets), 1))(*buckets)
         need = query_bytes(self.plan.db_rows, len(buckets))
-        out = (ctypes.c_uint8 * need)()
+        out, outp = _output(need)
         n = _sz()
-        _check(_cl_query(self._h, nonce, len(buckets), b, out, need, ctypes.byref(n)), "ipr_client_query")
-        return bytes(out)
+        _check(_cl_query(self._h, nonce, len(buckets), b, outp, need, ctypes.byref(n)), "ipr_client_query")
+        return out.tobytes()
 
     def decrypt(self, response: bytes):
         """plaintexts [responses][c][2048] (u16 mod 65535) of a serialized response"""
         import numpy as np
-        buf = (ctypes.c_uint8 * max(len(response), 1)).from_buffer_copy(response or b"\0")
+        keep, buf = _input(response or b"\0")
         n = _sz()
         st = _cl_decrypt(self._h, buf, len(response), None, 0, ctypes.byref(n))
         if st not in (0, -6):
             _check(st, "ipr_client_decrypt")
-        vals = np.zeros(n.value, dtype=np.uint16)
+        vals = np.empty(n.value, dtype=np.uint16)
         _check(_cl_decrypt(self._h, buf, len(response), vals.ctypes.data_as(ctypes.POINTER(ctypes.c_uint16)),
                            vals.size, ctypes.byref(n)), "ipr_client_decrypt")
         return vals.reshape(-1, self.plan.c, POLY_LEN)

@@ -902,9 +902,12 @@ int ipr_server_respond_batch(ipr_server* s, int n, const uint8_t* const* queries
         int st = ensure_batch(s, B);
         if (st == IPR_OK) {
             CU(cudaSetDevice(s->device));
-            for (int b = 0; b < B; b++) std::memcpy(s->h_bq + (size_t)b * qb, queries[batchable[c0 + b]], qb);
             CU(cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream));
-            CU(cudaMemcpyAsync(s->d_bq, s->h_bq, (size_t)B * qb, cudaMemcpyHostToDevice, s->stream));
+            for (int b = 0; b < B; b++) {  // a payload's upload runs while the next one is staged
+                std::memcpy(s->h_bq + (size_t)b * qb, queries[batchable[c0 + b]], qb);
+                CU(cudaMemcpyAsync(s->d_bq + (size_t)b * qb, s->h_bq + (size_t)b * qb, qb, cudaMemcpyHostToDevice,
+                                   s->stream));
+            }
             st = enqueue_batch(s, B, s->d_bq, s->d_bresp, next_profile_slot(s));
             if (st == IPR_OK) {
                 CU(cudaMemcpyAsync(s->h_bresp, s->d_bresp, (size_t)B * rb, cudaMemcpyDeviceToHost, s->stream));
