@@ -11,13 +11,12 @@
 //
 // B200 design.  Every twiddle X^e of the pass has e a multiple of S = 2N/I, so a shift
 // moves whole chunks of S coefficients and keeps the offset o = k mod S: the pass
-// splits into S independent sub-problems of I polynomials x I/2 chunks.  One CTA takes
-// 32 DB rows x one (fold group, offset): it reads its 32 x I x I/2 values once (16-byte
-// accesses of 8 rows, 64 bytes per column), runs all log2(I) levels in shared memory
-// (in place: each step reads its inputs into registers before a barrier, 8 rows
-// per thread and step), scales, and writes them back once — one HBM
-// round trip for the whole encode where the reference makes one per level plus a
-// gather and a scatter.
+// splits into S independent sub-problems of I polynomials x I/2 chunks.  The first three
+// levels stay inside sets of 8 polynomials x 4 chunks and the last two, after a fixed rotation
+// of each polynomial, inside sets of 4 x 2, so a warp takes 64 DB rows of such a set in
+// registers (32 words of two rows each per lane) and the values cross shared memory once
+// between the two rounds: one HBM round trip for the whole encode where the reference makes
+// one per level plus a gather and a scatter.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -30,7 +29,7 @@ void set_last_error(const char* msg);
 
 namespace {
 
-constexpr int E_ROWS = 32;  // DB rows per CTA (four 16-byte groups per column)
+constexpr int E_ROWS = 32;  // the row count is a multiple of this
 constexpr uint32_t PMOD = 65535;
 
 __device__ __forceinline__ uint32_t fold65535(uint32_t x) {
@@ -127,128 +126,168 @@ __global__ void k_encode_scale1(const uint16_t* __restrict__ in, uint16_t* __res
         out[i] = (uint16_t)fold65535(in[i]);
 }
 
-// a + b mod 65535 on both 16-bit halves (ones'-complement sum: the carry out of a half is
-// added back into it; operands and result in [0, 65535] with 65535 = 0).  One 64-bit add
-// gives the high half's carry c1 and the carry c0 out of the low half (bit 16 of
-// s ^ a ^ b); c0 moves from the high half back into the low one, c1 re-enters the high
-// half, and neither re-addition can carry again.
-__device__ __forceinline__ uint32_t oadd2(uint32_t a, uint32_t b) {
-    const uint64_t s64 = (uint64_t)a + b;
-    const uint32_t s = (uint32_t)s64;
-    const uint32_t c1 = (uint32_t)(s64 >> 32);
-    const uint32_t c0 = ((s ^ a ^ b) >> 16) & 1u;
-    return s + c0 * 0xFFFF0001u + (c1 << 16);
+constexpr int E_THREADS = 256, E_TILE = 64;  // 8 warps, 64 DB rows (2 per lane)
+
+// a + b * s on the multiply pipe: `s` is a kernel argument (1 or -1), so that the sums do not
+// compete with the shifts, permutes and minima for the ALU pipe
+__device__ __forceinline__ uint32_t e_add(uint32_t a, uint32_t b, uint32_t s) { return a + b * s; }
+
+// one radix-G pass (G a power of two) over G positions x G/2 ring elements, two unpacked rows:
+// level lv pairs positions ev, ev + 2^lv, the second one turned by G t / 2^(lv+1) elements of a ring in
+// which element G/2 is minus element 0.  Signed sums: below 65536 G in magnitude.
+template <int G>
+__device__ __forceinline__ void e_radix(uint32_t (&lo)[G][G > 1 ? G / 2 : 1], uint32_t (&hi)[G][G > 1 ? G / 2 : 1],
+                                        uint32_t one, uint32_t minus) {
+    constexpr int M = G > 1 ? G / 2 : 1;
+#pragma unroll
+    for (int half = 1; half < G; half *= 2) {
+#pragma unroll
+        for (int ev = 0; ev < G; ev++) {
+            if (ev & half) continue;
+            const int od = ev + half, t = ev % half;
+            uint32_t a[M], b[M];
+#pragma unroll
+            for (int m = 0; m < M; m++) a[m] = lo[od][m], b[m] = hi[od][m];
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                const int src = (m + G * t / (2 * half)) % G;
+                const uint32_t x = lo[ev][m], y = hi[ev][m], u = a[src % M], v = b[src % M];
+                const uint32_t s = src >= M ? minus : one, d = src >= M ? one : minus;
+                lo[ev][m] = e_add(x, u, s);
+                lo[od][m] = e_add(x, u, d);
+                hi[ev][m] = e_add(y, v, s);
+                hi[od][m] = e_add(y, v, d);
+            }
+        }
+    }
 }
 
-// x * 2^K mod 65535 on both halves, canonical (65535 -> 0): multiplying by 2^K modulo
-// 2^16 - 1 rotates the 16 bits left by K; afterwards a half that is all ones (a zero
-// in ones'-complement form) is cleared
+// x mod 65535, canonical, for a signed x of magnitude below 65536 G, G <= 8
+template <int G>
+__device__ __forceinline__ uint32_t e_mod(uint32_t x, uint32_t one) {
+    const uint32_t y = x + one * (G * PMOD);         // below 2^20; on the multiply pipe
+    const uint32_t f = y - (y >> 16) * PMOD;         // (y mod 2^16) + (y >> 16) <= 65535 + 15
+    return __viaddmin_u32(f, 0u - PMOD, f);          // f - 65535 wraps above f when f < 65535
+}
+template <int G>
+__device__ __forceinline__ uint32_t e_pack(uint32_t lo, uint32_t hi, uint32_t one) {
+    return __byte_perm(e_mod<G>(lo, one), e_mod<G>(hi, one), 0x5410);
+}
+
+// both canonical halves times 2^K mod 65535: a rotation of the 16 bits (never all ones)
 template <int K>
-__device__ __forceinline__ uint32_t rotl_canon2(uint32_t w) {
-    constexpr uint32_t HI = ((0xFFFFu << K) & 0xFFFFu) * 0x10001u, LO = ((1u << K) - 1) * 0x10001u;
-    w = ((w << K) & HI) | ((w >> (16 - K)) & LO);
-    const uint32_t nw = ~w;
-    const uint32_t nz = ((nw & 0x7FFF7FFFu) + 0x7FFF7FFFu) | nw;  // bit 15 of a half: that half of nw != 0
-    const uint32_t ones = ~nz & 0x80008000u;
-    return w & ~((ones >> 15) * 0xFFFFu);
+__device__ __forceinline__ uint32_t e_scale(uint32_t w) {
+    constexpr uint32_t HI = ((0xFFFFu << K) & 0xFFFFu) * 0x10001u;
+    return ((w << K) & HI) | ((w >> (16 - K)) & ~HI);
 }
 
-constexpr int E_THREADS = 256;
+// I = 32: a CTA takes one offset o, each warp two sets of the first round and eight of the second;
+// I = 16: two offsets; I <= 8: an offset per warp, no second round.
+// Bound by integer issue (ALU pipe 66-80% busy), hence the sums on the multiply pipe and the second
+// round's chunk table.  250,000 ML-KEM-768 keys (interp 32, 1.6 GB): 414 us (3.9 TB/s) against
+// 508 us for packed sums with a pass over shared memory per level; interp 8: 33 against 61 us
+// at 16,384 columns.
+template <int I>
+__global__ void __launch_bounds__(E_THREADS, I > 8 ? 3 : 2) k_encode(const uint16_t* __restrict__ in, uint16_t* __restrict__ out,
+                                                         int64_t db_rows, uint32_t one, uint32_t minus) {
+    constexpr int H = I / 2;      // chunks of S coefficients in [0, N)
+    constexpr int S = 2 * N / I;  // coefficient stride between chunks
+    constexpr int LOGI = I == 2 ? 1 : I == 4 ? 2 : I == 8 ? 3 : I == 16 ? 4 : 5;
+    constexpr int G = I < 8 ? I : 8, M = G / 2, G2 = I / G, M2 = G2 > 1 ? G2 / 2 : 1;
+    constexpr int C1 = I / G;               // chunk step of the first round's sets
+    constexpr int SETS1 = G2 * C1;          // per offset
+    constexpr int SETS2 = G * (H / M2);
+    constexpr int OFFS = 8 / SETS1 > 0 ? 8 / SETS1 : 1;  // offsets per CTA
+    extern __shared__ uint32_t ebuf[];      // [offset][position][chunk][32 lanes]
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform
+    const int64_t row0 = (int64_t)blockIdx.x * E_TILE + 2 * lane;
+    const bool live = row0 < db_rows;
+    const int64_t row = live ? row0 : db_rows - 2;  // lanes past the end read the last rows and store nothing
+    const int64_t base = (int64_t)blockIdx.z * I * N + (int64_t)blockIdx.y * OFFS;  // first column
+    auto at = [&](int off, int poly, int chunk) {  // byte offset of this lane's two rows
+        return 2 * ((base + off + (int64_t)poly * N + (int64_t)chunk * S) * db_rows + row);
+    };
+    // within a set, every column is a compile-time multiple of these many bytes away
+    const uint32_t step = (uint32_t)(2 * (N / 4) * db_rows);  // a quarter polynomial
+    const char* inb = reinterpret_cast<const char*>(in);
+    char* outb = reinterpret_cast<char*>(out);
+    for (int set = warp; set < OFFS * SETS1; set += E_THREADS / 32) {
+        const int off = set / SETS1, grp = set % SETS1 / C1, c0 = set % C1;
+        uint32_t w[G][M], lo[G][M], hi[G][M];
+        // bit-reversed order: position grp * G + p holds polynomial brev(p) * G2 + brev(grp)
+        const char* src = inb + at(off, G2 > 1 ? (int)(__brev((unsigned)grp) >> (32 - (LOGI - 3))) : 0, c0);
+#pragma unroll
+        for (int p = 0; p < G; p++) {
+            int bp = 0;
+            for (int bit = 1, r = G / 2; bit < G; bit *= 2, r /= 2) bp += p & bit ? r : 0;
+#pragma unroll
+            for (int m = 0; m < M; m++)  // chunks C1 apart: N / M coefficients
+                w[p][m] = __ldg(reinterpret_cast<const uint32_t*>(src + (uint64_t)step * (bp * G2 * 4 + m * (4 / M))));
+        }
+#pragma unroll
+        for (int p = 0; p < G; p++)
+#pragma unroll
+            for (int m = 0; m < M; m++) hi[p][m] = w[p][m] >> 16, lo[p][m] = w[p][m] - hi[p][m] * 65536u;
+        e_radix<G>(lo, hi, one, minus);
+        uint32_t* dst = ebuf + ((off * I + grp * G) * H + c0) * 32 + lane;
+        char* od = outb + at(off, 0, c0);
+#pragma unroll
+        for (int p = 0; p < G; p++)
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                const uint32_t r = e_pack<G>(lo[p][m], hi[p][m], one);
+                if constexpr (G2 > 1) dst[(p * H + m * C1) * 32] = r;
+                else if (live)
+                    *reinterpret_cast<uint32_t*>(od + (uint64_t)step * (p * 4 + m * (4 / M))) = e_scale<16 - LOGI>(r);
+            }
+    }
+    if constexpr (G2 > 1) {
+        // chunk and sign of every value of the second round: {byte offset in the buffer, complement mask}
+        uint2* tab = reinterpret_cast<uint2*>(ebuf + OFFS * I * H * 32);  // [t][chunk of the set][g][m]
+        for (int i = threadIdx.x; i < SETS2 * G2 * M2; i += E_THREADS) {
+            const int m = i % M2, g = i / M2 % G2, c0 = i / (M2 * G2) % (H / M2), t = i / (M2 * G2 * (H / M2));
+            // the twiddles common to the set: X^-(S * shift) on position g * G + t
+            const int shift = (g & 1) * (I * t / (2 * G)) + (g >> 1) * (I * t / (4 * G));
+            const int c = (c0 + m * (H / 2) + shift) % I;
+            tab[i] = make_uint2((uint32_t)(((g * G + t) * H + c % H) * 32 * 4), c >= H ? 0xFFFFFFFFu : 0u);  // X^N = -1
+        }
+        __syncthreads();
+        for (int set = warp; set < OFFS * SETS2; set += E_THREADS / 32) {
+            const int off = set / SETS2, t = set % SETS2 / (H / M2), c0 = set % (H / M2);
+            uint32_t lo[G2][M2], hi[G2][M2];
+            const char* buf = reinterpret_cast<const char*>(ebuf + off * I * H * 32 + lane);
+            const uint2* tb = tab + set % SETS2 * (G2 * M2);
+#pragma unroll
+            for (int g = 0; g < G2; g++)
+#pragma unroll
+                for (int m = 0; m < M2; m++) {
+                    const uint2 e = tb[g * M2 + m];
+                    const uint32_t x = *reinterpret_cast<const uint32_t*>(buf + e.x) ^ e.y;
+                    hi[g][m] = x >> 16;
+                    lo[g][m] = x - hi[g][m] * 65536u;
+                }
+            e_radix<G2>(lo, hi, one, minus);
+            char* od = outb + at(off, t, c0);
+#pragma unroll
+            for (int g = 0; g < G2; g++)
+#pragma unroll
+                for (int m = 0; m < M2; m++)
+                    if (live)
+                        *reinterpret_cast<uint32_t*>(od + (uint64_t)step * (g * G * 4 + m * 2)) =
+                            e_scale<16 - LOGI>(e_pack<G2>(lo[g][m], hi[g][m], one));
+        }
+    }
+}
 
 template <int I>
-__global__ void __launch_bounds__(E_THREADS) k_encode(const uint16_t* __restrict__ in, uint16_t* __restrict__ out,
-                                                      int64_t db_rows) {
-    constexpr int H = I / 2;        // chunks of S coefficients in [0, N)
-    constexpr int S = 2 * N / I;    // coefficient stride between chunks
-    constexpr int RG = E_ROWS / 8;  // 8-row groups per column
-    constexpr int GROUPS = I * H * RG;
-    constexpr int BFLY = (I / 2) * H * RG;  // butterflies (of 8 rows) per level
-    constexpr int BPT = (BFLY + E_THREADS - 1) / E_THREADS;
-    constexpr int LOGI = I == 2 ? 1 : I == 4 ? 2 : I == 8 ? 3 : I == 16 ? 4 : 5;
-    __shared__ __align__(16) uint16_t buf[I][H][E_ROWS];  // [poly][chunk][row], 32 KB at interp 32
-    // row tiles vary fastest: the CTAs resident together read whole 4 KB columns between them
-    const int64_t row0 = (int64_t)blockIdx.x * E_ROWS;
-    const int o = blockIdx.y;         // offset within a chunk, < S
-    const int64_t wp = blockIdx.z;    // fold group
-    const int64_t col0 = wp * I * N + o;
-
-    // gather in bit-reversed polynomial order, 16 bytes (8 rows) per access; the loads of
-    // a thread are all issued before the first store
-    {
-        constexpr int LPT = (GROUPS + E_THREADS - 1) / E_THREADS;
-        uint4 v[LPT];
-#pragma unroll
-        for (int u = 0; u < LPT; u++) {
-            const int i = threadIdx.x + u * E_THREADS;
-            if (GROUPS % E_THREADS == 0 || i < GROUPS) {
-                const int rg = i % RG, q = i / RG;
-                const int j = q / H, kc = q % H;
-                v[u] = __ldg(reinterpret_cast<const uint4*>(in + (col0 + (int64_t)j * N + (int64_t)kc * S) * db_rows +
-                                                            row0 + rg * 8));
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < LPT; u++) {
-            const int i = threadIdx.x + u * E_THREADS;
-            if (GROUPS % E_THREADS == 0 || i < GROUPS) {
-                const int rg = i % RG, q = i / RG;
-                const int j = q / H, kc = q % H;
-                const int jr = (int)(__brev((unsigned)j) >> (32 - LOGI));
-                *reinterpret_cast<uint4*>(&buf[jr][kc][rg * 8]) = v[u];
-            }
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int lv = 0; lv < LOGI; lv++) {
-        const int gs = 2 << lv, half = 1 << lv;
-        // each butterfly reads its two inputs into registers; after a barrier all outputs
-        // overwrite them in place
-        uint4 ra[BPT], rb[BPT];
-#pragma unroll
-        for (int u = 0; u < BPT; u++) {
-            const int i = threadIdx.x + u * E_THREADS;
-            if (BFLY % E_THREADS == 0 || i < BFLY) {
-                const int rg = i % RG, rest = i / RG;
-                const int kc = rest % H, pr = rest / H;
-                const int g = pr / half, t = pr % half;
-                const int ev = g * gs + t, od = ev + half;
-                const int e = (2 * N - 2 * N * t / gs) % (2 * N);  // twiddle X^e, e a multiple of S
-                const int src = (kc + I - e / S) % I;                // chunk of coefficient k - e (mod 2N)
-                // two values per 32-bit word in ones'-complement form (65535 stands for 0):
-                // -x is ~x and a sum folds its carry back in, so the butterfly runs on packed halves
-                const uint4 ov = *reinterpret_cast<const uint4*>(&buf[od][src < H ? src : src - H][rg * 8]);
-                const uint4 evv = *reinterpret_cast<const uint4*>(&buf[ev][kc][rg * 8]);
-                const bool neg = src >= H;  // X^N = -1
-                const uint4 tw = neg ? make_uint4(~ov.x, ~ov.y, ~ov.z, ~ov.w) : ov;
-                ra[u] = make_uint4(oadd2(evv.x, tw.x), oadd2(evv.y, tw.y), oadd2(evv.z, tw.z), oadd2(evv.w, tw.w));
-                rb[u] = make_uint4(oadd2(evv.x, ~tw.x), oadd2(evv.y, ~tw.y), oadd2(evv.z, ~tw.z), oadd2(evv.w, ~tw.w));
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < BPT; u++) {
-            const int i = threadIdx.x + u * E_THREADS;
-            if (BFLY % E_THREADS == 0 || i < BFLY) {
-                const int rg = i % RG, rest = i / RG;
-                const int kc = rest % H, pr = rest / H;
-                const int ev = pr / half * gs + pr % half;
-                *reinterpret_cast<uint4*>(&buf[ev][kc][rg * 8]) = ra[u];
-                *reinterpret_cast<uint4*>(&buf[ev + half][kc][rg * 8]) = rb[u];
-            }
-        }
-        __syncthreads();
-    }
-    // scale by I^-1 = 2^(16 - log2 I) mod 65535 and store in natural polynomial order
-#pragma unroll 4
-    for (int i = threadIdx.x; i < GROUPS; i += E_THREADS) {
-        const int rg = i % RG, q = i / RG;
-        const int j = q / H, kc = q % H;
-        uint4 w = *reinterpret_cast<const uint4*>(&buf[j][kc][rg * 8]);
-        w = make_uint4(rotl_canon2<16 - LOGI>(w.x), rotl_canon2<16 - LOGI>(w.y), rotl_canon2<16 - LOGI>(w.z),
-                       rotl_canon2<16 - LOGI>(w.w));
-        *reinterpret_cast<uint4*>(out + (col0 + (int64_t)j * N + (int64_t)kc * S) * db_rows + row0 + rg * 8) = w;
-    }
+cudaError_t launch_encode(const uint16_t* in, uint16_t* out, uint64_t db_rows, unsigned groups, cudaStream_t st) {
+    constexpr int G = I < 8 ? I : 8, SETS1 = (I / G) * (I / G), OFFS = 8 / SETS1 > 0 ? 8 / SETS1 : 1;
+    constexpr int smem = I > 8 ? OFFS * I * (I / 2) * 32 * 4 + G * (I / 2) * (I / G) * 8 : 0;  // values, then the table
+    cudaError_t e = cudaFuncSetAttribute(k_encode<I>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((unsigned)((db_rows + E_TILE - 1) / E_TILE), 2 * N / I / OFFS, groups);
+    k_encode<I><<<grid, E_THREADS, smem, st>>>(in, out, (int64_t)db_rows, 1u, 0u - 1u);
+    return cudaGetLastError();
 }
 
 int cuda_status(cudaError_t e) {
@@ -288,14 +327,15 @@ int encode_db_device(const uint16_t* d_raw, uint16_t* d_out, uint64_t db_rows, u
     if (interp == 1) {
         k_encode_scale1<<<148 * 8, 256, 0, st>>>(d_raw, d_out, (int64_t)(db_rows * db_cols));
     } else {
-        const dim3 grid((unsigned)(db_rows / E_ROWS), (unsigned)(2 * N / interp), (unsigned)c);
+        cudaError_t e;
         switch (interp) {
-            case 2: k_encode<2><<<grid, E_THREADS, 0, st>>>(d_raw, d_out, (int64_t)db_rows); break;
-            case 4: k_encode<4><<<grid, E_THREADS, 0, st>>>(d_raw, d_out, (int64_t)db_rows); break;
-            case 8: k_encode<8><<<grid, E_THREADS, 0, st>>>(d_raw, d_out, (int64_t)db_rows); break;
-            case 16: k_encode<16><<<grid, E_THREADS, 0, st>>>(d_raw, d_out, (int64_t)db_rows); break;
-            default: k_encode<32><<<grid, E_THREADS, 0, st>>>(d_raw, d_out, (int64_t)db_rows); break;
+            case 2: e = launch_encode<2>(d_raw, d_out, db_rows, (unsigned)c, st); break;
+            case 4: e = launch_encode<4>(d_raw, d_out, db_rows, (unsigned)c, st); break;
+            case 8: e = launch_encode<8>(d_raw, d_out, db_rows, (unsigned)c, st); break;
+            case 16: e = launch_encode<16>(d_raw, d_out, db_rows, (unsigned)c, st); break;
+            default: e = launch_encode<32>(d_raw, d_out, db_rows, (unsigned)c, st); break;
         }
+        if (e != cudaSuccess) return cuda_status(e);
     }
     return cuda_status(cudaGetLastError());
 }

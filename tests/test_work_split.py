@@ -165,3 +165,20 @@ def test_ntt_of_any_word_alignment(pkg, orc, count, shift):
         pkg.ntt_batch(body.data_ptr(), count, limb, inverse=True)
         assert np.array_equal(body.cpu().numpy().view(np.uint64).reshape(count, N), polys)
         assert (d[:shift] == 5).all() and (d[shift + count * N:] == 5).all()
+
+
+@pytest.mark.parametrize("interp", [1, 2, 4, 8, 16, 32])
+@pytest.mark.parametrize("rows", [32, 64, 96])
+def test_encode_row_tiles(pkg, orc, interp, rows):
+    """half a 64-row tile, a whole one, one and a half; two fold groups; 65535 (zero) among the values"""
+    import numpy as np
+    import torch
+    cols = 2 * interp * N
+    raw = np.random.default_rng(interp + rows).integers(0, 65536, (cols, rows)).astype(np.uint16)
+    raw[0] = raw[-1] = 65535
+    d_raw = torch.from_numpy(raw.view(np.int16)).cuda()
+    d_out = torch.full((cols * rows + 64,), 9, dtype=torch.int16, device="cuda")
+    pkg.encode_db(d_raw.data_ptr(), d_out.data_ptr(), rows, cols, interp)
+    got = d_out.cpu().numpy().view(np.uint16)
+    assert np.array_equal(got[:cols * rows], orc.encode_db(raw.reshape(-1), rows, cols, interp))
+    assert (got[cols * rows:] == 9).all()
