@@ -103,17 +103,24 @@ void launch_ntt_limb(uint64_t* polys, int64_t count, uint32_t q, const uint2* tw
     }
 }
 
-// out[j][p][s] = in[p][auto_src(ks[j], s)]: one CTA stages one input polynomial in shared
-// memory and writes its image under every requested automorphism
+// out[j][p][s] = in[p][auto_src(ks[j], s)]: a CTA stages one input polynomial in shared memory and
+// writes its image under its share of the requested automorphisms (blockIdx.y with SPLIT, else
+// all).  Bound by the writes.
+// 256 polynomials under 64 automorphisms 45 us (6.1 TB/s); 64 under 64 15 us, against 37 us with a CTA
+// per polynomial alone.  More CTAs per SM, eight unrolled stores or 32-byte stores of four slots
+// measured 47.5 us at 256 x 64.
+template <bool SPLIT>
 __global__ void __launch_bounds__(256) k_automorph(const uint64_t* __restrict__ in, int64_t count,
                                                    const uint32_t* __restrict__ ks, int nk,
                                                    uint64_t* __restrict__ out) {
     __shared__ uint64_t poly[N];
+    const int j0 = SPLIT ? (int)((int64_t)nk * blockIdx.y / gridDim.y) : 0;
+    const int j1 = SPLIT ? (int)((int64_t)nk * (blockIdx.y + 1) / gridDim.y) : nk;
     for (int64_t p = blockIdx.x; p < count; p += gridDim.x) {
         __syncthreads();
         for (int s = threadIdx.x; s < N; s += blockDim.x) poly[s] = in[p * N + s];
         __syncthreads();
-        for (int j = 0; j < nk; j++) {
+        for (int j = j0; j < j1; j++) {
             const uint32_t k = __ldg(ks + j);
             uint64_t* o = out + ((int64_t)j * count + p) * N;
             for (int s = threadIdx.x; s < N; s += blockDim.x) o[s] = poly[auto_src(k, (uint32_t)s)];
@@ -209,9 +216,13 @@ int ipr_automorph_batch(int device, const uint64_t* d_in, uint64_t count, const 
     if (st) return st;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int64_t grid = std::min<int64_t>((int64_t)count, (int64_t)sms * 8);
-    ipr::k_automorph<<<(unsigned)grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(d_in, (int64_t)count, d_ks, nk,
-                                                                                   d_out);
+    // fewer polynomials than two CTAs per SM are shared out by automorphism
+    const int64_t gx = std::min<int64_t>((int64_t)count, (int64_t)sms * 8);
+    const int64_t gy = std::min<int64_t>(std::max<int64_t>((int64_t)sms * 2 / gx, 1), std::min(nk, 65535));
+    const dim3 grid((unsigned)gx, (unsigned)gy);
+    auto cs = static_cast<cudaStream_t>(stream);
+    if (gy > 1) ipr::k_automorph<true><<<grid, 256, 0, cs>>>(d_in, (int64_t)count, d_ks, nk, d_out);
+    else ipr::k_automorph<false><<<grid, 256, 0, cs>>>(d_in, (int64_t)count, d_ks, nk, d_out);
     return ipr::cuda_status(cudaGetLastError());
 }
 
