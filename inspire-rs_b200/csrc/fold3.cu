@@ -566,7 +566,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
         uint32_t o[EPT];
         exchange(1, n, rank ^ 1, pr, o);
 #pragma unroll
-        for (int m = 0; m < EPT; m++) x[m] = add_q(l ? crt2m(o[m], pr[m]) : crt2m(pr[m], o[m]), pk[m]);
+        for (int m = 0; m < EPT; m++) x[m] = add_q(crt2m(l ? o[m] : pr[m], l ? pr[m] : o[m]), pk[m]);
     };
     if (t == 0) {
         for (int i = 0; i < 4; i++) umma::mbar_init(bars + i, 1);

@@ -247,10 +247,11 @@ __device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8]) {
 // reduced ones; their N^-1 sits in the W mask (with the Montgomery R) and in F.
 // One instance (2 chains) 4.6 us a step, 74 instances (two chains' CTAs per SM) 7.5 us, against
 // 14 us a step for one 512-thread CTA per chain, which also stored bold_t in 4-byte pieces.
-// A cluster barrier per exchange in place of the counted stores: 5.0 us (its memory barrier);
-// more registers (one CTA per SM, 138 instead of 128) measured the same.
-template <bool WROWS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
+// A cluster barrier per exchange in place of the counted stores: 5.0 us (its memory barrier); a
+// team of 256 threads per digit: 5.4 us (two more CTA barriers).  FEW, for at most one CTA per
+// SM, has the registers to load twiddles above the barriers: 4.4 us.
+template <bool WROWS, bool FEW>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, FEW ? 1 : 2)
     k_off_collapse(const uint32_t* __restrict__ F, int64_t inst0, const uint32_t* __restrict__ wmask,
                    const uint2* __restrict__ fwi, const uint2* __restrict__ iwi, CollapseScale sc,
                    uint64_t* __restrict__ bt, uint64_t* __restrict__ btb, uint32_t* __restrict__ r0,
@@ -287,14 +288,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
     };
     // y (N^-1 times the limb's values, layout D) -> x: inverse transform, exchange, CRT
     auto to_raw2 = [&](uint32_t n, uint32_t bytes) {
-        nttl::inverse_one(y, t, &sm.xb[0][0], 1, iw, q);
+        nttl::inverse_one<FEW>(y, t, &sm.xb[0][0], 1, iw, q);
         send(n, 0, y[0], y[1], y[2], y[3]);
         send(n, 1, y[4], y[5], y[6], y[7]);
         receive(n, bytes);
         const uint4 a = sm.ex[n & 1][0][t], b = sm.ex[n & 1][1][t];
         const uint32_t o[EPT] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int m = 0; m < EPT; m++) x[m] = g ? crt2m(o[m], y[m]) : crt2m(y[m], o[m]);
+        for (int m = 0; m < EPT; m++) x[m] = crt2m(g ? o[m] : y[m], g ? y[m] : o[m]);
     };
     if (t == 0) {
         umma::mbar_init(&sm.bars[0], 1);
@@ -318,7 +319,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
         for (int m = 0; m < EPT; m++)
 #pragma unroll
             for (int k = 0; k < 3; k++) v[k][m] = (uint32_t)((x[m] >> (GADGET_BITS * k)) & MASK19);
-        nttl::forward_digits<3>(v, t, &sm.xb[0][0], 1, fw, q);
+        nttl::forward_digits<3, FEW>(v, t, &sm.xb[0][0], 1, fw, q);
         uint32_t own[3][4];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
@@ -525,12 +526,26 @@ CollapseScale collapse_scale() {
 // shared-memory sizes of the collapse kernels, on the current device
 cudaError_t collapse_attributes() {
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_off_collapse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(ChainSmem))) ||
-        (e = cudaFuncSetAttribute(k_off_collapse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(ChainSmem))))
+    const int smem = (int)sizeof(ChainSmem);
+    if ((e = cudaFuncSetAttribute(k_off_collapse<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+        (e = cudaFuncSetAttribute(k_off_collapse<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+        (e = cudaFuncSetAttribute(k_off_collapse<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
         return e;
     return cudaFuncSetAttribute(k_off_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CollapseSmem));
+}
+
+// the collapse of c instances from F; wrows as k_off_collapse
+void launch_collapse(const uint32_t* F, int64_t inst0, int64_t c, const uint32_t* wmask, const uint2* fw, const uint2* iw,
+                     uint64_t* bt, uint64_t* btb, uint32_t* r0, uint64_t* xb, int* err_flag, int sm_count,
+                     cudaStream_t st) {
+    const dim3 grid((unsigned)(2 * c), 2);
+    const int smem = (int)sizeof(ChainSmem);
+    if (4 * c <= sm_count)
+        k_off_collapse<false, true><<<grid, 256, smem, st>>>(F, inst0, wmask, fw, iw, collapse_scale(), bt, btb, r0, xb,
+                                                             nullptr, err_flag);
+    else
+        k_off_collapse<false, false><<<grid, 256, smem, st>>>(F, inst0, wmask, fw, iw, collapse_scale(), bt, btb, r0, xb,
+                                                              nullptr, err_flag);
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
@@ -558,7 +573,7 @@ cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar
     k_off_to_f<<<148 * 8, 256, 0, st>>>(r_all, r_bar_all, cols, F);
     uint2* it = reinterpret_cast<uint2*>(itab);
     k_interleave<<<2 * N / 256, 256, 0, st>>>(fw, fwp, iw, it, it + 2 * N);
-    k_off_collapse<true><<<dim3((unsigned)(2 * cols), 2), 256, (int)sizeof(ChainSmem), st>>>(
+    k_off_collapse<true, false><<<dim3((unsigned)(2 * cols), 2), 256, (int)sizeof(ChainSmem), st>>>(
         F, 0, nullptr, it, it + 2 * N, collapse_scale(), bt, btb, r0, xb, wrows, err_flag);
     k_off_finish<<<(unsigned)cols, 512, coll_smem, st>>>(r0, xb, 0, vmask, fw, fwp, iw, iwp, bth, a_hat);
     return cudaGetLastError();
@@ -588,6 +603,10 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
         set_last_error("offline precomputation: db_rows must be a positive multiple of 2048, instances > 0");
         return IPR_E_ARGS;
     }
+    int device = 0, sm_count = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        sm_count = 0;  // the general form
     HostParams hp;
     host_params_init(hp);
     std::vector<uint32_t> query, wmask, vmask;
@@ -648,9 +667,8 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
                                                                         d_query, fwi, d_act);
             k_off_jntt<<<dim3(N / JS, (unsigned)c, 2), 256, JNTT_SMEM, st>>>(d_act, c, fwi, d_E);
             k_off_gather<<<dim3(N / GZ, (unsigned)c, 2), 256, gather_smem, st>>>(d_E, c, d_act);  // F reuses act
-            k_off_collapse<false><<<dim3((unsigned)(2 * c), 2), 256, (int)sizeof(ChainSmem), st>>>(
-                d_act, (int64_t)i0, d_wm, reinterpret_cast<uint2*>(d_fwi), reinterpret_cast<uint2*>(d_iwi),
-                collapse_scale(), d_bt, d_btb, d_r0, d_xb, nullptr, d_err);
+            launch_collapse(d_act, (int64_t)i0, c, d_wm, fwi, reinterpret_cast<uint2*>(d_iwi), d_bt, d_btb, d_r0, d_xb,
+                            d_err, sm_count, st);
             k_off_finish<<<(unsigned)c, 512, coll_smem, st>>>(d_r0, d_xb, (int64_t)i0, d_vm, d_fw, d_fwp, d_iw, d_iwp,
                                                               d_bth, d_a_hat);
             if ((e = cudaGetLastError()) != cudaSuccess) status = cuda_fail(e, "launch");
@@ -787,9 +805,8 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     k_off_jntt<<<dim3(N / JS, (unsigned)sets, 2), 256, JNTT_SMEM, st>>>(c->act, sets, reinterpret_cast<uint2*>(c->fwi),
                                                                         c->E);
     k_off_gather<<<dim3(N / GZ, (unsigned)sets, 2), 256, N * GZ * 4, st>>>(c->E, sets, c->act);
-    k_off_collapse<false><<<dim3((unsigned)(2 * sets), 2), 256, (int)sizeof(ChainSmem), st>>>(
-        c->act, 0, c->wm, reinterpret_cast<uint2*>(c->fwi), reinterpret_cast<uint2*>(c->iwi), collapse_scale(), c->bt,
-        c->btb, c->r0, c->xb, nullptr, c->d_err);
+    launch_collapse(c->act, 0, sets, c->wm, reinterpret_cast<uint2*>(c->fwi), reinterpret_cast<uint2*>(c->iwi), c->bt,
+                    c->btb, c->r0, c->xb, c->d_err, c->sm_count, st);
     k_off_finish<<<(unsigned)sets, 512, coll_smem, st>>>(c->r0, c->xb, 0, c->vm, c->fw, c->fwp, c->iw, c->iwp, c->bth,
                                                          c->a_hat);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "offline kernels");
