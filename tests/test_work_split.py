@@ -182,3 +182,29 @@ def test_encode_row_tiles(pkg, orc, interp, rows):
     got = d_out.cpu().numpy().view(np.uint16)
     assert np.array_equal(got[:cols * rows], orc.encode_db(raw.reshape(-1), rows, cols, interp))
     assert (got[cols * rows:] == 9).all()
+
+
+@pytest.mark.parametrize("sets", [1, 2, 38])
+def test_inspiring_pack_of_any_word_alignment(pkg, sets):
+    """LWE matrices 8 bytes past a 32-byte boundary pack like aligned ones, alone and beside others;
+    38 sets are more chains than SMs"""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(sets)
+    q0, q1 = 268369921, 249561089
+    one = (N + 1) * N
+    lwe = torch.randint(0, q0 * q1, (sets * one,), dtype=torch.int64, device="cuda", generator=gen)
+    keys = [torch.randint(0, q0, (3, N), dtype=torch.int64, device="cuda", generator=gen)
+            | (torch.randint(0, q1, (3, N), dtype=torch.int64, device="cuda", generator=gen) << 32) for _ in range(2)]
+    moved = torch.empty(sets * one + 4, dtype=torch.int64, device="cuda")[1:1 + sets * one]
+    moved.copy_(lwe)
+    assert lwe.data_ptr() % 32 == 0 and moved.data_ptr() % 32 == 8
+    outs = []
+    with pkg.InspiringPacker(sets) as packer:
+        for d in (lwe, moved):
+            out = torch.zeros((sets, 2, N), dtype=torch.int64, device="cuda")
+            packer.pack(sets, d.data_ptr(), keys[0].data_ptr(), keys[1].data_ptr(), out.data_ptr())
+            outs.append(out.cpu())
+        last = torch.zeros((1, 2, N), dtype=torch.int64, device="cuda")
+        packer.pack(1, lwe[-one:].data_ptr(), keys[0].data_ptr(), keys[1].data_ptr(), last.data_ptr())
+        assert torch.equal(outs[0], outs[1])
+        assert torch.equal(last.cpu()[0], outs[0][-1])
