@@ -219,8 +219,13 @@ struct ChainSmem {
 
 constexpr uint32_t INV5 = 3277;  // 5^-1 mod 2N
 
-// 32-byte store of eight words (one L2 sector)
-__device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8]) {
+// store of eight words, one L2 sector when the array is 32-byte aligned (`wide`)
+__device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8], bool wide) {
+    if (!wide) {
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) reinterpret_cast<uint64_t*>(p)[i / 2] = (uint64_t)w[i] | ((uint64_t)w[i + 1] << 32);
+        return;
+    }
     asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
                  "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                  : "memory");
@@ -265,6 +270,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, FEW ? 1 : 2)
     const uint32_t q = limb_q(g);
     const uint32_t* Fc = F + (I * 2 + chain) * (int64_t)HALF * 2 * N + g * N;  // [i][l][z], this limb
     uint32_t* out = reinterpret_cast<uint32_t*>((chain ? btb : bt) + (inst0 + I) * (int64_t)NINNER * N);
+    const bool wide = reinterpret_cast<uintptr_t>(out) % 32 == 0;
     const uint2 *fw = fwi + g * N, *iw = iwi + g * N;
     const uint32_t nv = sc.ninv[2 * g], nvp = sc.ninv[2 * g + 1];
     if (!WROWS)
@@ -381,7 +387,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, FEW ? 1 : 2)
                 w[2 * m] = g ? o[m] : own[k][m];
                 w[2 * m + 1] = g ? own[k][m] : o[m];
             }
-            st_sector(out + (((int64_t)i * 3 + k) * N + z8 + 4 * g) * 2, w);
+            st_sector(out + (((int64_t)i * 3 + k) * N + z8 + 4 * g) * 2, w, wide);
         }
     }
     if (chain == 1 && g == 0)

@@ -208,3 +208,22 @@ def test_inspiring_pack_of_any_word_alignment(pkg, sets):
         packer.pack(1, lwe[-one:].data_ptr(), keys[0].data_ptr(), keys[1].data_ptr(), last.data_ptr())
         assert torch.equal(outs[0], outs[1])
         assert torch.equal(last.cpu()[0], outs[0][-1])
+
+
+@pytest.mark.parametrize("instances", [2, 38])
+def test_offline_outputs_of_any_word_alignment(pkg, instances):
+    """outputs 8 bytes past a 32-byte boundary, and several instances per pass, equal aligned ones"""
+    import torch
+    db = torch.randint(0, 65535, (instances * N, N), dtype=torch.int32, device="cuda",
+                       generator=torch.Generator(device="cuda").manual_seed(instances)).to(torch.int16)
+    sizes = [instances * N, instances * 3069 * N, instances * 3069 * N, instances * 3 * N]
+    got = []
+    for shift, scratch in ((0, 0), (1, 0), (2, 0), (0, 1)):
+        bufs = [torch.full((n + 8,), 3, dtype=torch.int64, device="cuda") for n in sizes]
+        outs = [b[shift:shift + n] for b, n in zip(bufs, sizes)]
+        pkg.offline_precompute(db.data_ptr(), N, instances, *[o.data_ptr() for o in outs], scratch_bytes=scratch)
+        assert all((b[:shift] == 3).all() and (b[shift + n:] == 3).all() for b, n in zip(bufs, sizes))
+        got.append(outs)
+        del bufs
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
