@@ -614,8 +614,11 @@ cudaError_t narrow_u64(const uint64_t* in, int64_t n, uint32_t* out, cudaStream_
     return cudaGetLastError();
 }
 
-// scratch bytes per instance: act / F (32 MB) + E (32 MB) + the chain ends (32 KB)
-constexpr uint64_t kOfflineScratchPerInstance = 2ull * 2 * N * N * 4 + 2ull * N * 4 + (uint64_t)N * 8;
+// scratch bytes per instance: F (32 MB) and the chain ends (32 KB); act and E (32 MB each) are
+// dead before the collapse writes bold_t and bold_t_bar (48 MB each per instance) and live there
+// when those are 16-byte aligned, else in scratch too
+constexpr uint64_t kOfflineScratchPerInstance = 2ull * N * N * 4 + 2ull * N * 4 + (uint64_t)N * 8;
+static_assert(2ull * N * N * 4 <= (uint64_t)NINNER * N * 8, "act and E fit in the outputs");
 
 int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t instances, uint64_t* d_a_hat,
                               uint64_t* d_bt, uint64_t* d_btb, uint64_t* d_bth, uint64_t scratch_budget,
@@ -635,7 +638,9 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
     offline_host_inputs(hp, (unsigned)(db_rows / N), query, wmask, vmask);
     // chunk of instances per pass, bounded by the scratch budget (0 = 4 GiB)
     const uint64_t budget = scratch_budget ? scratch_budget : (4ull << 30);
-    const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(instances, budget / kOfflineScratchPerInstance));
+    const bool in_place = ((reinterpret_cast<uintptr_t>(d_bt) | reinterpret_cast<uintptr_t>(d_btb)) & 15) == 0;
+    const uint64_t per = kOfflineScratchPerInstance + (in_place ? 0 : 2 * 2ull * N * N * 4);
+    const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(instances, budget / per));
     // one allocation for everything (each costs about 0.8 ms with its release): the parts, each a
     // multiple of 256 bytes
     const size_t tb = 2 * N * sizeof(uint32_t);
@@ -646,14 +651,14 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
         used += (bytes + 255) / 256 * 256;
         return at;
     };
-    const size_t o_act = part(chunk * 2ull * N * N * 4), o_E = part(chunk * 2ull * N * N * 4),
+    const size_t plane = chunk * 2ull * N * N * 4;
+    const size_t o_F = part(plane), o_act = part(in_place ? 0 : plane), o_E = part(in_place ? 0 : plane),
                  o_r0 = part(chunk * 2ull * N * 4), o_xb = part(chunk * (uint64_t)N * 8), o_tab = part(8 * tb),
                  o_query = part(query.size() * 4), o_wv = part(2 * wmask.size() * 4), o_err = part(sizeof(int));
     cudaError_t e = cudaMalloc(&d_scratch, used);
     if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");
     auto u32 = [&](size_t at) { return reinterpret_cast<uint32_t*>(d_scratch + at); };
-    uint32_t *d_tab = u32(o_tab), *d_query = u32(o_query), *d_wv = u32(o_wv), *d_act = u32(o_act), *d_E = u32(o_E),
-             *d_r0 = u32(o_r0);
+    uint32_t *d_tab = u32(o_tab), *d_query = u32(o_query), *d_wv = u32(o_wv), *d_F = u32(o_F), *d_r0 = u32(o_r0);
     uint64_t* d_xb = reinterpret_cast<uint64_t*>(d_scratch + o_xb);
     int* d_err = reinterpret_cast<int*>(d_scratch + o_err);
     uint32_t *d_fw = d_tab, *d_fwp = d_tab + 2 * N, *d_iw = d_tab + 4 * N, *d_iwp = d_tab + 6 * N;
@@ -685,11 +690,13 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
             const int64_t c = (int64_t)std::min<uint64_t>(chunk, instances - i0);
             const int64_t ncols = c * N;
             const uint2* fwi = reinterpret_cast<uint2*>(d_fwi);
+            uint32_t* d_act = in_place ? reinterpret_cast<uint32_t*>(d_bt + i0 * NINNER * N) : u32(o_act);
+            uint32_t* d_E = in_place ? reinterpret_cast<uint32_t*>(d_btb + i0 * NINNER * N) : u32(o_E);
             k_off_hint<<<dim3((unsigned)(ncols / HP), 2), 256, 0, st>>>(d_db, (int64_t)db_rows, (int64_t)i0 * N, ncols,
                                                                         d_query, fwi, d_act);
             k_off_jntt<<<dim3(N / JS, (unsigned)c, 2), 256, JNTT_SMEM, st>>>(d_act, c, fwi, d_E);
-            k_off_gather<<<dim3(N / GZ, (unsigned)c, 2), 256, gather_smem, st>>>(d_E, c, d_act);  // F reuses act
-            launch_collapse(d_act, (int64_t)i0, c, d_wm, fwi, reinterpret_cast<uint2*>(d_iwi), d_bt, d_btb, d_r0, d_xb,
+            k_off_gather<<<dim3(N / GZ, (unsigned)c, 2), 256, gather_smem, st>>>(d_E, c, d_F);
+            launch_collapse(d_F, (int64_t)i0, c, d_wm, fwi, reinterpret_cast<uint2*>(d_iwi), d_bt, d_btb, d_r0, d_xb,
                             d_err, sm_count, st);
             k_off_finish<<<(unsigned)c, 512, coll_smem, st>>>(d_r0, d_xb, (int64_t)i0, d_vm, d_fw, d_fwp, d_iw, d_iwp,
                                                               d_bth, d_a_hat);
