@@ -219,9 +219,10 @@ struct ChainSmem {
 
 constexpr uint32_t INV5 = 3277;  // 5^-1 mod 2N
 
-// store of eight words, one L2 sector when the array is 32-byte aligned (`wide`)
-__device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8], bool wide) {
-    if (!wide) {
+// store of eight words: one L2 sector at a time (WIDE: 32-byte aligned), else 8 bytes at a time
+template <bool WIDE>
+__device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8]) {
+    if (!WIDE) {
 #pragma unroll
         for (int i = 0; i < 8; i += 2) reinterpret_cast<uint64_t*>(p)[i / 2] = (uint64_t)w[i] | ((uint64_t)w[i + 1] << 32);
         return;
@@ -255,7 +256,7 @@ __device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8], b
 // A cluster barrier per exchange in place of the counted stores: 5.0 us (its memory barrier); a
 // team of 256 threads per digit: 5.4 us (two more CTA barriers).  FEW, for at most one CTA per
 // SM, has the registers to load twiddles above the barriers: 4.4 us.
-template <bool WROWS, bool FEW>
+template <bool WROWS, bool FEW, bool WIDE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, FEW ? 1 : 2)
     k_off_collapse(const uint32_t* __restrict__ F, int64_t inst0, const uint32_t* __restrict__ wmask,
                    const uint2* __restrict__ fwi, const uint2* __restrict__ iwi, CollapseScale sc,
@@ -270,7 +271,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, FEW ? 1 : 2)
     const uint32_t q = limb_q(g);
     const uint32_t* Fc = F + (I * 2 + chain) * (int64_t)HALF * 2 * N + g * N;  // [i][l][z], this limb
     uint32_t* out = reinterpret_cast<uint32_t*>((chain ? btb : bt) + (inst0 + I) * (int64_t)NINNER * N);
-    const bool wide = reinterpret_cast<uintptr_t>(out) % 32 == 0;
     const uint2 *fw = fwi + g * N, *iw = iwi + g * N;
     const uint32_t nv = sc.ninv[2 * g], nvp = sc.ninv[2 * g + 1];
     if (!WROWS)
@@ -387,7 +387,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, FEW ? 1 : 2)
                 w[2 * m] = g ? o[m] : own[k][m];
                 w[2 * m + 1] = g ? own[k][m] : o[m];
             }
-            st_sector(out + (((int64_t)i * 3 + k) * N + z8 + 4 * g) * 2, w, wide);
+            st_sector<WIDE>(out + (((int64_t)i * 3 + k) * N + z8 + 4 * g) * 2, w);
         }
     }
     if (chain == 1 && g == 0)
@@ -549,11 +549,19 @@ CollapseScale collapse_scale() {
 cudaError_t collapse_attributes() {
     cudaError_t e;
     const int smem = (int)sizeof(ChainSmem);
-    if ((e = cudaFuncSetAttribute(k_off_collapse<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
-        (e = cudaFuncSetAttribute(k_off_collapse<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
-        (e = cudaFuncSetAttribute(k_off_collapse<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
+    if ((e = cudaFuncSetAttribute(k_off_collapse<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+        (e = cudaFuncSetAttribute(k_off_collapse<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+        (e = cudaFuncSetAttribute(k_off_collapse<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+        (e = cudaFuncSetAttribute(k_off_collapse<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) ||
+        (e = cudaFuncSetAttribute(k_off_collapse<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
         return e;
     return cudaFuncSetAttribute(k_off_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CollapseSmem));
+}
+
+// whether the collapse can write whole 32-byte sectors (the branch inside the kernel's serial loop
+// made one instance 4.58 ms instead of 4.49, so it is a form of its own)
+bool whole_sectors(const uint64_t* bt, const uint64_t* btb) {
+    return ((reinterpret_cast<uintptr_t>(bt) | reinterpret_cast<uintptr_t>(btb)) & 31) == 0;
 }
 
 // the collapse of c instances from F; wrows as k_off_collapse
@@ -562,12 +570,10 @@ void launch_collapse(const uint32_t* F, int64_t inst0, int64_t c, const uint32_t
                      cudaStream_t st) {
     const dim3 grid((unsigned)(2 * c), 2);
     const int smem = (int)sizeof(ChainSmem);
-    if (4 * c <= sm_count)
-        k_off_collapse<false, true><<<grid, 256, smem, st>>>(F, inst0, wmask, fw, iw, collapse_scale(), bt, btb, r0, xb,
-                                                             nullptr, err_flag);
-    else
-        k_off_collapse<false, false><<<grid, 256, smem, st>>>(F, inst0, wmask, fw, iw, collapse_scale(), bt, btb, r0, xb,
-                                                              nullptr, err_flag);
+    const auto kernel = !whole_sectors(bt, btb)  ? k_off_collapse<false, false, false>
+                        : 4 * c <= sm_count ? k_off_collapse<false, true, true>
+                                            : k_off_collapse<false, false, true>;
+    kernel<<<grid, 256, smem, st>>>(F, inst0, wmask, fw, iw, collapse_scale(), bt, btb, r0, xb, nullptr, err_flag);
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
@@ -595,7 +601,8 @@ cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar
     k_off_to_f<<<148 * 8, 256, 0, st>>>(r_all, r_bar_all, cols, F);
     uint2* it = reinterpret_cast<uint2*>(itab);
     k_interleave<<<2 * N / 256, 256, 0, st>>>(fw, fwp, iw, it, it + 2 * N);
-    k_off_collapse<true, false><<<dim3((unsigned)(2 * cols), 2), 256, (int)sizeof(ChainSmem), st>>>(
+    const auto kernel = whole_sectors(bt, btb) ? k_off_collapse<true, false, true> : k_off_collapse<true, false, false>;
+    kernel<<<dim3((unsigned)(2 * cols), 2), 256, (int)sizeof(ChainSmem), st>>>(
         F, 0, nullptr, it, it + 2 * N, collapse_scale(), bt, btb, r0, xb, wrows, err_flag);
     k_off_finish<<<(unsigned)cols, 512, coll_smem, st>>>(r0, xb, 0, vmask, fw, fwp, iw, iwp, bth, a_hat);
     return cudaGetLastError();
