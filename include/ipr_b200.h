@@ -191,7 +191,8 @@ int ipr_server_set_profiling(ipr_server *srv, int on);
 #define IPR_OPT_TENSOR_GEMV 1
 /* IPR_OPT_FOLD_REGISTER_NTT: the form of the RGSW fold.  3 (default) = register-
  * resident NTTs with the packing post-process (INTT + CRT + b add) fused into the
- * fold's own inverse transforms, one chain per CTA, chosen per call between two CTAs
+ * fold's own inverse transforms, one chain per CTA, chosen per call between a cluster of four CTAs per
+ * chain (few chains), two CTAs
  * per SM (the query's RGSW bodies staged through shared memory) and three per SM (the
  * bodies read from L2 where they are used) by the rounds each needs for the call's
  * chains; 4 = always three per SM; 5 = always two per SM; 2 = the same fused fold on two chains of one
@@ -306,7 +307,9 @@ int ipr_offline_precompute(int device, const uint16_t *d_db, uint64_t db_rows, u
  * mod q1).  d_out [sets][2][2048] u64: row 0 = a_hat mod q, row 1 = b + the packed
  * sum mod q (not reduced, < 2q, as add_raw leaves it).  The context holds the
  * tables, the W / V masks and scratch for up to max_sets sets (about 150 MB each);
- * calls on one context must not overlap on the GPU. */
+ * calls on one context must not overlap on the GPU.  A bounded device-side wait that ran
+ * out makes the next ipr_inspiring_pack on the context return IPR_E_TIMEOUT (and
+ * ipr_offline_precompute, which waits for its outputs, return it itself). */
 typedef struct ipr_inspiring ipr_inspiring;
 int ipr_inspiring_create(int device, int max_sets, ipr_inspiring **out);
 int ipr_inspiring_pack(ipr_inspiring *ctx, int sets, const uint64_t *d_lwe, const uint64_t *d_y_body,
