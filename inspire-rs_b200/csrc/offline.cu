@@ -19,8 +19,7 @@
 // itself is the slot permutation tau_{-1} of NTT(DB column) * query: the hint's INTT/NTT
 // pair cancels.  Kernels, per limb:
 //   k_off_hint     column NTTs of the DB, * query, tau_{-1}          -> act[l][I][j][s]
-//   k_off_jntt     NTT over j of 8 slots per CTA, * N^-1             -> E[l][I][s][z]
-//   k_off_gather   per 8-column tile of E, the two slot gathers        -> F[I][chain][i][l][z]
+//   k_off_jntt     NTT over j of 8 slots per CTA, * N^-1, the gather -> F[I][chain][i][l][z]
 //   k_off_collapse one CTA pair per (instance, chain): 1023 sequential steps of register NTTs
 //   k_off_finish   bold_t_hat and a_hat per instance
 // All values leave canonical, so the outputs equal the reference's bit for bit.
@@ -51,7 +50,6 @@ constexpr int HALF = N / 2;   // packing outputs per instance (num_to_pack_half)
 constexpr int HCOLS = 4;      // LWE columns per CTA in k_lwe_prep
 constexpr int HP = 2;         // DB columns per CTA in k_off_hint
 constexpr int JS = 8;         // slots per CTA in k_off_jntt
-constexpr int GZ = 8;         // z columns per CTA in k_off_gather
 constexpr uint64_t MASK19 = (1ull << GADGET_BITS) - 1;
 
 __device__ __forceinline__ uint32_t limb_q(int g) { return g ? Q1 : Q0; }
@@ -63,6 +61,19 @@ __device__ __forceinline__ uint32_t gen_pow(uint32_t i) {
     for (; i; i >>= 1, b = (b * b) & (2 * N - 1))
         if (i & 1) r = (r * b) & (2 * N - 1);
     return r;
+}
+
+// store of eight words: one L2 sector at a time (WIDE: 32-byte aligned), else 8 bytes at a time
+template <bool WIDE>
+__device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8]) {
+    if (!WIDE) {
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) reinterpret_cast<uint64_t*>(p)[i / 2] = (uint64_t)w[i] | ((uint64_t)w[i + 1] << 32);
+        return;
+    }
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
 }
 
 // act[l][c][s] = tau_{-1}-permuted NTT_l(DB column c) * query, for chunk-local columns c.
@@ -115,11 +126,54 @@ __global__ void __launch_bounds__(256, 4)
     }
 }
 
+// rows of F: v[u >> 1] = chain * HALF + i with u = 5^i (chain 0) or -5^i (chain 1) mod 2N; every
+// odd u is one of them
+struct RowOfPower {
+    uint16_t v[N];
+};
+constexpr RowOfPower rows_of_powers() {
+    RowOfPower r{};
+    uint32_t u = 1;
+    for (int i = 0; i < HALF; i++, u = u * 5 % (2 * N)) {
+        r.v[u >> 1] = (uint16_t)i;
+        r.v[(2 * N - u) >> 1] = (uint16_t)(HALF + i);
+    }
+    return r;
+}
+__device__ const RowOfPower d_row_of_power = rows_of_powers();
+
+__host__ __device__ constexpr int rev3(int x) { return ((x & 1) << 2) | (x & 2) | ((x >> 2) & 1); }
+
+// E[s][z] = v[s - s0][z - z8], s = s0 .. s0 + 7, z = z8 .. z8 + 7 -> the F sectors made of them.
+// A group of eight slots has exponents e + 512 r (r = the reversed low bits of the slot), and
+// u (e + 512 r) = u e + 512 u r: tau_u takes groups to groups.  The eight u that take this z group
+// to this s group are (e_s + 512 h) / e_z, h = 0 .. 7, all with the same u mod 8 = A, and tau_u
+// takes r to h + A r.
+template <int A>
+__device__ __forceinline__ void store_sectors(const uint32_t (&v)[JS][EPT], uint32_t es, uint32_t ez_inv,
+                                              uint32_t* __restrict__ F) {
+#pragma unroll
+    for (int h = 0; h < 8; h++) {
+        const uint32_t u = ((es + 512 * h) * ez_inv) & (2 * N - 1);
+        uint32_t* dst = F + (int64_t)__ldg(&d_row_of_power.v[u >> 1]) * 2 * N;
+        uint32_t w[8];
+#pragma unroll
+        for (int m = 0; m < 8; m++) w[m] = v[rev3((h + A * rev3(m)) & 7)][m];
+        st_sector<true>(dst, w);
+    }
+}
+
 // E[l][I][s][z] = N^-1 * NTT over j of act[l][I][j][s], JS consecutive slots per CTA (the 32 bytes
-// of a row that they take are one sector).  grid (N / JS, instances, 2 limbs), 256 threads, 64 KB
-// of dynamic shared memory
+// of a row that they take are one sector).  GATHER: written as
+//   F[I][chain][i][l][z] = E[l][I][tau(z)][z], tau = tau_{5^i} (chain 0) or tau_{-5^i} (chain 1),
+// which a thread can do from its registers, a whole sector at a time (store_sectors); else as E
+// (`out`, 32-byte aligned, is not act).
+// 96 instances (act and F 3.2 GB each): 2.73 ms (2.4 TB/s; bound by the transforms' issue), against
+// 2.50 ms for writing E and 1.76 ms for a gather over tiles of eight columns of it.
+// grid (N / JS, instances, 2 limbs), 256 threads, 64 KB of dynamic shared memory
+template <bool GATHER>
 __global__ void __launch_bounds__(256, 2)
-    k_off_jntt(const uint32_t* __restrict__ act, int64_t inst, const uint2* __restrict__ fwi, uint32_t* __restrict__ E) {
+    k_off_jntt(const uint32_t* __restrict__ act, int64_t inst, const uint2* __restrict__ fwi, uint32_t* __restrict__ out) {
     extern __shared__ __align__(16) uint32_t jbuf[];  // [JS][N]
     const int t = threadIdx.x;
     const int s0 = blockIdx.x * JS, l = blockIdx.z;
@@ -136,42 +190,28 @@ __global__ void __launch_bounds__(256, 2)
     nttl::forward_digits<JS, false, true>(v, t, jbuf, 1, fwi + l * N, q);  // canonical in: below 15 q through stage 6
     const uint32_t ninv = q - (q - 1) / N, ninvp = (uint32_t)(((uint64_t)ninv << 32) / q);  // N^-1 mod q_l
 #pragma unroll
-    for (int p = 0; p < JS; p++) {
-        uint32_t o[EPT];
+    for (int p = 0; p < JS; p++)
 #pragma unroll
-        for (int k = 0; k < EPT; k++) o[k] = nttl::mul_canon(v[p][k], ninv, ninvp, q);
-        uint4* dst = reinterpret_cast<uint4*>(E + base + (int64_t)(s0 + p) * N + eD(t, 0));
-        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        for (int k = 0; k < EPT; k++) v[p][k] = nttl::mul_canon(v[p][k], ninv, ninvp, q);
+    const int z8 = eD(t, 0);
+    if (!GATHER) {
+#pragma unroll
+        for (int p = 0; p < JS; p++) st_sector<true>(out + base + (int64_t)(s0 + p) * N + z8, v[p]);
+        return;
+    }
+    const uint32_t es = exponent_of_slot((uint32_t)s0), ez = exponent_of_slot((uint32_t)z8);
+    uint32_t inv = ez;  // 1 / ez mod 8, then mod 64, 2^12
+    inv *= 2 - ez * inv;
+    inv *= 2 - ez * inv;
+    uint32_t* F = out + ((int64_t)blockIdx.y * 2 * HALF * 2 + l) * N + z8;
+    switch ((es * inv) & 7) {  // the same for a warp: ez mod 8 comes from the two high bits of t
+        case 1: store_sectors<1>(v, es, inv, F); break;
+        case 3: store_sectors<3>(v, es, inv, F); break;
+        case 5: store_sectors<5>(v, es, inv, F); break;
+        default: store_sectors<7>(v, es, inv, F); break;
     }
 }
 constexpr int JNTT_SMEM = JS * N * 4;
-
-// F[I][chain][i][l][z] = E[l][I][tau(z)][z], tau = tau_{5^i} (chain 0) or tau_{-5^i} (chain 1),
-// for a tile of GZ columns z.  grid (N / GZ, instances, 2 limbs), 256 threads, 64 KB dynamic smem
-__global__ void __launch_bounds__(256)
-    k_off_gather(const uint32_t* __restrict__ E, int64_t inst, uint32_t* __restrict__ F) {
-    extern __shared__ __align__(16) uint32_t tile[];  // [N][GZ]
-    const int t = threadIdx.x;
-    const int z0 = blockIdx.x * GZ, l = blockIdx.z;
-    const int64_t I = blockIdx.y;
-    const uint32_t* src = E + ((int64_t)l * inst + I) * N * N + z0;
-    for (int s = t; s < N; s += 256) {
-        const uint4* p = reinterpret_cast<const uint4*>(src + (int64_t)s * N);
-        const uint4 a = __ldg(p), b = __ldg(p + 1);
-        *reinterpret_cast<uint4*>(&tile[s * GZ]) = a;
-        *reinterpret_cast<uint4*>(&tile[s * GZ + 4]) = b;
-    }
-    __syncthreads();
-    uint32_t gi = gen_pow((uint32_t)t / GZ);  // 5^i of this thread's i = t / GZ + 256 / GZ * round
-    const uint32_t g_step = gen_pow(256 / GZ);
-    for (int idx = t; idx < HALF * GZ; idx += 256, gi = (gi * g_step) & (2 * N - 1)) {
-        const int i = idx / GZ, zz = idx % GZ;
-        const uint32_t z = (uint32_t)(z0 + zz);
-        F[(((I * 2 + 0) * HALF + i) * 2 + l) * N + z] = tile[auto_src(gi, z) * GZ + zz];
-        F[(((I * 2 + 1) * HALF + i) * 2 + l) * N + z] = tile[auto_src(2 * N - gi, z) * GZ + zz];
-    }
-}
 
 // smem of the finish kernel
 struct CollapseSmem {
@@ -218,19 +258,6 @@ struct ChainSmem {
 };
 
 constexpr uint32_t INV5 = 3277;  // 5^-1 mod 2N
-
-// store of eight words: one L2 sector at a time (WIDE: 32-byte aligned), else 8 bytes at a time
-template <bool WIDE>
-__device__ __forceinline__ void st_sector(uint32_t* p, const uint32_t (&w)[8]) {
-    if (!WIDE) {
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) reinterpret_cast<uint64_t*>(p)[i / 2] = (uint64_t)w[i] | ((uint64_t)w[i + 1] << 32);
-        return;
-    }
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                 : "memory");
-}
 
 // One cluster of two CTAs (one per limb) of 256 threads per (instance, chain); chain 0 folds
 // r_all with W rotated by 5^i into bold_t, chain 1 folds r_bar_all with W rotated by -5^i
@@ -610,9 +637,9 @@ cudaError_t offline_collapse_arrays(const uint64_t* r_all, const uint64_t* r_bar
 
 // E[l][I][s][z] = N^-1 * NTT over j of act[l][I][j][s] for `inst` instances
 cudaError_t offline_jntt(const uint32_t* act, int64_t inst, const uint2* fwi, uint32_t* E, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(k_off_jntt, cudaFuncAttributeMaxDynamicSharedMemorySize, JNTT_SMEM);
+    cudaError_t e = cudaFuncSetAttribute(k_off_jntt<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, JNTT_SMEM);
     if (e != cudaSuccess) return e;
-    k_off_jntt<<<dim3(N / JS, (unsigned)inst, 2), 256, JNTT_SMEM, st>>>(act, inst, fwi, E);
+    k_off_jntt<false><<<dim3(N / JS, (unsigned)inst, 2), 256, JNTT_SMEM, st>>>(act, inst, fwi, E);
     return cudaGetLastError();
 }
 
@@ -621,11 +648,11 @@ cudaError_t narrow_u64(const uint64_t* in, int64_t n, uint32_t* out, cudaStream_
     return cudaGetLastError();
 }
 
-// scratch bytes per instance: F (32 MB) and the chain ends (32 KB); act and E (32 MB each) are
-// dead before the collapse writes bold_t and bold_t_bar (48 MB each per instance) and live there
-// when those are 16-byte aligned, else in scratch too
+// scratch bytes per instance: F (32 MB) and the chain ends (32 KB); act (32 MB) is dead before the
+// collapse writes bold_t (48 MB per instance) and lives there when that is 16-byte aligned, else
+// in scratch too
 constexpr uint64_t kOfflineScratchPerInstance = 2ull * N * N * 4 + 2ull * N * 4 + (uint64_t)N * 8;
-static_assert(2ull * N * N * 4 <= (uint64_t)NINNER * N * 8, "act and E fit in the outputs");
+static_assert(2ull * N * N * 4 <= (uint64_t)NINNER * N * 8, "act fits in bold_t");
 
 int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t instances, uint64_t* d_a_hat,
                               uint64_t* d_bt, uint64_t* d_btb, uint64_t* d_bth, uint64_t scratch_budget,
@@ -645,8 +672,8 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
     offline_host_inputs(hp, (unsigned)(db_rows / N), query, wmask, vmask);
     // chunk of instances per pass, bounded by the scratch budget (0 = 4 GiB)
     const uint64_t budget = scratch_budget ? scratch_budget : (4ull << 30);
-    const bool in_place = ((reinterpret_cast<uintptr_t>(d_bt) | reinterpret_cast<uintptr_t>(d_btb)) & 15) == 0;
-    const uint64_t per = kOfflineScratchPerInstance + (in_place ? 0 : 2 * 2ull * N * N * 4);
+    const bool in_place = reinterpret_cast<uintptr_t>(d_bt) % 16 == 0;
+    const uint64_t per = kOfflineScratchPerInstance + (in_place ? 0 : 2ull * N * N * 4);
     const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(instances, budget / per));
     // one allocation for everything (each costs about 0.8 ms with its release): the parts, each a
     // multiple of 256 bytes
@@ -659,7 +686,7 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
         return at;
     };
     const size_t plane = chunk * 2ull * N * N * 4;
-    const size_t o_F = part(plane), o_act = part(in_place ? 0 : plane), o_E = part(in_place ? 0 : plane),
+    const size_t o_F = part(plane), o_act = part(in_place ? 0 : plane),
                  o_r0 = part(chunk * 2ull * N * 4), o_xb = part(chunk * (uint64_t)N * 8), o_tab = part(8 * tb),
                  o_query = part(query.size() * 4), o_wv = part(2 * wmask.size() * 4), o_err = part(sizeof(int));
     cudaError_t e = cudaMalloc(&d_scratch, used);
@@ -686,9 +713,8 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
             status = cuda_fail(e, "table upload");
             break;
         }
-        const int gather_smem = N * GZ * 4, coll_smem = (int)sizeof(CollapseSmem);
-        if ((e = cudaFuncSetAttribute(k_off_jntt, cudaFuncAttributeMaxDynamicSharedMemorySize, JNTT_SMEM)) ||
-            (e = cudaFuncSetAttribute(k_off_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, gather_smem)) ||
+        const int coll_smem = (int)sizeof(CollapseSmem);
+        if ((e = cudaFuncSetAttribute(k_off_jntt<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, JNTT_SMEM)) ||
             (e = collapse_attributes())) {
             status = cuda_fail(e, "kernel attributes");
             break;
@@ -698,11 +724,9 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
             const int64_t ncols = c * N;
             const uint2* fwi = reinterpret_cast<uint2*>(d_fwi);
             uint32_t* d_act = in_place ? reinterpret_cast<uint32_t*>(d_bt + i0 * NINNER * N) : u32(o_act);
-            uint32_t* d_E = in_place ? reinterpret_cast<uint32_t*>(d_btb + i0 * NINNER * N) : u32(o_E);
             k_off_hint<<<dim3((unsigned)(ncols / HP), 2), 256, 0, st>>>(d_db, (int64_t)db_rows, (int64_t)i0 * N, ncols,
                                                                         d_query, fwi, d_act);
-            k_off_jntt<<<dim3(N / JS, (unsigned)c, 2), 256, JNTT_SMEM, st>>>(d_act, c, fwi, d_E);
-            k_off_gather<<<dim3(N / GZ, (unsigned)c, 2), 256, gather_smem, st>>>(d_E, c, d_F);
+            k_off_jntt<true><<<dim3(N / JS, (unsigned)c, 2), 256, JNTT_SMEM, st>>>(d_act, c, fwi, d_F);
             launch_collapse(d_F, (int64_t)i0, c, d_wm, fwi, reinterpret_cast<uint2*>(d_iwi), d_bt, d_btb, d_r0, d_xb,
                             d_err, sm_count, st);
             k_off_finish<<<(unsigned)c, 512, coll_smem, st>>>(d_r0, d_xb, (int64_t)i0, d_vm, d_fw, d_fwp, d_iw, d_iwp,
@@ -751,7 +775,7 @@ struct ipr_inspiring {
     std::vector<void*> allocs;
     uint32_t *fw = nullptr, *fwp = nullptr, *iw = nullptr, *iwp = nullptr, *wm = nullptr, *vm = nullptr;
     uint32_t *fwi = nullptr, *iwi = nullptr;  // the twiddles interleaved with their companions
-    uint32_t *act = nullptr, *E = nullptr, *r0 = nullptr, *S = nullptr;
+    uint32_t *act = nullptr, *F = nullptr, *r0 = nullptr, *S = nullptr;
     int *h_err = nullptr, *d_err = nullptr;  // mapped host memory: a device-side wait ran out
     uint64_t *xb = nullptr, *a_hat = nullptr, *bt = nullptr, *btb = nullptr, *bth = nullptr, *R = nullptr;
     template <typename T>
@@ -793,7 +817,7 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
     if ((e = c->alloc(&c->fw, tb)) || (e = c->alloc(&c->fwp, tb)) || (e = c->alloc(&c->iw, tb)) ||
         (e = c->alloc(&c->iwp, tb)) || (e = c->alloc(&c->fwi, 2 * tb)) || (e = c->alloc(&c->iwi, 2 * tb)) || (e = c->alloc(&c->wm, wmask.size() * 4)) ||
         (e = c->alloc(&c->vm, vmask.size() * 4)) || (e = c->alloc(&c->act, ms * 2 * NN * 4)) ||
-        (e = c->alloc(&c->E, ms * 2 * NN * 4)) || (e = c->alloc(&c->r0, ms * 2 * ipr::N * 4)) ||
+        (e = c->alloc(&c->F, ms * 2 * NN * 4)) || (e = c->alloc(&c->r0, ms * 2 * ipr::N * 4)) ||
         (e = c->alloc(&c->xb, ms * ipr::N * 8)) || (e = c->alloc(&c->a_hat, ms * ipr::N * 8)) ||
         (e = c->alloc(&c->bt, ms * ipr::NINNER * ipr::N * 8)) || (e = c->alloc(&c->btb, ms * ipr::NINNER * ipr::N * 8)) ||
         (e = c->alloc(&c->bth, ms * 3 * ipr::N * 8)) || (e = c->alloc(&c->S, ms * 2 * ipr::N * 4)) ||
@@ -810,8 +834,7 @@ int ipr_inspiring_create(int device, int max_sets, ipr_inspiring** out) {
         (e = cudaMemcpy(c->vm, vmask.data(), vmask.size() * 4, cudaMemcpyHostToDevice)) ||
         (e = ipr::make_pack_map(&c->tm_bt, c->bt, max_sets)) || (e = ipr::make_pack_map(&c->tm_btb, c->btb, max_sets)) ||
         (e = ipr::init_device_kernels()) || (e = ipr::set_constants(hp.barrett, hp.q0_inv_mod_q1)) ||
-        (e = cudaFuncSetAttribute(ipr::k_off_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, ipr::N * ipr::GZ * 4)) ||
-        (e = cudaFuncSetAttribute(ipr::k_off_jntt, cudaFuncAttributeMaxDynamicSharedMemorySize, ipr::JNTT_SMEM)) ||
+        (e = cudaFuncSetAttribute(ipr::k_off_jntt<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ipr::JNTT_SMEM)) ||
         (e = ipr::collapse_attributes())) {
         ipr_inspiring_destroy(c);
         return ipr::cuda_fail(e, "ipr_inspiring_create");
@@ -840,9 +863,8 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     const dim3 lwe_grid(N / HCOLS, (unsigned)sets, 2);
     if (reinterpret_cast<uintptr_t>(d_lwe) % 32 == 0) k_lwe_prep<true><<<lwe_grid, 256, 0, st>>>(d_lwe, sets, fwi, c->act);
     else k_lwe_prep<false><<<lwe_grid, 256, 0, st>>>(d_lwe, sets, fwi, c->act);
-    k_off_jntt<<<dim3(N / JS, (unsigned)sets, 2), 256, JNTT_SMEM, st>>>(c->act, sets, fwi, c->E);
-    k_off_gather<<<dim3(N / GZ, (unsigned)sets, 2), 256, N * GZ * 4, st>>>(c->E, sets, c->act);
-    launch_collapse(c->act, 0, sets, c->wm, reinterpret_cast<uint2*>(c->fwi), reinterpret_cast<uint2*>(c->iwi), c->bt,
+    k_off_jntt<true><<<dim3(N / JS, (unsigned)sets, 2), 256, JNTT_SMEM, st>>>(c->act, sets, fwi, c->F);
+    launch_collapse(c->F, 0, sets, c->wm, reinterpret_cast<uint2*>(c->fwi), reinterpret_cast<uint2*>(c->iwi), c->bt,
                     c->btb, c->r0, c->xb, c->d_err, c->sm_count, st);
     k_off_finish<<<(unsigned)sets, 512, coll_smem, st>>>(c->r0, c->xb, 0, c->vm, c->fw, c->fwp, c->iw, c->iwp, c->bth,
                                                          c->a_hat);
