@@ -207,8 +207,10 @@ __global__ void __launch_bounds__(E_THREADS, I > 8 ? 3 : 2) k_encode(const uint1
     auto at = [&](int off, int poly, int chunk) {  // byte offset of this lane's two rows
         return 2 * ((base + off + (int64_t)poly * N + (int64_t)chunk * S) * db_rows + row);
     };
-    // within a set, every column is a compile-time multiple of these many bytes away
-    const uint32_t step = (uint32_t)(2 * (N / 4) * db_rows);  // a quarter polynomial
+    // within a set, every column is a compile-time number of quarter polynomials away: one 32 x 32 ->
+    // 64-bit product (a quarter polynomial has 2^32 bytes at 2^22 rows; no memory holds 2^32 rows)
+    const uint32_t rows = (uint32_t)db_rows;
+    auto quarters = [&](int n) { return (uint64_t)rows * (uint32_t)(2 * (N / 4) * n); };
     const char* inb = reinterpret_cast<const char*>(in);
     char* outb = reinterpret_cast<char*>(out);
     for (int set = warp; set < OFFS * SETS1; set += E_THREADS / 32) {
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(E_THREADS, I > 8 ? 3 : 2) k_encode(const uint1
             for (int bit = 1, r = G / 2; bit < G; bit *= 2, r /= 2) bp += p & bit ? r : 0;
 #pragma unroll
             for (int m = 0; m < M; m++)  // chunks C1 apart: N / M coefficients
-                w[p][m] = __ldg(reinterpret_cast<const uint32_t*>(src + (uint64_t)step * (bp * G2 * 4 + m * (4 / M))));
+                w[p][m] = __ldg(reinterpret_cast<const uint32_t*>(src + quarters(bp * G2 * 4 + m * (4 / M))));
         }
 #pragma unroll
         for (int p = 0; p < G; p++)
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(E_THREADS, I > 8 ? 3 : 2) k_encode(const uint1
                 const uint32_t r = e_pack<G>(lo[p][m], hi[p][m], one);
                 if constexpr (G2 > 1) dst[(p * H + m * C1) * 32] = r;
                 else if (live)
-                    *reinterpret_cast<uint32_t*>(od + (uint64_t)step * (p * 4 + m * (4 / M))) = e_scale<16 - LOGI>(r);
+                    *reinterpret_cast<uint32_t*>(od + quarters(p * 4 + m * (4 / M))) = e_scale<16 - LOGI>(r);
             }
     }
     if constexpr (G2 > 1) {
@@ -273,7 +275,7 @@ __global__ void __launch_bounds__(E_THREADS, I > 8 ? 3 : 2) k_encode(const uint1
 #pragma unroll
                 for (int m = 0; m < M2; m++)
                     if (live)
-                        *reinterpret_cast<uint32_t*>(od + (uint64_t)step * (g * G * 4 + m * 2)) =
+                        *reinterpret_cast<uint32_t*>(od + quarters(g * G * 4 + m * 2)) =
                             e_scale<16 - LOGI>(e_pack<G2>(lo[g][m], hi[g][m], one));
         }
     }
