@@ -105,7 +105,8 @@ void launch_ntt_limb(uint64_t* polys, int64_t count, uint32_t q, const uint2* tw
 
 // out[j][p][s] = in[p][auto_src(ks[j], s)]: a CTA stages one input polynomial in shared memory and
 // writes its image under its share of the requested automorphisms (blockIdx.y with SPLIT, else
-// all).  Bound by the writes.
+// all).  Bound by the writes.  Without SPLIT a polynomial is read by one CTA alone, before that CTA
+// writes, so an output block may lie on the input; with SPLIT the two must not overlap.
 // 256 polynomials under 64 automorphisms 45 us (6.1 TB/s); 64 under 64 15 us, against 37 us with a CTA
 // per polynomial alone.  More CTAs per SM, eight unrolled stores or 32-byte stores of four slots
 // measured 47.5 us at 256 x 64.
@@ -216,9 +217,14 @@ int ipr_automorph_batch(int device, const uint64_t* d_in, uint64_t count, const 
     if (st) return st;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    // fewer polynomials than two CTAs per SM are shared out by automorphism
+    // fewer polynomials than two CTAs per SM are shared out by automorphism, unless the output overlaps
+    // the input: another CTA could then have written a polynomial before it is read
+    const uint64_t bytes = count * ipr::N * 8, in0 = reinterpret_cast<uintptr_t>(d_in),
+                   out0 = reinterpret_cast<uintptr_t>(d_out);
+    const bool overlap = in0 < out0 + bytes * (uint64_t)nk && out0 < in0 + bytes;
     const int64_t gx = std::min<int64_t>((int64_t)count, (int64_t)sms * 8);
-    const int64_t gy = std::min<int64_t>(std::max<int64_t>((int64_t)sms * 2 / gx, 1), std::min(nk, 65535));
+    const int64_t share = overlap ? 1 : std::max<int64_t>((int64_t)sms * 2 / gx, 1);
+    const int64_t gy = std::min<int64_t>(share, std::min(nk, 65535));
     const dim3 grid((unsigned)gx, (unsigned)gy);
     auto cs = static_cast<cudaStream_t>(stream);
     if (gy > 1) ipr::k_automorph<true><<<grid, 256, 0, cs>>>(d_in, (int64_t)count, d_ks, nk, d_out);
