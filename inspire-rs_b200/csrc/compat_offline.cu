@@ -195,12 +195,14 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// act[l][j][s] (u32) from prepacked a_ct[j][l*N + s] (u64) of one column group
+// act[l][j][s] (u32) from prepacked a_ct[j][l*N + s] (u64) of one column group, reduced: the transform
+// over j is lazy and takes canonical residues
 __global__ void k_act_from_u64(const uint64_t* __restrict__ a_ct, uint32_t* __restrict__ act) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)N * CC;
          e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = e / CC, ls = e % CC;
-        act[(ls / N) * (int64_t)N * N + j * N + (ls % N)] = (uint32_t)a_ct[e];
+        const int l = (int)(ls / N);
+        act[l * (int64_t)N * N + j * N + (ls % N)] = mod64(a_ct[e], l ? Q1 : Q0, l ? BR1 : BR0);
     }
 }
 
