@@ -289,8 +289,9 @@ int ipr_automorph_batch(int device, const uint64_t *d_in, uint64_t count, const 
  * condensed, d_bold_t_hat [instances][3][2048] condensed.  Replaces the reference's
  * gpu_hint_*, gpu_prep_pack_*, gpu_packing_* and gpu_collapse_* sequence.  Scratch is
  * allocated inside, at most scratch_bytes (0 = 4 GiB; 32 MiB per instance processed
- * together, 64 MiB when d_bold_t is not 16-byte aligned: it holds intermediate values until
- * it is written); the call returns when the outputs are complete. */
+ * together, 64 MiB when d_bold_t is not 16-byte aligned or d_db lies inside it: it holds
+ * intermediate values until it is written); the call returns when the outputs are complete.
+ * d_db may lie inside an output when all instances are processed together. */
 int ipr_offline_precompute(int device, const uint16_t *d_db, uint64_t db_rows, uint64_t instances,
                            uint64_t *d_a_hat, uint64_t *d_bold_t, uint64_t *d_bold_t_bar, uint64_t *d_bold_t_hat,
                            uint64_t scratch_bytes, void *stream);

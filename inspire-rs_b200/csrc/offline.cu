@@ -649,8 +649,8 @@ cudaError_t narrow_u64(const uint64_t* in, int64_t n, uint32_t* out, cudaStream_
 }
 
 // scratch bytes per instance: F (32 MB) and the chain ends (32 KB); act (32 MB) is dead before the
-// collapse writes bold_t (48 MB per instance) and lives there when that is 16-byte aligned, else
-// in scratch too
+// collapse writes bold_t (48 MB per instance) and lives there when that is 16-byte aligned and
+// apart from the DB (which is read until act is complete), else in scratch too
 constexpr uint64_t kOfflineScratchPerInstance = 2ull * N * N * 4 + 2ull * N * 4 + (uint64_t)N * 8;
 static_assert(2ull * N * N * 4 <= (uint64_t)NINNER * N * 8, "act fits in bold_t");
 
@@ -672,7 +672,9 @@ int offline_precompute_device(const uint16_t* d_db, uint64_t db_rows, uint64_t i
     offline_host_inputs(hp, (unsigned)(db_rows / N), query, wmask, vmask);
     // chunk of instances per pass, bounded by the scratch budget (0 = 4 GiB)
     const uint64_t budget = scratch_budget ? scratch_budget : (4ull << 30);
-    const bool in_place = reinterpret_cast<uintptr_t>(d_bt) % 16 == 0;
+    const uint64_t db0 = reinterpret_cast<uintptr_t>(d_db), bt0 = reinterpret_cast<uintptr_t>(d_bt);
+    const bool apart = db0 >= bt0 + instances * NINNER * N * 8 || bt0 >= db0 + instances * N * db_rows * 2;
+    const bool in_place = apart && bt0 % 16 == 0;
     const uint64_t per = kOfflineScratchPerInstance + (in_place ? 0 : 2ull * N * N * 4);
     const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(instances, budget / per));
     // one allocation for everything (each costs about 0.8 ms with its release): the parts, each a
