@@ -307,13 +307,18 @@ int ipr_offline_precompute(int device, const uint16_t *d_db, uint64_t db_rows, u
  * mod q1).  d_out [sets][2][2048] u64: row 0 = a_hat mod q, row 1 = b + the packed
  * sum mod q (not reduced, < 2q, as add_raw leaves it).  The context holds the
  * tables, the W / V masks and scratch for up to max_sets sets (about 150 MB each);
- * calls on one context must not overlap on the GPU.  A bounded device-side wait that ran
- * out makes the next ipr_inspiring_pack on the context return IPR_E_TIMEOUT (and
- * ipr_offline_precompute, which waits for its outputs, return it itself). */
+ * calls on one context must not overlap on the GPU.
+ * ipr_inspiring_pack only enqueues its kernels, so a bounded device-side wait that ran out in one
+ * of them is reported later: by ipr_inspiring_sync, which waits for `stream` (the one given
+ * to the calls) and returns IPR_E_TIMEOUT when that happened in any call since the last report, or by
+ * the next ipr_inspiring_pack, which then enqueues nothing.  Each report clears the state and
+ * the context stays usable.  The outputs of a series of calls are valid once ipr_inspiring_sync has
+ * returned IPR_OK after it (and no pack in between has returned IPR_E_TIMEOUT). */
 typedef struct ipr_inspiring ipr_inspiring;
 int ipr_inspiring_create(int device, int max_sets, ipr_inspiring **out);
 int ipr_inspiring_pack(ipr_inspiring *ctx, int sets, const uint64_t *d_lwe, const uint64_t *d_y_body,
                        const uint64_t *d_z_body, uint64_t *d_out, void *stream);
+int ipr_inspiring_sync(ipr_inspiring *ctx, void *stream);
 void ipr_inspiring_destroy(ipr_inspiring *ctx);
 
 /* Server state file (no reference counterpart: the reference reruns encode and the
@@ -370,6 +375,10 @@ void ipr_client_destroy(ipr_client *c);
  * succeed and the one after fails as an out-of-memory would (IPR_E_OOM from the call that
  * needed it); the hook then switches itself off.  after < 0 switches it off at once. */
 int ipr_debug_fail_allocation(int64_t after);
+
+/* Fault injection for tests: sets the error word of a packing context to `code` (not 0), as one of
+ * its kernels does when a wait runs out. */
+int ipr_debug_inspiring_error(ipr_inspiring *ctx, int code);
 
 /* The compute capability the library's device code was compiled for, as the CUDA runtime
  * reports it for one of its kernels on `device` (100 for sm_100a), without reading the

@@ -135,6 +135,8 @@ _dbg_cut = _sig("ipr_debug_cut_fold_extent", _i32, ctypes.c_int64)
 _offline = _sig("ipr_offline_precompute", _i32, _i32, _vp, _u64, _u64, _vp, _vp, _vp, _vp, _u64, _vp)
 _insp_create = _sig("ipr_inspiring_create", _i32, _i32, _i32, ctypes.POINTER(_vp))
 _insp_pack = _sig("ipr_inspiring_pack", _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp)
+_insp_sync = _sig("ipr_inspiring_sync", _i32, _vp, _vp)
+_insp_debug_error = _sig("ipr_debug_inspiring_error", _i32, _vp, _i32)
 _insp_destroy = _sig("ipr_inspiring_destroy", None, _vp)
 _save = _sig("ipr_server_save", _i32, _vp, ctypes.c_char_p)
 _load = _sig("ipr_server_load", _i32, _i32, ctypes.c_char_p, ctypes.POINTER(_vp))
@@ -262,7 +264,17 @@ class InspiringPacker:
         self._h, self.max_sets, self.device = h, max_sets, device
 
     def pack(self, sets: int, d_lwe: int, d_y_body: int, d_z_body: int, d_out: int, stream: int = 0):
+        """enqueues on `stream`; the outputs are valid once sync() has returned without an error"""
         _check(_insp_pack(self._h, sets, d_lwe, d_y_body, d_z_body, d_out, stream or None), "ipr_inspiring_pack")
+
+    def sync(self, stream: int = 0):
+        """waits for `stream` and raises IprError (IPR_E_TIMEOUT) when a device-side wait of a pack
+        since the last report ran out"""
+        _check(_insp_sync(self._h, stream or None), "ipr_inspiring_sync")
+
+    def debug_error(self, code: int):
+        """ipr_debug_inspiring_error: the state a kernel leaves when one of its waits runs out (tests)"""
+        _check(_insp_debug_error(self._h, code), "ipr_debug_inspiring_error")
 
     def close(self):
         if self._h and self._h.value:

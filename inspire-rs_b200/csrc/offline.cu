@@ -789,6 +789,19 @@ struct ipr_inspiring {
     }
 };
 
+namespace {
+// the status of the calls whose kernels have run since the last report: the error word is taken
+// and cleared in one, so each failure is reported once
+int inspiring_error(ipr_inspiring* c) {
+    const int code = __atomic_exchange_n(c->h_err, 0, __ATOMIC_ACQ_REL);
+    if (!code) return IPR_OK;
+    char buf[128];
+    snprintf(buf, sizeof(buf), "ipr_inspiring: a device-side wait of an earlier pack ran out (code %d)", code);
+    ipr::set_last_error(buf);
+    return IPR_E_TIMEOUT;
+}
+}  // namespace
+
 extern "C" {
 
 void ipr_inspiring_destroy(ipr_inspiring* ctx) {
@@ -854,10 +867,8 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
     }
     cudaError_t e = cudaSetDevice(c->device);
     if (e != cudaSuccess) return ipr::cuda_fail(e, "set device");
-    if (*static_cast<volatile int*>(c->h_err)) {
-        ipr::set_last_error("ipr_inspiring_pack: a device-side wait of an earlier call ran out");
-        return IPR_E_TIMEOUT;
-    }
+    int st0 = inspiring_error(c);
+    if (st0) return st0;
     using namespace ipr;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int coll_smem = (int)sizeof(CollapseSmem);
@@ -876,6 +887,23 @@ int ipr_inspiring_pack(ipr_inspiring* c, int sets, const uint64_t* d_lwe, const 
         return cuda_fail(e, "online kernels");
     k_inspiring_out<<<148, 256, 0, st>>>(c->a_hat, c->R, d_lwe, sets, d_out);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "output");
+    return IPR_OK;
+}
+
+int ipr_inspiring_sync(ipr_inspiring* c, void* stream) {
+    if (!c) {
+        ipr::set_last_error("ipr_inspiring_sync: null context");
+        return IPR_E_ARGS;
+    }
+    cudaError_t e = cudaSetDevice(c->device);
+    if (e != cudaSuccess) return ipr::cuda_fail(e, "set device");
+    if ((e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream))) != cudaSuccess) return ipr::cuda_fail(e, "run");
+    return inspiring_error(c);
+}
+
+int ipr_debug_inspiring_error(ipr_inspiring* c, int code) {
+    if (!c || !code) return IPR_E_ARGS;
+    __atomic_store_n(c->h_err, code, __ATOMIC_RELEASE);
     return IPR_OK;
 }
 
