@@ -385,11 +385,12 @@ int ipr_debug_inspiring_error(ipr_inspiring *ctx, int code);
  * binary. */
 int ipr_device_binary_version(int device, int *binary_version);
 
-/* Failure detection self-test: launches one CTA that waits, with the bounded wait every
- * tensor-core kernel of this library uses on its mbarriers, on a barrier nothing arrives
- * on.  The wait gives up after limit_us microseconds of GPU global time (1 .. 1,000,000,
- * else IPR_E_ARGS); the call returns IPR_E_TIMEOUT (the status a server call returns when
- * one of its kernels' waits runs out, after 100 ms there) and the device stays usable. */
+/* Failure detection self-test: launches one CTA that waits, with each of the two bounded waits
+ * that the kernels of this library use on their mbarriers (inside a CTA, and for data of
+ * another CTA of a cluster), on a barrier nothing arrives on.  Each wait gives up after limit_us
+ * microseconds of GPU global time (1 .. 1,000,000, else IPR_E_ARGS); the call returns
+ * IPR_E_TIMEOUT when both have (the status a server call returns when one of its kernels'
+ * waits runs out, after 100 ms there) and the device stays usable. */
 int ipr_selftest_bounded_wait(int device, uint32_t limit_us);
 
 /* Bounds-checked debug build (libipr_b200_dbg.so, built with -DIPR_BOUNDS_CHECK by

@@ -129,9 +129,11 @@ __global__ void __launch_bounds__(256) k_automorph(const uint64_t* __restrict__ 
     }
 }
 
-// The bounded wait the tensor-core kernels use on their mbarriers (umma::mbar_wait), on a
-// barrier nothing arrives on: the wait gives up after `limit_ns` of global time and the kernel
-// reports it instead of hanging, as the GEMM kernels do through their error flags.
+// The bounded waits that the kernels use on their mbarriers (umma::mbar_wait, and
+// umma::mbar_wait_cluster for data from another CTA of the cluster), one after the other on a
+// barrier nothing arrives on: each gives up after `limit_ns` of global time and the kernel reports
+// it instead of hanging, as the kernels do through their error flags.  out: the waits that
+// completed, a bit each.
 __global__ void k_wait_selftest(uint64_t limit_ns, int* out) {
     __shared__ uint64_t bar;
     if (threadIdx.x == 0) {
@@ -140,7 +142,8 @@ __global__ void k_wait_selftest(uint64_t limit_ns, int* out) {
     }
     __syncthreads();
     const bool done = umma::mbar_wait(&bar, 0, limit_ns);  // phase 0 never completes
-    if (threadIdx.x == 0) *out = done ? 1 : 0;
+    const bool cluster_done = umma::mbar_wait_cluster(&bar, 0, limit_ns);
+    if (threadIdx.x == 0) *out = (done ? 1 : 0) | (cluster_done ? 2 : 0);
 }
 
 // per-device NTT tables (forward and plain inverse twiddles interleaved with their Shoup companions:
