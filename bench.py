@@ -169,6 +169,13 @@ def read_traffic(kernel="k_pack"):
     return None
 
 
+def pack_stream_bytes(instances, batch):
+    """bytes of precomputation that one packing launch streams for `instances` outputs"""
+    if batch > 1:  # slot-indexed bytes, once per batch: [limb][output][slot][4 bytes][6144]
+        return 2 * instances * N * 4 * 3 * N
+    return instances * (2 * 3069 + 3) * N * 8  # bold_t + bold_t_bar + bold_t_hat
+
+
 class CpuFullRespond:
     """The oracle's respond() (the CPU restatement of KeywordServer::respond,
     src/pir/server/keyword.rs:534-628) on the whole 1M workload, measured, not scaled.
@@ -869,12 +876,8 @@ def main():
 
     peak, peak_kind = read_peaks()
     pack_ms = stage_ms["pack"] / max(calls, 1)
-    if B > 1:  # the packing GEMM streams the slot-indexed precomputation once per batch
-        pack_bytes = N * 2 * ((local.instances + 31) // 32) * 128 * 3 * N  # [slot][limb][tile][128 rows][6144]
-        kname = "k_pack_mma"
-    else:
-        pack_bytes = local.instances * (2 * 3069 + 3) * N * 8  # bold_t + bold_t_bar + bold_t_hat per launch
-        kname = "k_pack"
+    pack_bytes = pack_stream_bytes(local.instances, B)
+    kname = "k_pack_mma" if B > 1 else "k_pack"
     achieved = pack_bytes / (pack_ms / 1000.0) / 1e9
     tensor = None
     if B > 1:
