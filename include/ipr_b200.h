@@ -229,14 +229,15 @@ int ipr_server_set_option(ipr_server *srv, int option, int64_t value);
 
 /* Autotuner for the batch path: runs `reps` timed batches of `payloads` synthetic payloads,
  * and as many of payloads / 4 (from 4 payloads up), after one warm-up each, under every
- * candidate of IPR_OPT_PACK_CTA_PAIR {2 (automatic), 0, 1} x IPR_OPT_GEMV_TILE {256, 128},
- * timed with CUDA events on the server's stream, round-robin.  It leaves the server set
+ * IPR_OPT_GEMV_TILE {256, 128}, timed with CUDA events on the server's stream, round-robin.
+ * The list holds each of them for every value of IPR_OPT_PACK_CTA_PAIR {2, 0, 1}, which run the
+ * same kernels and share the times.  It leaves the server set
  * to the candidate with the least device time per payload summed over the two sizes, so a
  * choice that only suits full batches does not slow the smaller ones a serving loop also
  * runs.  Every candidate gives identical responses.  On an error the options are restored. */
 #define IPR_AUTOTUNE_MAX 8
 typedef struct {
-    int candidates;                    /* how many were timed */
+    int candidates;                    /* entries of the arrays below */
     int pack_cta_pair[IPR_AUTOTUNE_MAX]; /* the option's value; no effect on the work */
     int gemv_tile[IPR_AUTOTUNE_MAX];
     double ms[IPR_AUTOTUNE_MAX];       /* mean device time per batch of `payloads` */

@@ -1011,17 +1011,19 @@ int ipr_server_autotune(ipr_server* s, int payloads, int reps, ipr_autotune_resu
     }
     CU(cudaMemcpyAsync(s->d_bq, s->h_bq, (size_t)payloads * qb, cudaMemcpyHostToDevice, s->stream));
     const int old_pair = s->pack_pair, old_tile = s->g1_tile;
-    // every value of the packing option is listed although all run the same kernel; every candidate
-    // is timed at the requested batch size and at a quarter of it: the score is the device time
-    // per payload summed over both
+    // a candidate per value of the packing option and of the GEMM tile.  All values of the packing
+    // option run the same kernels, so a tile is timed once (the first `timed` candidates, with the
+    // option's default) and the others share its times; each is timed at the requested batch
+    // size and at a quarter of it: the score is the device time per payload summed over both
     static const int pairs[] = {2, 0, 1}, tiles[] = {0, 128};
+    constexpr int timed = (int)(sizeof(tiles) / sizeof(tiles[0]));
     *out = ipr_autotune_result{};
     for (int pr : pairs)
         for (int tl : tiles) {
             out->pack_cta_pair[out->candidates] = pr;
             out->gemv_tile[out->candidates++] = tl ? tl : 256;
         }
-    const int nc = out->candidates;
+    const int nc = timed;
     const int sizes[2] = {payloads, payloads >= 4 ? payloads / 4 : 0};
     const int nsz = sizes[1] ? 2 : 1;
     out->small_payloads = sizes[1];
@@ -1082,6 +1084,7 @@ int ipr_server_autotune(ipr_server* s, int payloads, int reps, ipr_autotune_resu
             best_score = score;
         }
     }
+    for (int i = nc; i < out->candidates; i++) out->ms[i] = out->ms[i % nc], out->ms_small[i] = out->ms_small[i % nc];
     cleanup();
     if (st) {
         cudaStreamSynchronize(s->stream);
