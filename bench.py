@@ -609,9 +609,9 @@ def main():
                          "groups of every payload; NCCL broadcast of the queries and gather of the parts) "
                          "instead of one replica per rank")
     ap.add_argument("--fold-form", type=int, default=3, choices=[1, 2, 3, 4, 5],
-                    help="3: fold with the packing post-process fused in, one chain per CTA, two or three CTAs "
-                         "per SM by chain count (default); 4 / 5: always three / two per SM; 2: the same on two "
-                         "chains per CTA; 1: separate INTT + CRT pass")
+                    help="3: fold with the packing post-process fused in, a chain per CTA (two per SM) or per four "
+                         "CTAs by chain count (default); 4 / 5: always a chain per CTA, three / two per SM; 2: the "
+                         "same on two chains per CTA; 1: separate INTT + CRT pass")
     ap.add_argument("--cuda-core-gemv", type=int, default=None, metavar="FORM",
                     help="with --batch 1: the first dimension on the CUDA-core GEMV of this IPR_OPT_GEMV_FORM "
                          "instead of the tensor-core GEMV (a profiling case for that kernel)")

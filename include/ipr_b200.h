@@ -191,11 +191,11 @@ int ipr_server_set_profiling(ipr_server *srv, int on);
 #define IPR_OPT_TENSOR_GEMV 1
 /* IPR_OPT_FOLD_REGISTER_NTT: the form of the RGSW fold.  3 (default) = register-
  * resident NTTs with the packing post-process (INTT + CRT + b add) fused into the
- * fold's own inverse transforms, one chain per CTA, chosen per call between a cluster of four CTAs per
- * chain (few chains), two CTAs
- * per SM (the query's RGSW bodies staged through shared memory) and three per SM (the
- * bodies read from L2 where they are used) by the rounds each needs for the call's
- * chains; 4 = always three per SM; 5 = always two per SM; 2 = the same fused fold on two chains of one
+ * fold's own inverse transforms, chosen per call by the call's chains (sub-queries x fold
+ * groups): few chains run on a cluster of four CTAs each, more of them one per CTA with two CTAs per
+ * SM (the query's RGSW bodies staged through shared memory); 4 = always one per CTA, three
+ * per SM (the bodies read from L2 where they are used); 5 = always one per CTA, two per SM;
+ * 2 = the same fused fold on two chains of one
  * query per CTA sharing the bodies in shared memory (an odd fold-group count leaves
  * half a CTA idle); 1 = register-resident NTTs after a separate INTT + CRT pass;
  * 0 = shared-memory NTTs after that pass (single-payload calls only; batches then

@@ -134,21 +134,21 @@ int ensure_scratch(ipr_server* s, unsigned nq) {
 // (chains per SM x SMs).  In hundredths of a round of two chains per SM staging the RGSW bodies
 // in shared memory (806 us for 31 steps):
 //   two per SM, staged       100 a round, 57 for a last round of at most one chain per SM (460 us)
-//   three per SM, bodies from L2 (more warps to hide latency, 80 registers)  157 a round
 //   four CTAs per chain      19 (150 us) while the chip is not full, then 66 per chain and SM
 // Measured at 148 SMs (us, staged form / four CTAs per chain): 32 chains 460 / 151, 64 460 / 259,
-// 96 460 / 351, 162 806 / 571, 240 806 / 904, 384 1254 / 1374, 768 2506 / 2614.  Forms 4 / 5 force one
-// occupancy.
+// 96 460 / 351, 162 806 / 571, 240 806 / 904, 384 1254 / 1374, 768 2506 / 2614.
+// Three per SM reading the bodies from L2 (form 4) is never ahead.  Below two chains per SM it takes
+// 2 to 15% longer than two per SM.  Beyond that the two differ by no more than two runs of one of
+// them (medians of five in turn, two per SM twice / three: 462 chains 1837, 1845 / 1885, 704 2398, 2418 /
+// 2400, 880 2797, 2773 / 2780, 1056 3728, 3754 / 3694, 1408 4639, 4728 / 4602).  Forms 4 / 5 force one occupancy.
 ipr::FoldForm fold_form(const ipr_server* s, int chains) {
     if (s->fold_mode == 4) return ipr::FoldForm::kThreePerSm;
     if (s->fold_mode == 5) return ipr::FoldForm::kStaged;
     const int64_t sm = s->sm_count > 0 ? s->sm_count : 1;
     const int64_t rest = chains % (2 * sm);
     const int64_t staged = chains / (2 * sm) * 100 + (rest == 0 ? 0 : (rest <= sm ? 57 : 100));
-    const int64_t three = (chains + 3 * sm - 1) / (3 * sm) * 157;
     const int64_t cluster = chains * 66 / sm > 19 ? chains * 66 / sm : 19;
-    if (cluster < staged && cluster < three) return ipr::FoldForm::kCluster;
-    return three >= staged ? ipr::FoldForm::kStaged : ipr::FoldForm::kThreePerSm;
+    return cluster < staged ? ipr::FoldForm::kCluster : ipr::FoldForm::kStaged;
 }
 
 // enqueue the device pipeline for one payload; `prof` = event slot base or -1
