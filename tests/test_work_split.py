@@ -1,7 +1,9 @@
 """Work splits chosen by size, at the sizes where the choice changes.
 
-Every comparison is bit-exact against the oracle, on the first and last output of the
-synthetic server (the oracle generates one output's state alone)."""
+Every comparison is bit-exact: against the oracle, on the first and last output of the synthetic
+server (the oracle generates one output's state alone), or, for the alignments of the offline
+precomputation and the InspiRING pack, against the aligned call (test_offline_oracle.py compares
+those with the oracle)."""
 import pytest
 
 pytestmark = pytest.mark.gpu
