@@ -11,13 +11,15 @@
 // transform of the sum: the packing output S[j] joins the fold's own row-1 accumulator
 // in the NTT domain and no separate INTT + CRT pass (nor its u64 output array) exists.
 //
-// Layout of the work: a CTA of 512 threads takes two fold groups (chains) of one query;
-// each team of 256 threads runs one chain alone (its own named barrier), both teams
-// sharing the query's six RGSW bodies in shared memory.  A thread owns 8 coefficients
-// (layout A of ntt_regs.cuh, e = t + 256 m) of both rows of s as u64 values mod q, kept
-// in a shared-memory slot only that thread touches, and runs the transforms of both CRT
-// limbs itself, so the CRT compose, the packed-row add and the gadget decomposition need
-// no exchange between threads.
+// Three layouts of the work: a chain per CTA of 256 threads (k_fold4) or per cluster of four CTAs
+// (k_fold_cluster), chosen by the number of chains (server.cu, fold_form), and k_fold3 (option
+// value 2): a CTA of 512 threads takes two fold groups (chains) of one query; each team of 256 threads
+// runs one chain alone (its own named barrier), both teams sharing the query's six RGSW bodies
+// in shared memory.  In k_fold3 and k_fold4 a thread owns 8 coefficients (layout A of
+// ntt_regs.cuh, e = t + 256 m) of both rows of s as u64 values mod q, kept in a shared-memory
+// slot only that thread touches, and runs the transforms of both CRT limbs itself, so the
+// CRT compose, the packed-row add and the gadget decomposition need no exchange between
+// threads.
 //
 // Arithmetic: the inverse transforms are Gentleman-Sande butterflies with the plain
 // inverse twiddles (the reference pre-halves them, ntt.rs:93-96, to fold in N^-1);

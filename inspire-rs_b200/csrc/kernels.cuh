@@ -22,11 +22,11 @@ cudaError_t launch_parse_query(const uint8_t* qb, int nq, int db_rows, uint64_t*
 // rows).  One query always takes 16 columns per warp.
 cudaError_t launch_gemv(const uint16_t* db, int db_rows, int64_t db_cols, int nq, const uint32_t* a_il,
                         uint64_t* c, int sm_count, cudaStream_t st, int form = 0, int* err_flag = nullptr);
-// 2D tensor map over the column-major u16 DB ([db_cols][db_rows]), boxes of box_rows x box_cols
-// with the 32-byte swizzle (box_rows = 16)
 // 2D map over [rows][row_words] u64, boxes of box_words x box_rows, not swizzled
 cudaError_t make_u64_row_map(CUtensorMap* map, const uint64_t* base, uint64_t row_words, uint64_t rows,
                              uint32_t box_words, uint32_t box_rows);
+// 2D tensor map over the column-major u16 DB ([db_cols][db_rows]), boxes of box_rows x box_cols
+// with the 32-byte swizzle (box_rows = 16)
 cudaError_t make_u16_col_map(CUtensorMap* map, const uint16_t* db, int db_rows, int64_t db_cols, uint32_t box_rows,
                              uint32_t box_cols);
 // S: sums of at most 15 residues per entry (not reduced), from the arrays behind the two maps

@@ -1,5 +1,6 @@
-"""Full batches of several databases overlapping on the device: the CTA-pair packing GEMM of one
-beside the first-dimension GEMM of another.  Every response equals the one computed alone."""
+"""Full batches of several databases overlapping on the device: the packing GEMM of one beside the
+first-dimension GEMM of another (an earlier form of the packing GEMM, on CTA pairs, did not finish
+here).  Every response equals the one computed alone."""
 import pytest
 
 pytestmark = pytest.mark.gpu
